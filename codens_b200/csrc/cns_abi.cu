@@ -126,7 +126,7 @@ cudaError_t dev_alloc(cns_ctx* c, T** p, size_t n, bool zero = true) {
   if (e != cudaSuccess) return e;
   c->allocs.push_back(q);
   c->scratch_bytes += (long long)bytes;
-  if (zero) e = cudaMemset(q, 0, bytes);
+  if (zero) e = cudaMemsetAsync(q, 0, bytes, c->st);
   *p = static_cast<T*>(q);
   return e;
 }
@@ -142,12 +142,22 @@ void dev_free(cns_ctx* c, T* p) {
   cudaFree(p);
 }
 
+// host data into device memory, ordered on the context's stream and complete
+// on return.  The context's streams do not wait for the default stream, and
+// a copy of pageable memory may return before its last transfer is done, so
+// a plain cudaMemcpy here let a kernel read a tile list still on its way.
+cudaError_t copy_in(cns_ctx* c, void* d, const void* h, size_t bytes) {
+  if (bytes == 0) return cudaSuccess;
+  cudaError_t e = cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, c->st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(c->st);
+  return e;
+}
+
 template <typename T>
 cudaError_t upload(cns_ctx* c, T** p, const T* h, size_t n) {
   cudaError_t e = dev_alloc(c, p, n, false);
   if (e != cudaSuccess) return e;
-  if (n > 0) e = cudaMemcpy(*p, h, sizeof(T) * n, cudaMemcpyHostToDevice);
-  return e;
+  return copy_in(c, *p, h, sizeof(T) * n);
 }
 
 // index space with extent ext(B) per block and its tile work list
@@ -1430,8 +1440,7 @@ int cns_set_scheme(cns_ctx* c, const cns_scheme_t* s) {
     B.ki4 = s->ki4_l ? s->ki4_l[b] : s->ki4;
   }
   if (c->d_blks)
-    CK(cudaMemcpy(c->d_blks, c->lay.blks.data(), sizeof(Blk) * c->lay.blks.size(),
-                  cudaMemcpyHostToDevice));
+    CK(copy_in(c, c->d_blks, c->lay.blks.data(), sizeof(Blk) * c->lay.blks.size()));
   drop_graphs(c);
   persistent_sweep32(c);  // the Euler and Navier-Stokes instantiations differ
   c->mixed_iter = 0;  // a new scheme restarts the defect refresh schedule

@@ -239,11 +239,14 @@ struct IoBufs {
   }
 };
 
-cudaError_t upload_recs(const IoPlan& p, IoRec** d) {
+// on the stream of the kernel that reads them (the context's streams do not
+// wait for the default stream)
+cudaError_t upload_recs(const IoPlan& p, IoRec** d, cudaStream_t st) {
   if (p.recs.empty()) return cudaSuccess;
   cudaError_t e = cudaMalloc(d, sizeof(IoRec) * p.recs.size());
   if (e == cudaSuccess)
-    e = cudaMemcpy(*d, p.recs.data(), sizeof(IoRec) * p.recs.size(), cudaMemcpyHostToDevice);
+    e = cudaMemcpyAsync(*d, p.recs.data(), sizeof(IoRec) * p.recs.size(),
+                        cudaMemcpyHostToDevice, st);
   return e;
 }
 
@@ -292,8 +295,8 @@ int io_read(IoStage& stage, const IoPlan& p, const IoPlan& zero, const Blk* d_bl
   IoBufs bf;
   cudaError_t e = io_stage_init(stage);
   if (e == cudaSuccess) e = cudaMalloc(&bf.d, sizeof(double) * (size_t)(p.nval > 0 ? p.nval : 1));
-  if (e == cudaSuccess) e = upload_recs(p, &bf.d_recs);
-  if (e == cudaSuccess) e = upload_recs(zero, &bf.d_zero);
+  if (e == cudaSuccess) e = upload_recs(p, &bf.d_recs, st);
+  if (e == cudaSuccess) e = upload_recs(zero, &bf.d_zero, st);
   if (e != cudaSuccess) {
     fclose(f);
     return io_fail(err, CNS_ECUDA, std::string("file buffers: ") + cudaGetErrorString(e));
@@ -329,7 +332,7 @@ int io_write(IoStage& stage, const IoPlan& p, const Blk* d_blks, const char* pat
   IoBufs bf;
   cudaError_t e = io_stage_init(stage);
   if (e == cudaSuccess) e = cudaMalloc(&bf.d, sizeof(double) * (size_t)(p.nval > 0 ? p.nval : 1));
-  if (e == cudaSuccess) e = upload_recs(p, &bf.d_recs);
+  if (e == cudaSuccess) e = upload_recs(p, &bf.d_recs, st);
   if (e == cudaSuccess && p.nval > 0) {
     k_io<<<grid_of(p.nval), 256, 0, st>>>(d_blks, bf.d_recs, (int)p.recs.size(), p.nval, bf.d,
                                           1);

@@ -356,6 +356,15 @@ __device__ __forceinline__ bool mbar_wait_bounded(unsigned long long* bar, unsig
   return true;
 }
 
+// the maps are in global memory, written by a host copy: a thread acquires a
+// map through the tensor-map proxy before it issues boxes from it (the copy
+// may have replaced an earlier context's map at the same address)
+__device__ __forceinline__ void map_acquire(const CUtensorMap* map) {
+  asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;\n" ::"l"(
+                   reinterpret_cast<unsigned long long>(map))
+               : "memory");
+}
+
 // one 4D box (x, y, z, component) of a tensor map into shared memory,
 // completing on the transaction count of bar
 __device__ __forceinline__ void box_load(void* dst, const CUtensorMap* map,
@@ -413,6 +422,10 @@ __device__ __forceinline__ bool sweep_f32_tile(const int4 t, const Blk* __restri
     const int ii = x0 + qx, jj = y0 + qy;
     colin[r] = q < NP && ii >= 1 && ii <= B.ni - 1 && jj >= 1 && jj <= B.nj - 1;
     boxo[r] = qy * NXP + qx;
+  }
+  if (BOX && threadIdx.x == 0) {
+    map_acquire(map_d + t.x);
+    map_acquire(static_cast<const CUtensorMap*>(a.map_st) + t.x);
   }
   auto raw_d = [&](int b) { return reinterpret_cast<float*>(sm.raw + b * (S::RD + S::RS)); };
   auto raw_s = [&](int b) {
