@@ -736,7 +736,7 @@ cudaError_t enqueue_step(cns_ctx* c, bool first, bool dt_on) {
   if (e == cudaSuccess) e = launch_prim(0, c->lay.ncells, s.v, ld, c->w.prim, c->st);
   if (e == cudaSuccess && c->sc.ns) {
     e = launch_grad(c->d_blks, all, c->ph, s.v, c->w.prim, ld, s.mu, s.mut, s.tau, s.sn,
-                    s.vol, s.ztemp, c->st);
+                    s.vol, s.ztemp, c->w.rv, c->st);
     if (e == cudaSuccess) e = launch_tau_ghosts(c->bd, s.tau, ld, c->st);
     if (e == cudaSuccess)
       e = enqueue_cllparoi1(c, s.v, s.mu, s.mut, c->sa_dist, s.ztemp, s.tau);
@@ -750,10 +750,9 @@ cudaError_t enqueue_step(cns_ctx* c, bool first, bool dt_on) {
   }
   if (e == cudaSuccess && c->sc.kfmg == 3) e = enqueue_dual(c, nullptr);
   if (e == cudaSuccess)
-    e = launch_implicit(c->d_blks, all, c->tiles64.view(-1), c->faces, -1, c->ph, c->sc,
-                        !c->sc.ns,
+    e = launch_implicit(c->d_blks, all, c->tiles64.view(-1), c->ph, c->sc, !c->sc.ns,
                         c->sc.lmax, s.u, s.dt, s.v, nullptr, s.mu, s.mut, s.sn, s.vol,
-                        s.pression, s.cson, c->w, 1, c->st);
+                        s.pression, s.cson, 1, c->w, 1, c->st);
   if (e == cudaSuccess)
     e = launch_norm_finalize(c->d_blks, c->d_cells_tile0, 0, (int)c->lay.blks.size(),
                              c->w.normpart, c->w.blocksum, c->w.norms, c->st);
@@ -865,7 +864,7 @@ cudaError_t enqueue_step_mixed(cns_ctx* c, MixedMode mode, bool first, bool dt_o
   }
   if (e == cudaSuccess && c->sc.ns) {
     e = launch_grad(c->d_blks, all, c->ph, s.v, w.prim, ld, s.mu, s.mut, s.tau, s.sn, s.vol,
-                    s.ztemp, c->st);
+                    s.ztemp, nullptr, c->st);
     if (e == cudaSuccess) e = launch_tau_ghosts(c->bd, s.tau, ld, c->st);
     if (e == cudaSuccess)
       e = enqueue_cllparoi1(c, s.v, s.mu, s.mut, c->sa_dist, s.ztemp, s.tau);
@@ -2178,9 +2177,8 @@ int cns_adjoint_prepare(cns_ctx* c) {
   CK(launch_rbord(c->bd, c->ph, s.v, ld, s.pression, s.ztemp, s.cson, c->n_idd_ent,
                   c->d_idd_ents, c->d_idd_masks, c->st));
   CK(launch_prim(0, c->lay.ncells, s.v, ld, c->w.prim, c->st));
-  CK(launch_implicit_coefficients(c->d_blks, all, c->faces, -1, c->ph, 1, s.dt, s.v, c->w.prim,
-                                  s.mu, s.mut, s.sn, s.vol, s.cson, c->w, nullptr, nullptr,
-                                  c->st));
+  CK(launch_implicit_coefficients(c->d_blks, all, c->ph, 1, 0., s.dt, s.v, c->w.prim, s.mu,
+                                  s.mut, s.sn, s.vol, s.cson, nullptr, 0, nullptr, c->w, c->st));
   CK(launch_face_jac(c->d_blks, c->faces, c->ph, c->sc, s.v, s.pression, ld, s.sn, c->adj_J,
                      c->st));
   if (c->sc.precision != 0) {
@@ -2238,7 +2236,7 @@ int cns_zvisqc(cns_ctx* c, const double* v, const double* mu, const double* mut,
   CK(sg.err);
   CK(prim_of(c, 0, dv));
   CK(launch_grad(c->d_blks, c->cells.view(-1), c->ph, dv, c->w.prim, ld, dmu, dmut, dtau, dsn,
-                 dvol, dtemp, c->st));
+                 dvol, dtemp, nullptr, c->st));
   CK(launch_tau_ghosts(c->bd, dtau, ld, c->st));
   CK(sg.finish());
   return CNS_OK;
@@ -2283,9 +2281,9 @@ static int implimf(cns_ctx* c, int l, int eu, const double* u, const double* dt,
   CK(prim_of(c, l, dv));
   Scheme sc = c->sc;
   if (sc.kfmg == 3) sc.dt1min = dtpas;
-  CK(launch_implicit(c->d_blks, c->cells.view(l - 1), c->tiles64.view(l - 1), c->faces, l - 1,
-                     c->ph, sc, eu, lmx, du, ddt, dv, dd, dmu, dmut, sn_base(c, l, dsn), dvol,
-                     dps, dcson, c->w, 0, c->st));
+  CK(launch_implicit(c->d_blks, c->cells.view(l - 1), c->tiles64.view(l - 1), c->ph, sc, eu,
+                     lmx, du, ddt, dv, dd, dmu, dmut, sn_base(c, l, dsn), dvol, dps, dcson, 0,
+                     c->w, 0, c->st));
   CK(sg.finish());
   return CNS_OK;
 }

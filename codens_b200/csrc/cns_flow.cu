@@ -452,7 +452,8 @@ __global__ void __launch_bounds__(kTile) k_grad(const Blk* __restrict__ blks,
                                                 double* __restrict__ tau,
                                                 const double* __restrict__ sn,
                                                 const double* __restrict__ vol,
-                                                const double* __restrict__ temp) {
+                                                const double* __restrict__ temp,
+                                                double* __restrict__ rv) {
   int b, i, j, k;
   if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
@@ -460,7 +461,6 @@ __global__ void __launch_bounds__(kTile) k_grad(const Blk* __restrict__ blks,
   double g[12];
 #pragma unroll
   for (int a = 0; a < 12; ++a) g[a] = 0.;
-  (void)s;
   const double fc[4] = {prim[n], prim[ld + n], prim[2 * ld + n], temp[n]};
   // directions in the reference's order: k faces, then j, then i
 #pragma unroll
@@ -520,94 +520,123 @@ __global__ void __launch_bounds__(kTile) k_grad(const Blk* __restrict__ blks,
   tau[ld + n] = m * (dvxy + dvyx);
   tau[2 * ld + n] = m * (dvxz + dvzx);
   tau[4 * ld + n] = m * (dvyz + dvzy);
-  const double kq = ph.cp * (mu[n] / ph.pr + mut[n] / ph.prt);
+  const double kd = mu[n] / ph.pr + mut[n] / ph.prt;
+  const double kq = ph.cp * kd;
   tau[6 * ld + n] = kq * g[9];
   tau[7 * ld + n] = kq * g[10];
   tau[8 * ld + n] = kq * g[11];
+  // the viscous spectral factor of the implicit phase (k_impl_rv)
+  if (rv) rv[n] = ph.gam * kd / s[n];
 }
 
-// per real cell: coefdiag seed (vol/dt, or vol*(fact+1/dt) with fact = 0 or,
-// with dual time stepping, 1.5/dt1min) and the viscous spectral factor rv
-// (implimf_3d.f90:95-105, implimf_eu.f90:82-85, 124-134)
-__global__ void __launch_bounds__(kTile) k_impl_cell0(
-    const Blk* __restrict__ blks, Space sp, Phys ph, int eu, double fact,
-    const double* __restrict__ v, const double* __restrict__ dt,
-    const double* __restrict__ mu, const double* __restrict__ mut,
-    const double* __restrict__ vol, double* coefdiag, double* rv) {
+// the viscous spectral factor rv of a real cell (implimf_3d.f90:95-105), for
+// the calls that do not run k_grad before the implicit phase
+__global__ void __launch_bounds__(kTile) k_impl_rv(const Blk* __restrict__ blks, Space sp,
+                                                   Phys ph, const double* __restrict__ v,
+                                                   const double* __restrict__ mu,
+                                                   const double* __restrict__ mut, double* rv) {
   int b, i, j, k;
   if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
   const long long n = cell_index(blks[b], i, j, k);
-  if (eu) {
-    coefdiag[n] = vol[n] * (fact + 1. / dt[n]);
-  } else {
-    rv[n] = ph.gam * (mu[n] / ph.pr + mut[n] / ph.prt) / v[n];
-    coefdiag[n] = vol[n] / dt[n];
-  }
+  rv[n] = ph.gam * (mu[n] / ph.pr + mut[n] / ph.prt) / v[n];
 }
 
-// per face: spectral radius coefe (implimf_eu.f90:141-159,
-// implimf_3d.f90:110-190)
-template <class TO>
-__global__ void __launch_bounds__(kTile) k_impl_coefe(
-    const Blk* __restrict__ blks, Space sp, int dir, int eu,
-    const double* __restrict__ v, const double* __restrict__ prim, long long ld,
-    const double* __restrict__ sn,
-    const double* __restrict__ vol, const double* __restrict__ cson,
-    const double* __restrict__ rv, double* coefe, TO* coefe_out) {
-  int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
-  const Blk& B = blks[b];
-  const long long inc = ninc_of(B, dir);
-  const long long n = cell_index(B, i, j, k), nl = n - inc;
-  const double sx = sn_ptr(sn, B, dir, 0)[n], sy = sn_ptr(sn, B, dir, 1)[n],
-               sz = sn_ptr(sn, B, dir, 2)[n];
+// spectral radius of one face (implimf_eu.f90:141-159, implimf_3d.f90:110-190)
+// from its two cells q = (u, v, w, c, rv, vol) (Euler: u, v, w from the
+// reciprocal density); every sum of the two cells is symmetric, so both cells
+// of a face form the same value
+template <bool EU>
+__device__ __forceinline__ double face_radius(const double a[6], const double b[6], double sx,
+                                              double sy, double sz) {
   const double cnds = sx * sx + sy * sy + sz * sz;
-  const double cc = 0.5 * (cson[n] + cson[nl]);
-  double ce;
-  if (eu) {
-    const double norm = 1. / v[n], norm1 = 1. / v[nl];
-    const double uu = 0.5 * (v[ld + n] * norm + v[ld + nl] * norm1);
-    const double vv = 0.5 * (v[2 * ld + n] * norm + v[2 * ld + nl] * norm1);
-    const double ww = 0.5 * (v[3 * ld + n] * norm + v[3 * ld + nl] * norm1);
-    ce = 0.5 * (fabs(uu * sx + vv * sy + ww * sz)) + sqrt(cnds) * cc;
-  } else {
-    const double uu = 0.5 * (prim[n] + prim[nl]);
-    const double vv = 0.5 * (prim[ld + n] + prim[ld + nl]);
-    const double ww = 0.5 * (prim[2 * ld + n] + prim[2 * ld + nl]);
-    const double vn = uu * sx + vv * sy + ww * sz;
-    ce = 0.5 * (fabs(vn) + sqrt(cnds) * cc) + (rv[n] + rv[nl]) * cnds / (vol[n] + vol[nl]);
-  }
-  coefe[(long long)dir * ld + n] = ce;
-  if (coefe_out) coefe_out[(long long)dir * ld + n] = (TO)ce;
+  const double cc = 0.5 * (a[3] + b[3]);
+  const double uu = 0.5 * (a[0] + b[0]), vv = 0.5 * (a[1] + b[1]), ww = 0.5 * (a[2] + b[2]);
+  const double vn = uu * sx + vv * sy + ww * sz;
+  if (EU) return 0.5 * (fabs(vn)) + sqrt(cnds) * cc;
+  return 0.5 * (fabs(vn) + sqrt(cnds) * cc) + (a[4] + b[4]) * cnds / (a[5] + b[5]);
 }
 
-// per real cell: coefdiag += coefe of the six faces (implimf_eu.f90:161-170,
-// implimf_3d.f90:192-203: the same left-to-right chain); dtpas > 0: then
-// + 1.5*vol/dtpas, the physical time term of dual time stepping
-// (implimf_3d.f90:213-224)
-template <class TO>
-__global__ void __launch_bounds__(kTile) k_impl_diag(const Blk* __restrict__ blks,
-                                                     Space sp, long long ld,
-                                                     const double* __restrict__ coefe,
-                                                     const double* __restrict__ vol,
-                                                     double dtpas,
-                                                     double* coefdiag, TO* coefdiag_out) {
+template <bool EU>
+__device__ __forceinline__ void radius_cell(const double* __restrict__ v,
+                                            const double* __restrict__ prim, long long ld,
+                                            const double* __restrict__ vol,
+                                            const double* __restrict__ cson,
+                                            const double* __restrict__ rv, long long n,
+                                            double q[6]) {
+  if (EU) {
+    const double norm = 1. / v[n];
+    q[0] = v[ld + n] * norm;
+    q[1] = v[2 * ld + n] * norm;
+    q[2] = v[3 * ld + n] * norm;
+    q[4] = q[5] = 0.;
+  } else {
+    q[0] = prim[n];
+    q[1] = prim[ld + n];
+    q[2] = prim[2 * ld + n];
+    q[4] = rv[n];
+    q[5] = vol[n];
+  }
+  q[3] = cson[n];
+}
+
+// The implicit coefficients of a real cell and its first Jacobi iterate, in
+// one pass: the spectral radii of the cell's six faces (implimf_eu.f90:141-159,
+// implimf_3d.f90:110-190; the lower faces stored, and the upper face at the
+// end of each line), the diagonal in the reference's left-to-right chain --
+// vol/dt, or for the Euler form vol*(1.5/dtpas + 1/dt), then the faces
+// (implimf_eu.f90:82-85, 161-170, implimf_3d.f90:192-203), then 1.5*vol/dtpas
+// for the Navier-Stokes form (implimf_3d.f90:213-224; dtpas > 0: dual time
+// stepping) -- and d1 = -u / cd, the first sweep from a zero iterate, whose
+// face terms are all zero (-u + 0.: +0 for u = 0, as those terms leave it).
+// Bound by the loads of the seven cells (L1 and L2 hits); each interior face
+// is evaluated by both its cells, which costs less than the launches and the
+// re-reads of a seed, a face pass per direction, a diagonal and a first-sweep
+// kernel (one launch instead of six): 10 us less of a 170 us iteration on
+// 64x32x32 Euler cells, 13 us less of 263 us with Navier-Stokes, 15 us less
+// of 2.33 ms on a 1.07M-cell Navier-Stokes channel.
+template <bool EU>
+__global__ void __launch_bounds__(kTile) k_impl_coefs(
+    const Blk* __restrict__ blks, Space sp, double dtpas, const double* __restrict__ v,
+    const double* __restrict__ prim, long long ld, const double* __restrict__ sn,
+    const double* __restrict__ vol, const double* __restrict__ cson,
+    const double* __restrict__ rv, const double* __restrict__ dt,
+    const double* __restrict__ u, double* __restrict__ coefe, double* __restrict__ coefdiag,
+    double* __restrict__ d1) {
   int b, i, j, k;
   if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const long long n = cell_index(B, i, j, k);
-  double c = coefdiag[n];
+  double q0[6];
+  radius_cell<EU>(v, prim, ld, vol, cson, rv, n, q0);
+  const double vn = vol[n];
+  double c;
+  if (EU)
+    c = vn * ((dtpas > 0. ? 1.5 / dtpas : 0.) + 1. / dt[n]);
+  else
+    c = vn / dt[n];
 #pragma unroll
   for (int dir = 0; dir < 3; ++dir) {
     const long long inc = ninc_of(B, dir);
-    c = c + coefe[(long long)dir * ld + n];
-    c = c + coefe[(long long)dir * ld + n + inc];
+    const int p = dir == 0 ? i : (dir == 1 ? j : k);
+    const double *s0 = sn_ptr(sn, B, dir, 0), *s1 = sn_ptr(sn, B, dir, 1),
+                 *s2 = sn_ptr(sn, B, dir, 2);
+    double ql[6], qu[6];
+    radius_cell<EU>(v, prim, ld, vol, cson, rv, n - inc, ql);
+    radius_cell<EU>(v, prim, ld, vol, cson, rv, n + inc, qu);
+    const double cl = face_radius<EU>(q0, ql, s0[n], s1[n], s2[n]);
+    const double cu = face_radius<EU>(qu, q0, s0[n + inc], s1[n + inc], s2[n + inc]);
+    coefe[(long long)dir * ld + n] = cl;
+    if (p == nd_of(B, dir) - 1) coefe[(long long)dir * ld + n + inc] = cu;
+    c = c + cl;
+    c = c + cu;
   }
-  if (dtpas > 0.) c = c + 1.5 * vol[n] / dtpas;
+  if (!EU && dtpas > 0.) c = c + 1.5 * vn / dtpas;
   coefdiag[n] = c;
-  if (coefdiag_out) coefdiag_out[n] = (TO)c;
+  if (d1) {
+#pragma unroll
+    for (int a = 0; a < 5; ++a) d1[a * ld + n] = (-u[a * ld + n] + 0.) / c;
+  }
 }
-
 
 // standalone residual partials from stored arrays (rscpsv.f90 called with u0)
 __global__ void __launch_bounds__(kTile) k_norm_partials(
@@ -822,10 +851,11 @@ cudaError_t launch_tau_ghosts(const Bnd& bd, double* tau, long long ld,
 cudaError_t launch_grad(const Blk* blks, Space sp, Phys ph, const double* v,
                         const double* prim, long long ld, const double* mu,
                         const double* mut, double* tau, const double* sn,
-                        const double* vol, const double* temp, cudaStream_t st) {
+                        const double* vol, const double* temp, double* rv,
+                        cudaStream_t st) {
   if (sp.ntiles > 0)
     k_grad<<<grid_of(sp), kTile, 0, st>>>(blks, sp, ph, v, prim, ld, mu, mut, tau, sn,
-                                          vol, temp);
+                                          vol, temp, rv);
   return cudaGetLastError();
 }
 
@@ -884,44 +914,27 @@ cudaError_t init_jacobi_25d() {
   return e;
 }
 
-// the FP64 sweeps: the first (zero previous iterate) per cell, the others
-// 2.5D-blocked with the increments evaluated by the reference expressions
-// (bit-identical to storing them, implimf_3d.f90:222-466)
+// the FP64 sweeps after the first, whose iterate the coefficient kernel
+// writes into dpp[0]: 2.5D-blocked with the increments evaluated by the
+// reference expressions (bit-identical to storing them,
+// implimf_3d.f90:222-466)
 template <>
-cudaError_t launch_sweeps_t<double>(const Blk* blks, Space cells, Tiles tl, Phys ph,
-                                    Scheme sc, int eu, int lmx, long long ld, const double* u,
-                                    const double* v, const double* prim, const double* ps,
-                                    const double* sn, const double* coefe,
-                                    const double* coefdiag, double* const dpp[2],
-                                    int* cur_out, cudaStream_t st) {
-  const int g = grid_of(cells);
+cudaError_t launch_sweeps_t<double>(const Blk* blks, Tiles tl, Phys ph, Scheme sc, int eu,
+                                    int lmx, long long ld, const double* u, const double* v,
+                                    const double* prim, const double* ps, const double* sn,
+                                    const double* coefe, const double* coefdiag,
+                                    double* const dpp[2], int* cur_out, cudaStream_t st) {
   int cur = 0;
   if (lmx == 0) {
     cudaError_t e0 = cudaMemsetAsync(dpp[0], 0, sizeof(double) * 5 * ld, st);
     if (e0 != cudaSuccess) return e0;
   }
   const int q = eu ? sc.qfix_dfez : 0;
-  for (int ls = 1; ls <= lmx; ++ls) {
-    const int nxt = (ls == 1) ? 0 : 1 - cur;
-    const double* din = dpp[cur];
-    double* dout = dpp[nxt];
-    if (ls == 1) {
-      if (g > 0) {
-        if (eu)
-          k_jacobi_rc<double, true, true><<<g, kTile, 0, st>>>(blks, cells, ph, q, ld, u, v,
-                                                               prim, ps, sn, coefe, coefdiag,
-                                                               din, dout);
-        else
-          k_jacobi_rc<double, false, true><<<g, kTile, 0, st>>>(blks, cells, ph, q, ld, u, v,
-                                                                prim, ps, sn, coefe, coefdiag,
-                                                                din, dout);
-      }
-    } else {
-      cudaError_t e1 = launch_jacobi_25d_t<double>(blks, tl, ph, q, eu, ld, u, v, prim, ps, sn,
-                                                   coefe, coefdiag, din, dout, st);
-      if (e1 != cudaSuccess) return e1;
-    }
-    cur = nxt;
+  for (int ls = 2; ls <= lmx; ++ls) {
+    cudaError_t e1 = launch_jacobi_25d_t<double>(blks, tl, ph, q, eu, ld, u, v, prim, ps, sn,
+                                                 coefe, coefdiag, dpp[cur], dpp[1 - cur], st);
+    if (e1 != cudaSuccess) return e1;
+    cur = 1 - cur;
   }
   *cur_out = cur;
   return cudaGetLastError();
@@ -937,63 +950,43 @@ cudaError_t launch_update_t<double>(const Blk* blks, Space cells, long long ld,
   return cudaGetLastError();
 }
 
-// implicit coefficients computed in FP64 (coefdiag seed, face spectral radii,
-// diagonal); TO copies for the reduced-precision sweeps when given
-template <class TO>
-static cudaError_t implicit_coefficients(const Blk* blks, Space cells,
-                                         const SpaceBuf* faces, int l0, Phys ph, int eu,
+cudaError_t launch_implicit_coefficients(const Blk* blks, Space cells, Phys ph, int eu,
                                          double dtpas, const double* dt, const double* v,
                                          const double* prim, const double* mu,
                                          const double* mut, const double* sn,
-                                         const double* vol, const double* cson, Work& w,
-                                         TO* coefe_out, TO* coefdiag_out, cudaStream_t st) {
-  const long long ld = w.ld;
+                                         const double* vol, const double* cson,
+                                         const double* u, int rv_done, double* d1, Work& w,
+                                         cudaStream_t st) {
+  if (cells.ntiles == 0) return cudaSuccess;
   const int g = grid_of(cells);
-  // dtpas > 0: dual time stepping with physical step dtpas
-  const double fact = dtpas > 0. ? 1.5 / dtpas : 0.;
-  k_impl_cell0<<<g, kTile, 0, st>>>(blks, cells, ph, eu, fact, v, dt, mu, mut, vol,
-                                    w.coefdiag, w.rv);
-  for (int dir = 0; dir < 3; ++dir) {
-    const Space fs = faces[dir].view(l0);
-    if (fs.ntiles > 0)
-      k_impl_coefe<TO><<<fs.ntiles, kTile, 0, st>>>(blks, fs, dir, eu, v, prim, ld, sn, vol,
-                                                    cson, w.rv, w.coefe, coefe_out);
+  if (eu) {
+    k_impl_coefs<true><<<g, kTile, 0, st>>>(blks, cells, dtpas, v, prim, w.ld, sn, vol, cson,
+                                            nullptr, dt, u, w.coefe, w.coefdiag, d1);
+  } else {
+    if (!rv_done) k_impl_rv<<<g, kTile, 0, st>>>(blks, cells, ph, v, mu, mut, w.rv);
+    k_impl_coefs<false><<<g, kTile, 0, st>>>(blks, cells, dtpas, v, prim, w.ld, sn, vol, cson,
+                                             w.rv, dt, u, w.coefe, w.coefdiag, d1);
   }
-  k_impl_diag<TO><<<g, kTile, 0, st>>>(blks, cells, ld, w.coefe, vol, eu ? 0. : dtpas,
-                                       w.coefdiag, coefdiag_out);
   return cudaGetLastError();
 }
 
-cudaError_t launch_implicit_coefficients(const Blk* blks, Space cells,
-                                         const SpaceBuf* faces, int l0, Phys ph, int eu,
-                                         const double* dt, const double* v,
-                                         const double* prim, const double* mu,
-                                         const double* mut, const double* sn,
-                                         const double* vol, const double* cson, Work& w,
-                                         float* coefe32, float* coefdiag32,
-                                         cudaStream_t st) {
-  if (cells.ntiles == 0) return cudaSuccess;
-  return implicit_coefficients<float>(blks, cells, faces, l0, ph, eu, 0., dt, v, prim, mu, mut,
-                                      sn, vol, cson, w, coefe32, coefdiag32, st);
-}
-
-cudaError_t launch_implicit(const Blk* blks, Space cells, Tiles tl, const SpaceBuf* faces,
-                            int l0, Phys ph, Scheme sc, int eu, int lmx,
-                            const double* u, const double* dt, double* v,
+cudaError_t launch_implicit(const Blk* blks, Space cells, Tiles tl, Phys ph, Scheme sc, int eu,
+                            int lmx, const double* u, const double* dt, double* v,
                             double* d_out, const double* mu, const double* mut,
-                            const double* sn, const double* vol,
-                            const double* ps, const double* cson, Work& w,
-                            int want_norms, cudaStream_t st) {
+                            const double* sn, const double* vol, const double* ps,
+                            const double* cson, int rv_done, Work& w, int want_norms,
+                            cudaStream_t st) {
   const long long ld = w.ld;
   if (cells.ntiles == 0) return cudaSuccess;
-  cudaError_t e = implicit_coefficients<double>(blks, cells, faces, l0, ph, eu,
-                                                sc.kfmg == 3 ? sc.dt1min : 0., dt, v, w.prim,
-                                                mu, mut, sn, vol, cson, w, nullptr, nullptr,
-                                                st);
+  // dtpas > 0: dual time stepping with physical step dtpas
+  cudaError_t e = launch_implicit_coefficients(blks, cells, ph, eu,
+                                               sc.kfmg == 3 ? sc.dt1min : 0., dt, v, w.prim,
+                                               mu, mut, sn, vol, cson, u, rv_done,
+                                               lmx >= 1 ? w.dpp[0] : nullptr, w, st);
   int cur = 0;
   if (e == cudaSuccess)
-    e = launch_sweeps_t<double>(blks, cells, tl, ph, sc, eu, lmx, ld, u, v, w.prim, ps, sn,
-                                w.coefe, w.coefdiag, w.dpp, &cur, st);
+    e = launch_sweeps_t<double>(blks, tl, ph, sc, eu, lmx, ld, u, v, w.prim, ps, sn, w.coefe,
+                                w.coefdiag, w.dpp, &cur, st);
   if (e == cudaSuccess)
     e = launch_update_t<double>(blks, cells, ld, w.dpp[cur], v, dt, d_out,
                                 want_norms ? w.normpart : nullptr, st);

@@ -3,9 +3,8 @@
 //   k_ratio       limiter slope-ratio recurrence (sch_roe.f90:146-194)
 //   k_face_flux   Roe-MUSCL face flux, Euler or Navier-Stokes (sch_roe*.f90)
 //   k_accumulate  face-owned residual accumulation, always summed in FP64
-//   k_jacobi_rc   first point-Jacobi sweep, per cell (implimf_eu.f90,
-//                 implimf_3d.f90)
-//   k_jacobi_25d  the following sweeps, 2.5D-blocked through shared memory
+//   k_jacobi_25d  the point-Jacobi sweeps after the first (implimf_eu.f90,
+//                 implimf_3d.f90), 2.5D-blocked through shared memory
 //   k_update      v += d in FP64 and the residual-norm partials
 //
 // The FP64 instantiations (cns_flow.cu, built with --fmad=false) evaluate the
@@ -1165,69 +1164,6 @@ __device__ __forceinline__ void face_tn(const T du[5], const T dl[5], const T fu
     tn[3] = h * s[2] * sx + h * s[5] * sy + h * s[7] * sz;
     tn[4] = h * s[3] * sx + h * s[6] * sy + h * s[8] * sz;
   }
-}
-
-template <class T, bool EU, bool FIRST>
-__global__ void __launch_bounds__(kTile) k_jacobi_rc(
-    const Blk* __restrict__ blks, Space sp, Phys ph64, int qfix, long long ld,
-    const T* __restrict__ u, const T* __restrict__ v, const T* __restrict__ prim,
-    const T* __restrict__ ps, const T* __restrict__ sn, const T* __restrict__ coefe,
-    const T* __restrict__ coefdiag, const T* __restrict__ d_in, T* __restrict__ d_out) {
-  int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
-  const Blk& B = blks[b];
-  const long long n = cell_index(B, i, j, k);
-  const T gam1 = T(ph64.gam1), pinfl = T(ph64.pinfl);
-  T d0[5], f0[9];
-  if (FIRST) {
-#pragma unroll
-    for (int a = 0; a < 5; ++a) d0[a] = T(0.);
-#pragma unroll
-    for (int q = 0; q < 9; ++q) f0[q] = T(0.);
-  } else {
-    df_of<T, EU>(v, prim, ps, d_in, ld, n, gam1, pinfl, qfix, d0, f0);
-  }
-  T d2w[5];
-#pragma unroll
-  for (int a = 0; a < 5; ++a) d2w[a] = -u[a * ld + n];
-#pragma unroll
-  for (int dir = 0; dir < 3; ++dir) {
-    const long long inc = ninc_of(B, dir);
-    const int nd = nd_of(B, dir);
-    const int p = dir == 0 ? i : (dir == 1 ? j : k);
-    const T *s0 = sn_ptr(sn, B, dir, 0), *s1 = sn_ptr(sn, B, dir, 1),
-            *s2 = sn_ptr(sn, B, dir, 2);
-    const T* ce = coefe + (long long)dir * ld;
-    T dl[5], fl[9], du[5], fu[9];
-    if (FIRST || p == 1) {
-#pragma unroll
-      for (int a = 0; a < 5; ++a) dl[a] = T(0.);
-#pragma unroll
-      for (int q = 0; q < 9; ++q) fl[q] = T(0.);
-    } else {
-      df_of<T, EU>(v, prim, ps, d_in, ld, n - inc, gam1, pinfl, qfix, dl, fl);
-    }
-    if (FIRST || p == nd - 1) {
-#pragma unroll
-      for (int a = 0; a < 5; ++a) du[a] = T(0.);
-#pragma unroll
-      for (int q = 0; q < 9; ++q) fu[q] = T(0.);
-    } else {
-      df_of<T, EU>(v, prim, ps, d_in, ld, n + inc, gam1, pinfl, qfix, du, fu);
-    }
-    T tn[5];
-    face_tn<T, EU>(d0, dl, f0, fl, s0[n], s1[n], s2[n], tn);
-    const T cel = ce[n], ceu = ce[n + inc];
-#pragma unroll
-    for (int a = 0; a < 5; ++a) d2w[a] = d2w[a] + tn[a] + cel * dl[a] + ceu * du[a];
-    const long long nu = n + inc;
-    face_tn<T, EU>(du, d0, fu, f0, s0[nu], s1[nu], s2[nu], tn);
-#pragma unroll
-    for (int a = 0; a < 5; ++a) d2w[a] = d2w[a] - tn[a];
-  }
-  const T cd = coefdiag[n];
-#pragma unroll
-  for (int a = 0; a < 5; ++a) d_out[a * ld + n] = d2w[a] / cd;
 }
 
 // ---------------------------------------------------------------------------

@@ -184,10 +184,13 @@ cudaError_t launch_tau_ghosts(const Bnd& bd, double* tau, long long ld,
 cudaError_t launch_prim(long long n0, long long n1, const double* v, long long ld,
                         double* prim, cudaStream_t st);
 
+// viscous gradients and stresses; rv (or null): the implicit phase's viscous
+// spectral factor of the real cells
 cudaError_t launch_grad(const Blk* blks, Space sp, Phys ph, const double* v,
                         const double* prim, long long ld, const double* mu,
                         const double* mut, double* tau, const double* sn,
-                        const double* vol, const double* temp, cudaStream_t st);
+                        const double* vol, const double* temp, double* rv,
+                        cudaStream_t st);
 
 // hot kernels templated on the real type T (double: cns_flow.cu, bit-exact;
 // float: cns_mixed.cu, the reduced-precision half of the mixed form)
@@ -210,7 +213,7 @@ cudaError_t launch_accumulate_t(const Blk* blks, Space sp, const T* G, long long
                                 cudaStream_t st, const T* V);
 // lmx Jacobi sweeps over the real cells; the final iterate is in dpp[*cur_out]
 template <class T>
-cudaError_t launch_sweeps_t(const Blk* blks, Space cells, Tiles tl, Phys ph, Scheme sc, int eu,
+cudaError_t launch_sweeps_t(const Blk* blks, Tiles tl, Phys ph, Scheme sc, int eu,
                             int lmx, long long ld, const T* u, const T* v, const T* prim,
                             const T* ps, const T* sn, const T* coefe, const T* coefdiag,
                             T* const dpp[2], int* cur_out,
@@ -237,7 +240,7 @@ CNS_DECLARE_HOT(double)
 CNS_DECLARE_HOT(float)
 #undef CNS_DECLARE_HOT
 template <>
-cudaError_t launch_sweeps_t<double>(const Blk*, Space, Tiles, Phys, Scheme, int, int, long long,
+cudaError_t launch_sweeps_t<double>(const Blk*, Tiles, Phys, Scheme, int, int, long long,
                                     const double*, const double*, const double*, const double*,
                                     const double*, const double*, const double*,
                                     double* const[2], int*, cudaStream_t);
@@ -492,14 +495,15 @@ inline cudaError_t launch_accumulate(const Blk* blks, Space sp, const double* G,
   return launch_accumulate_t<double>(blks, sp, G, ld, nullptr, u, nullptr, st, V);
 }
 
-// FP64 implicit coefficients with float copies for the mixed sweeps
-cudaError_t launch_implicit_coefficients(const Blk* blks, Space cells,
-                                         const SpaceBuf* faces, int l0, Phys ph, int eu,
-                                         const double* dt, const double* v,
+// the FP64 implicit coefficients w.coefe, w.coefdiag of the cells (dtpas > 0:
+// dual time stepping) and, when d1 is given, the first Jacobi iterate -u / cd;
+// rv_done: w.rv already holds the viscous factor (launch_grad wrote it)
+cudaError_t launch_implicit_coefficients(const Blk* blks, Space cells, Phys ph, int eu,
+                                         double dtpas, const double* dt, const double* v,
                                          const double* prim, const double* mu,
                                          const double* mut, const double* sn,
-                                         const double* vol, const double* cson, Work& w,
-                                         float* coefe32, float* coefdiag32,
+                                         const double* vol, const double* cson,
+                                         const double* u, int rv_done, double* d1, Work& w,
                                          cudaStream_t st);
 
 // The single-precision copies the primitive-velocity kernel writes for the
@@ -552,14 +556,13 @@ cudaError_t launch_face_flux_fma(const Blk* blks, const SpaceBuf* faces, int l0,
 // the implicit phase of implimf_eu (eu = 1) or implimf_3d (eu = 0) on the
 // cells of the space: coefficients, lmx Jacobi sweeps, v += d; d_out
 // (optional) receives the final increment, want_norms stores per-tile
-// residual partials in w.normpart
-cudaError_t launch_implicit(const Blk* blks, Space cells, Tiles tl, const SpaceBuf* faces,
-                            int l0, Phys ph, Scheme sc, int eu, int lmx,
-                            const double* u, const double* dt, double* v,
+// residual partials in w.normpart; rv_done as launch_implicit_coefficients
+cudaError_t launch_implicit(const Blk* blks, Space cells, Tiles tl, Phys ph, Scheme sc, int eu,
+                            int lmx, const double* u, const double* dt, double* v,
                             double* d_out, const double* mu, const double* mut,
-                            const double* sn, const double* vol,
-                            const double* ps, const double* cson, Work& w,
-                            int want_norms, cudaStream_t st);
+                            const double* sn, const double* vol, const double* ps,
+                            const double* cson, int rv_done, Work& w, int want_norms,
+                            cudaStream_t st);
 
 cudaError_t launch_norm_partials(const Blk* blks, Space cells, long long ld,
                                  const double* u0, const double* v,

@@ -73,8 +73,7 @@ __device__ __forceinline__ float face_coef(const float4 qh, const float4 ql, flo
 // pass over memory); a neighbour's inputs are two vector loads of the packed
 // cq32 = (u, v, w, c) and cv32 = (vol, rv) the primitive kernel writes.
 // With d1 given, the cell's first Jacobi iterate too: with a zero previous
-// iterate every face term of the first sweep is zero, so d1 = -u / cd
-// (the value k_jacobi_rc<FIRST> computes, up to the sign of a zero), in
+// iterate every face term of the first sweep is zero, so d1 = -u / cd, in
 // the padded layout.
 template <bool EU>
 __global__ void __launch_bounds__(kTile) k_coef32(
