@@ -55,6 +55,21 @@ struct Space {
   int ntiles;
 };
 
+// the index spaces of the three directions in one launch: CTA q takes tile
+// q / 3 of direction q % 3 (a grid of 3 x the most tiles of a direction), so
+// the CTAs of one place of a block run close together in time
+struct Space3 {
+  Space s[3];
+  int grid() const {
+    int m = 0;
+    for (const Space& a : s) m = a.ntiles > m ? a.ntiles : m;
+    return 3 * m;
+  }
+  __device__ __forceinline__ Space at(int dir) const {  // selects, no local copy
+    return dir == 0 ? s[0] : (dir == 1 ? s[1] : s[2]);
+  }
+};
+
 struct Phys {
   double gam, gam1, pinfl, pr, prt, cp, reynz, suth_a, pa1, aa1, omg;
 };

@@ -863,12 +863,7 @@ template <>
 cudaError_t launch_ratio_t<double>(const Blk* blks, const SpaceBuf* lines, int l0,
                                    const double* v, const double* prim, long long ld,
                                    const double* ps, double* R, cudaStream_t st) {
-  for (int dir = 0; dir < 3; ++dir) {
-    const Space sp = lines[dir].view(l0);
-    if (sp.ntiles > 0)
-      k_ratio<double><<<dim3(grid_of(sp), 5), kTile, 0, st>>>(blks, sp, dir, v, prim, ld, ps, R);
-  }
-  return cudaGetLastError();
+  return ratio_launch<double>(blks, lines, l0, v, prim, ld, ps, R, st);
 }
 
 cudaError_t launch_residual_fused(const Blk* blks, Tiles tl, Phys ph, Scheme sc, const double* v,

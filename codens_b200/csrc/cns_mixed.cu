@@ -189,12 +189,7 @@ template <>
 cudaError_t launch_ratio_t<float>(const Blk* blks, const SpaceBuf* lines, int l0,
                                   const float* v, const float* prim, long long ld,
                                   const float* ps, float* R, cudaStream_t st) {
-  for (int dir = 0; dir < 3; ++dir) {
-    const Space sp = lines[dir].view(l0);
-    if (sp.ntiles > 0)
-      k_ratio<float><<<dim3(grid_of(sp), 5), kTile, 0, st>>>(blks, sp, dir, v, prim, ld, ps, R);
-  }
-  return cudaGetLastError();
+  return ratio_launch<float>(blks, lines, l0, v, prim, ld, ps, R, st);
 }
 
 template <>
@@ -204,16 +199,15 @@ cudaError_t launch_face_flux_t<float>(const Blk* blks, const SpaceBuf* faces, in
                                       const float* sn, const float* R, float* G,
                                       cudaStream_t st, float* V) {
   (void)V;  // the single-precision fluxes are Roe only (defect correction)
-  for (int dir = 0; dir < 3; ++dir) {
-    const Space sp = faces[dir].view(l0);
-    if (sp.ntiles == 0) continue;
-    if (sc.ns)
-      k_face_flux<float, true><<<grid_of(sp), kTile, 0, st>>>(blks, sp, dir, ph, sc, v, prim,
-                                                              ld, ps, tau, sn, R, G);
-    else
-      k_face_flux<float, false><<<grid_of(sp), kTile, 0, st>>>(blks, sp, dir, ph, sc, v, prim,
-                                                               ld, ps, tau, sn, R, G);
-  }
+  const Space3 sp{{faces[0].view(l0), faces[1].view(l0), faces[2].view(l0)}};
+  const int g = sp.grid();
+  if (g == 0) return cudaSuccess;
+  if (sc.ns)
+    k_face_flux<float, true><<<g, kTile, 0, st>>>(blks, sp, ph, sc, v, prim, ld, ps, tau, sn, R,
+                                                  G);
+  else
+    k_face_flux<float, false><<<g, kTile, 0, st>>>(blks, sp, ph, sc, v, prim, ld, ps, tau, sn, R,
+                                                   G);
   return cudaGetLastError();
 }
 
