@@ -291,6 +291,13 @@ int check_status(cns_ctx* c) {
   return CNS_OK;
 }
 
+// the residual norms of all blocks from the tile partials
+cudaError_t finalize_norms(cns_ctx* c) {
+  Work& w = c->w;
+  return launch_norm_finalize(c->d_blks, c->d_cells_tile0, (int)c->lay.blks.size(), w.norm_chunks,
+                              w.normpart, w.chunksum, w.norm_count, w.norms, c->st);
+}
+
 // primitive velocities of the cells of block l (0: every block)
 cudaError_t prim_of(cns_ctx* c, int l, const double* v) {
   long long n0, n1;
@@ -754,8 +761,7 @@ cudaError_t enqueue_step(cns_ctx* c, bool first, bool dt_on) {
                         c->sc.lmax, s.u, s.dt, s.v, nullptr, s.mu, s.mut, s.sn, s.vol,
                         s.pression, s.cson, 1, c->w, 1, c->st);
   if (e == cudaSuccess)
-    e = launch_norm_finalize(c->d_blks, c->d_cells_tile0, 0, (int)c->lay.blks.size(),
-                             c->w.normpart, c->w.blocksum, c->w.norms, c->st);
+    e = finalize_norms(c);
   return e;
 }
 
@@ -931,8 +937,7 @@ cudaError_t enqueue_step_mixed(cns_ctx* c, MixedMode mode, bool first, bool dt_o
   if (e == cudaSuccess)
     e = launch_update32(c->d_blks, all, ld, w.d32pp[cur], s.v, s.dt, w.normpart, c->st);
   if (e == cudaSuccess)
-    e = launch_norm_finalize(c->d_blks, c->d_cells_tile0, 0, (int)c->lay.blks.size(),
-                             w.normpart, w.blocksum, w.norms, c->st);
+    e = finalize_norms(c);
   return e;
 }
 
@@ -1361,7 +1366,14 @@ int cns_create(const cns_layout_t* layout, const cns_phys_t* phys,
   }
   if (e == cudaSuccess) e = dev_alloc(c, &c->w.normpart, (size_t)(15 * c->cells.ntiles));
   if (e == cudaSuccess) e = dev_alloc(c, &c->w.norms, 16);
-  if (e == cudaSuccess) e = dev_alloc(c, &c->w.blocksum, (size_t)(15 * c->lay.blks.size()));
+  for (size_t b = 0; b < c->lay.blks.size(); ++b) {
+    const int t = c->cells.blk_tile0[b + 1] - c->cells.blk_tile0[b];
+    const int n = (t + kNormChunk - 1) / kNormChunk;
+    if (n > c->w.norm_chunks) c->w.norm_chunks = n;
+  }
+  if (e == cudaSuccess)
+    e = dev_alloc(c, &c->w.chunksum, 15 * c->lay.blks.size() * (size_t)c->w.norm_chunks);
+  if (e == cudaSuccess) e = dev_alloc(c, &c->w.norm_count, 1);
   if (e == cudaSuccess) e = ensure_hllc_v(c);
   if (e == cudaSuccess) e = dev_alloc(c, &c->w.status, 1);
   if (e == cudaSuccess) e = cudaMallocHost(&c->h_norms, 16 * sizeof(double));
@@ -2325,8 +2337,7 @@ int cns_rscpsv(cns_ctx* c, const double* u0, const double* v, const double* dt,
   const double* ddt = sg.in(dt, ld);
   CK(sg.err);
   CK(launch_norm_partials(c->d_blks, c->cells.view(-1), ld, du0, dv, ddt, c->w.normpart, c->st));
-  CK(launch_norm_finalize(c->d_blks, c->d_cells_tile0, 0, (int)c->lay.blks.size(),
-                          c->w.normpart, c->w.blocksum, c->w.norms, c->st));
+  CK(finalize_norms(c));
   CK(cudaMemcpyAsync(c->h_norms, c->w.norms, 15 * sizeof(double), cudaMemcpyDeviceToHost,
                      c->st));
   CK(cudaStreamSynchronize(c->st));

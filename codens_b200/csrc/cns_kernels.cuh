@@ -131,7 +131,9 @@ struct Work {
   double* dpp[2] = {nullptr, nullptr};   // Jacobi iterates, [5][ld] each
   double* normpart = nullptr; // per tile partial norms [ntiles][15]
   double* norms = nullptr;    // [16]
-  double* blocksum = nullptr; // per block norm sums [nblk][15]
+  double* chunksum = nullptr; // norm sums [nblk * norm_chunks][15]
+  int norm_chunks = 1;        // the most kNormChunk-tile chunks of a block
+  int* norm_count = nullptr;  // finished CTAs of the norm kernel (0 between launches)
   int* status = nullptr;      // device status word
   // mixed precision (allocated on first use)
   bool mixed_ready = false;
@@ -569,8 +571,12 @@ cudaError_t launch_norm_partials(const Blk* blks, Space cells, long long ld,
                                  const double* dt, double* normpart,
                                  cudaStream_t st);
 
-cudaError_t launch_norm_finalize(const Blk* blks, const int* blk_tile0_dev,
-                                 int b0, int b1, const double* normpart,
-                                 double* blocksum, double* norms, cudaStream_t st);
+// the residual norms from the tile partials of nblk blocks, `chunks` (the
+// most kNormChunk-tile chunks of a block) CTAs a block; chunksum: [nblk *
+// chunks][15] scratch, counter: zero before and after
+constexpr int kNormChunk = 512;
+cudaError_t launch_norm_finalize(const Blk* blks, const int* blk_tile0_dev, int nblk, int chunks,
+                                 const double* normpart, double* chunksum, int* counter,
+                                 double* norms, cudaStream_t st);
 
 }  // namespace cns
