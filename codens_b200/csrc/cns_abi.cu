@@ -800,6 +800,8 @@ cudaError_t ensure_mixed(cns_ctx* c) {
   if (e == cudaSuccess) e = dev_alloc(c, &w.st32, (size_t)(6 * ldp));
   if (e == cudaSuccess) e = dev_alloc(c, &w.cq32, (size_t)ld);
   if (e == cudaSuccess) e = dev_alloc(c, &w.cv32, (size_t)ld);
+  for (int q = 0; q < 2 && e == cudaSuccess && point_sweeps(c->lay); ++q)
+    e = dev_alloc(c, &w.pt32[q], (size_t)(4 * ldp), false);
   if (e == cudaSuccess) {
     std::vector<unsigned char> maps;
     e = encode_sweep32_maps(c->lay.blks, w.st32, w.d32pp, maps);
@@ -925,13 +927,19 @@ cudaError_t enqueue_step_mixed(cns_ctx* c, MixedMode mode, bool first, bool dt_o
   }
   if (e == cudaSuccess && c->sc.kfmg == 3) e = enqueue_dual(c, w.u32);
   // single-precision coefficients and implicit sweeps, FP64 update
+  const bool point = w.pt32[0] && c->sc.lmax >= 2;
   if (e == cudaSuccess)
     e = launch_coefficients32(c->d_blks, all, !c->sc.ns, ld,
                               c->sc.kfmg == 3 ? c->sc.dt1min : 0., s.dt, s.vol, w.cq32,
                               w.cv32, w.sn32, w.coefe32, w.coefdiag32, w.snc32, w.u32,
-                              c->sc.lmax >= 1 ? w.d32pp[0] : nullptr, c->st);
+                              c->sc.lmax >= 1 && !point ? w.d32pp[0] : nullptr,
+                              point ? w.pt32[0] : nullptr, w.st32, c->ph,
+                              c->sc.ns ? 0 : c->sc.qfix_dfez, c->st);
   int cur = 0;
-  if (e == cudaSuccess)
+  if (e == cudaSuccess && point)
+    e = launch_point_sweeps32(c->d_blks, all, c->ph, c->sc, !c->sc.ns, c->sc.lmax, ld,
+                              sweep32_args(c), w.snc32, w.pt32, w.d32pp[0], c->st);
+  else if (e == cudaSuccess)
     e = launch_sweeps32(c->tiles32.view(-1), c->d_blks, c->ph, c->sc, !c->sc.ns, c->sc.lmax,
                         ld, c->lay.ldp, sweep32_args(c), w.d32pp, &cur, c->st);
   if (e == cudaSuccess)
@@ -1363,6 +1371,8 @@ int cns_create(const cns_layout_t* layout, const cns_phys_t* phys,
   if (e == cudaSuccess) e = dev_alloc(c, &c->w.rv, (size_t)ld);
   for (int q = 0; q < 2 && e == cudaSuccess; ++q) {
     e = dev_alloc(c, &c->w.dpp[q], (size_t)(5 * ld));
+    if (e == cudaSuccess && point_sweeps(c->lay))
+      e = dev_alloc(c, &c->w.pt[q], (size_t)(7 * ld), false);
   }
   if (e == cudaSuccess) e = dev_alloc(c, &c->w.normpart, (size_t)(15 * c->cells.ntiles));
   if (e == cudaSuccess) e = dev_alloc(c, &c->w.norms, 16);
@@ -2190,7 +2200,9 @@ int cns_adjoint_prepare(cns_ctx* c) {
                   c->d_idd_ents, c->d_idd_masks, c->st));
   CK(launch_prim(0, c->lay.ncells, s.v, ld, c->w.prim, c->st));
   CK(launch_implicit_coefficients(c->d_blks, all, c->ph, 1, 0., s.dt, s.v, c->w.prim, s.mu,
-                                  s.mut, s.sn, s.vol, s.cson, nullptr, 0, nullptr, c->w, c->st));
+                                  s.mut, s.sn, s.vol, s.cson, nullptr, 0, nullptr, nullptr,
+                                  nullptr, 0,
+                                  c->w, c->st));
   CK(launch_face_jac(c->d_blks, c->faces, c->ph, c->sc, s.v, s.pression, ld, s.sn, c->adj_J,
                      c->st));
   if (c->sc.precision != 0) {

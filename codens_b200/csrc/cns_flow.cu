@@ -556,6 +556,40 @@ __device__ __forceinline__ double face_radius(const double a[6], const double b[
   return 0.5 * (fabs(vn) + sqrt(cnds) * cc) + (a[4] + b[4]) * cnds / (a[5] + b[5]);
 }
 
+// the flux increments of the iterate d of cell n (the reference expressions)
+template <bool EU>
+__device__ __forceinline__ void point_df(const double* __restrict__ v,
+                                         const double* __restrict__ prim,
+                                         const double* __restrict__ ps, long long ld,
+                                         long long n, double gam1, double pinfl, int qfix,
+                                         const double d[5], double f[9]) {
+  jacobi_df<double, EU>(d, v[n], v[ld + n], v[2 * ld + n], v[3 * ld + n], v[4 * ld + n], ps[n],
+                        EU ? 0. : prim[n], EU ? 0. : prim[ld + n], EU ? 0. : prim[2 * ld + n],
+                        gam1, pinfl, qfix, f);
+}
+
+// (d, f) of cell n of the point sweeps' packed iterate; zero unless in
+__device__ __forceinline__ void point_load(const double2* __restrict__ p, long long ld,
+                                           long long n, bool in, double d[5], double f[9]) {
+  double2 x[7];
+#pragma unroll
+  for (int q = 0; q < 7; ++q) x[q] = in ? p[q * ld + n] : make_double2(0., 0.);
+  d[0] = x[0].x, d[1] = x[0].y, d[2] = x[1].x, d[3] = x[1].y, d[4] = x[2].x;
+  f[0] = x[2].y, f[1] = x[3].x, f[2] = x[3].y, f[3] = x[4].x, f[4] = x[4].y;
+  f[5] = x[5].x, f[6] = x[5].y, f[7] = x[6].x, f[8] = x[6].y;
+}
+
+__device__ __forceinline__ void point_store(double2* __restrict__ p, long long ld, long long n,
+                                            const double d[5], const double f[9]) {
+  p[n] = make_double2(d[0], d[1]);
+  p[ld + n] = make_double2(d[2], d[3]);
+  p[2 * ld + n] = make_double2(d[4], f[0]);
+  p[3 * ld + n] = make_double2(f[1], f[2]);
+  p[4 * ld + n] = make_double2(f[3], f[4]);
+  p[5 * ld + n] = make_double2(f[5], f[6]);
+  p[6 * ld + n] = make_double2(f[7], f[8]);
+}
+
 template <bool EU>
 __device__ __forceinline__ void radius_cell(const double* __restrict__ v,
                                             const double* __restrict__ prim, long long ld,
@@ -594,6 +628,8 @@ __device__ __forceinline__ void radius_cell(const double* __restrict__ v,
 // kernel (one launch instead of six): 10 us less of a 170 us iteration on
 // 64x32x32 Euler cells, 13 us less of 263 us with Navier-Stokes, 15 us less
 // of 2.33 ms on a 1.07M-cell Navier-Stokes channel.
+// With p1 given (the point sweeps) the iterate goes there together with its
+// flux increments instead.
 template <bool EU>
 __global__ void __launch_bounds__(kTile) k_impl_coefs(
     const Blk* __restrict__ blks, Space sp, double dtpas, const double* __restrict__ v,
@@ -601,7 +637,8 @@ __global__ void __launch_bounds__(kTile) k_impl_coefs(
     const double* __restrict__ vol, const double* __restrict__ cson,
     const double* __restrict__ rv, const double* __restrict__ dt,
     const double* __restrict__ u, double* __restrict__ coefe, double* __restrict__ coefdiag,
-    double* __restrict__ d1) {
+    double* __restrict__ d1, double2* __restrict__ p1, const double* __restrict__ ps, Phys ph,
+    int qfix) {
   int b, i, j, k;
   if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
@@ -632,9 +669,80 @@ __global__ void __launch_bounds__(kTile) k_impl_coefs(
   }
   if (!EU && dtpas > 0.) c = c + 1.5 * vn / dtpas;
   coefdiag[n] = c;
+  if (!d1 && !p1) return;
+  double d[5];
+#pragma unroll
+  for (int a = 0; a < 5; ++a) d[a] = (-u[a * ld + n] + 0.) / c;
   if (d1) {
 #pragma unroll
-    for (int a = 0; a < 5; ++a) d1[a * ld + n] = (-u[a * ld + n] + 0.) / c;
+    for (int a = 0; a < 5; ++a) d1[a * ld + n] = d[a];
+  } else {
+    double f[9];
+    point_df<EU>(v, prim, ps, ld, n, ph.gam1, ph.pinfl, qfix, d, f);
+    point_store(p1, ld, n, d, f);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Point sweep: the Jacobi sweep of grids small enough for every array of the
+// sweeps to stay in L2 (point_sweeps() in cns_kernels.cuh has the line and
+// both sides' figures).  One thread per cell reads its own and its six
+// neighbours' iterate and flux increment (d, f), evaluates the six faces and
+// the new iterate with the expressions and order of the 2.5D sweep, then the
+// new iterate's increment once, for the next sweep: no tile prologue, no
+// plane-by-plane chain, every load of a cell independent of the others.  (On
+// a large grid the stored increments would cost 72 B more a cell and sweep,
+// and the k neighbours come from HBM again: the 2.5D sweep stays.)  Same
+// inputs through the same operations as the 2.5D sweep: the same bits.
+// (d, f) is packed as seven double2 [d0 d1][d2 d3][d4 f0][f1 f2][f3 f4]
+// [f5 f6][f7 f8], component-major: a warp's loads are whole lines.
+// ---------------------------------------------------------------------------
+template <bool EU, bool LAST>
+__global__ void __launch_bounds__(kTile) k_jacobi_point(
+    const Blk* __restrict__ blks, Space sp, Phys ph, int qfix, long long ld,
+    const double* __restrict__ u, const double* __restrict__ v,
+    const double* __restrict__ prim, const double* __restrict__ ps,
+    const double* __restrict__ sn, const double* __restrict__ coefe,
+    const double* __restrict__ coefdiag, const double2* __restrict__ p_in,
+    double2* __restrict__ p_out, double* __restrict__ d_out) {
+  int b, i, j, k;
+  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  const Blk& B = blks[b];
+  const long long n = cell_index(B, i, j, k);
+  double d0[5], f0[9], w[5];
+  point_load(p_in, ld, n, true, d0, f0);
+#pragma unroll
+  for (int a = 0; a < 5; ++a) w[a] = -u[a * ld + n];
+#pragma unroll
+  for (int dir = 0; dir < 3; ++dir) {
+    const long long inc = ninc_of(B, dir);
+    const int p = dir == 0 ? i : (dir == 1 ? j : k);
+    const double *s0 = sn_ptr(sn, B, dir, 0), *s1 = sn_ptr(sn, B, dir, 1),
+                 *s2 = sn_ptr(sn, B, dir, 2);
+    const double* ce = coefe + (long long)dir * ld;
+    double dl[5], fl[9], du[5], fu[9], tl[5], tu[5];
+    point_load(p_in, ld, n - inc, p > 1, dl, fl);
+    point_load(p_in, ld, n + inc, p < nd_of(B, dir) - 1, du, fu);
+    face_tn<double, EU>(d0, dl, f0, fl, s0[n], s1[n], s2[n], tl);
+    face_tn<double, EU>(du, d0, fu, f0, s0[n + inc], s1[n + inc], s2[n + inc], tu);
+    const double cel = ce[n], ceu = ce[n + inc];
+#pragma unroll
+    for (int a = 0; a < 5; ++a) {
+      w[a] = w[a] + tl[a] + cel * dl[a] + ceu * du[a];
+      w[a] = w[a] - tu[a];
+    }
+  }
+  const double cd = coefdiag[n];
+  double d[5];
+#pragma unroll
+  for (int a = 0; a < 5; ++a) d[a] = w[a] / cd;
+  if (LAST) {
+#pragma unroll
+    for (int a = 0; a < 5; ++a) d_out[a * ld + n] = d[a];
+  } else {
+    double f[9];
+    point_df<EU>(v, prim, ps, ld, n, ph.gam1, ph.pinfl, qfix, d, f);
+    point_store(p_out, ld, n, d, f);
   }
 }
 
@@ -970,17 +1078,43 @@ cudaError_t launch_implicit_coefficients(const Blk* blks, Space cells, Phys ph, 
                                          const double* prim, const double* mu,
                                          const double* mut, const double* sn,
                                          const double* vol, const double* cson,
-                                         const double* u, int rv_done, double* d1, Work& w,
+                                         const double* u, int rv_done, double* d1,
+                                         double2* p1, const double* ps, int qfix, Work& w,
                                          cudaStream_t st) {
   if (cells.ntiles == 0) return cudaSuccess;
   const int g = grid_of(cells);
   if (eu) {
     k_impl_coefs<true><<<g, kTile, 0, st>>>(blks, cells, dtpas, v, prim, w.ld, sn, vol, cson,
-                                            nullptr, dt, u, w.coefe, w.coefdiag, d1);
+                                            nullptr, dt, u, w.coefe, w.coefdiag, d1, p1, ps, ph,
+                                            qfix);
   } else {
     if (!rv_done) k_impl_rv<<<g, kTile, 0, st>>>(blks, cells, ph, v, mu, mut, w.rv);
     k_impl_coefs<false><<<g, kTile, 0, st>>>(blks, cells, dtpas, v, prim, w.ld, sn, vol, cson,
-                                             w.rv, dt, u, w.coefe, w.coefdiag, d1);
+                                             w.rv, dt, u, w.coefe, w.coefdiag, d1, p1, ps, ph,
+                                             qfix);
+  }
+  return cudaGetLastError();
+}
+
+// sweeps 2..lmx of a small grid (the first iterate is in w.pt[0]); the final
+// iterate in w.dpp[0]
+static cudaError_t point_sweeps64(const Blk* blks, Space cells, Phys ph, int qfix, int eu,
+                                  int lmx, const double* u, const double* v, const double* ps,
+                                  const double* sn, Work& w, cudaStream_t st) {
+  const int g = grid_of(cells);
+  auto run = [&](auto kernel, const double2* in, double2* out) {
+    kernel<<<g, kTile, 0, st>>>(blks, cells, ph, qfix, w.ld, u, v, w.prim, ps, sn, w.coefe,
+                                w.coefdiag, in, out, w.dpp[0]);
+  };
+  for (int ls = 2; ls <= lmx; ++ls) {
+    const double2* in = w.pt[ls & 1];
+    double2* out = w.pt[(ls & 1) ^ 1];
+    if (eu)
+      ls < lmx ? run(k_jacobi_point<true, false>, in, out)
+               : run(k_jacobi_point<true, true>, in, out);
+    else
+      ls < lmx ? run(k_jacobi_point<false, false>, in, out)
+               : run(k_jacobi_point<false, true>, in, out);
   }
   return cudaGetLastError();
 }
@@ -993,13 +1127,17 @@ cudaError_t launch_implicit(const Blk* blks, Space cells, Tiles tl, Phys ph, Sch
                             cudaStream_t st) {
   const long long ld = w.ld;
   if (cells.ntiles == 0) return cudaSuccess;
+  const int qfix = eu ? sc.qfix_dfez : 0;
+  const bool point = w.pt[0] && lmx >= 2;
   // dtpas > 0: dual time stepping with physical step dtpas
-  cudaError_t e = launch_implicit_coefficients(blks, cells, ph, eu,
-                                               sc.kfmg == 3 ? sc.dt1min : 0., dt, v, w.prim,
-                                               mu, mut, sn, vol, cson, u, rv_done,
-                                               lmx >= 1 ? w.dpp[0] : nullptr, w, st);
+  cudaError_t e = launch_implicit_coefficients(
+      blks, cells, ph, eu, sc.kfmg == 3 ? sc.dt1min : 0., dt, v, w.prim, mu, mut, sn, vol, cson,
+      u, rv_done, lmx >= 1 && !point ? w.dpp[0] : nullptr, point ? w.pt[0] : nullptr, ps, qfix, w,
+      st);
   int cur = 0;
-  if (e == cudaSuccess)
+  if (e == cudaSuccess && point)
+    e = point_sweeps64(blks, cells, ph, qfix, eu, lmx, u, v, ps, sn, w, st);
+  else if (e == cudaSuccess)
     e = launch_sweeps_t<double>(blks, tl, ph, sc, eu, lmx, ld, u, v, w.prim, ps, sn, w.coefe,
                                 w.coefdiag, w.dpp, &cur, st);
   if (e == cudaSuccess)

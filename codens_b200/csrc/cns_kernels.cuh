@@ -115,6 +115,16 @@ struct TileBuf {
   }
 };
 
+// Whether a layout's Jacobi sweeps run as point sweeps (one thread per cell
+// from stored increments) instead of 2.5D tiles: while all that the sweeps
+// touch stays in the 126 MB L2.  Whole iterations of ten sweeps, tiles
+// against points: 64x32x32 cells 161 -> 113 us (Euler), 197 -> 135
+// (Navier-Stokes), mixed 131 -> 89 and 145 -> 105; 131k cells 241 -> 189,
+// 313 -> 226, 150 -> 132, 178 -> 158; at 196k FP64 is even (289 and 306, 355
+// and 351).
+constexpr long long kPointCells = 200000;
+inline bool point_sweeps(const HostLayout& lay) { return lay.nreal <= kPointCells; }
+
 // per-step scratch (device)
 struct Work {
   long long ld = 0;
@@ -129,6 +139,8 @@ struct Work {
   double* coefdiag = nullptr; // [ld]
   double* rv = nullptr;       // [ld]
   double* dpp[2] = {nullptr, nullptr};   // Jacobi iterates, [5][ld] each
+  double2* pt[2] = {nullptr, nullptr};   // point sweeps: (d, f) packed, [7][ld] each
+  float4* pt32[2] = {nullptr, nullptr};  // and in FP32, padded [4][ldp] each
   double* normpart = nullptr; // per tile partial norms [ntiles][15]
   double* norms = nullptr;    // [16]
   double* chunksum = nullptr; // norm sums [nblk * norm_chunks][15]
@@ -264,6 +276,11 @@ struct Sweep32 {
   int nblk;
   int* status;         // bit 4: a box wait gave up
 };
+// sweeps 2..lmx of a small grid (point_sweeps): the first iterate with its
+// increments in pt[0], the final iterate in d_out
+cudaError_t launch_point_sweeps32(const Blk* blks, Space cells, Phys ph, Scheme sc, int eu,
+                                  int lmx, long long ld, const Sweep32& a, const float4* faces,
+                                  float4* const pt[2], float* d_out, cudaStream_t st);
 // sweeps 2..lmx, 2.5D over tl, after launch_coefficients32 has written the
 // first iterate into dpp[0] (lmx = 0: dpp[0] is zeroed); the final iterate
 // in dpp[*cur_out]; ldp: the padded arrays' component stride
@@ -498,14 +515,16 @@ inline cudaError_t launch_accumulate(const Blk* blks, Space sp, const double* G,
 }
 
 // the FP64 implicit coefficients w.coefe, w.coefdiag of the cells (dtpas > 0:
-// dual time stepping) and, when d1 is given, the first Jacobi iterate -u / cd;
+// dual time stepping) and, when d1 is given, the first Jacobi iterate -u / cd
+// (p1: that iterate with its flux increments, packed for the point sweeps);
 // rv_done: w.rv already holds the viscous factor (launch_grad wrote it)
 cudaError_t launch_implicit_coefficients(const Blk* blks, Space cells, Phys ph, int eu,
                                          double dtpas, const double* dt, const double* v,
                                          const double* prim, const double* mu,
                                          const double* mut, const double* sn,
                                          const double* vol, const double* cson,
-                                         const double* u, int rv_done, double* d1, Work& w,
+                                         const double* u, int rv_done, double* d1,
+                                         double2* p1, const double* ps, int qfix, Work& w,
                                          cudaStream_t st);
 
 // The single-precision copies the primitive-velocity kernel writes for the
@@ -537,12 +556,14 @@ cudaError_t launch_defect(const Blk* blks, Space cells, long long ld, const doub
                           const double* ur32, double* corr, cudaStream_t st);
 // the FP32 implicit coefficients (coefe32 per face, coefdiag32 per cell) of
 // the mixed sweeps in one pass over the real cells
-// (the per-cell inputs cq32, cv32 of PrimShadow)
+// (the per-cell inputs cq32, cv32 of PrimShadow); the first iterate in d1, or
+// with its increments in p1
 cudaError_t launch_coefficients32(const Blk* blks, Space cells, int eu, long long ld,
                                   double dtpas, const double* dt, const double* vol,
                                   const float4* cq32, const float2* cv32, const float* sn32,
                                   float* coefe32, float* coefdiag32, float4* snc32,
-                                  const float* u32, float* d1, cudaStream_t st);
+                                  const float* u32, float* d1, float4* p1, const float* st32,
+                                  Phys ph, int qfix, cudaStream_t st);
 // the face lanes of the FP32 sweep's pack: snc[3n + dir].xyz = S/2 of cell n's
 // lower face in dir (exact halves of sn32), .w = 0 until k_coef32 writes it
 cudaError_t launch_pack_faces32(const Blk* blks, int nblk, long long ncells, const float* sn32,

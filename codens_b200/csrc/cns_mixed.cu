@@ -48,6 +48,38 @@ __global__ void __launch_bounds__(kTile) k_defect(const Blk* __restrict__ blks, 
   for (int a = 0; a < 5; ++a) corr[a * ld + n] = u64[a * ld + n] - ur32[a * ld + n];
 }
 
+// the increment (d, f) of a cell, packed as four float4 quads (quad g of cell
+// q at g * np + q)
+struct Inc {
+  float d[5], f[9];
+};
+
+__device__ __forceinline__ void quad_load(const float4* __restrict__ s, long long np, long long q,
+                                          Inc& x) {
+  const float4 a = s[q], b = s[np + q], c = s[2 * np + q], e = s[3 * np + q];
+  x.d[0] = a.x; x.d[1] = a.y; x.d[2] = a.z; x.d[3] = a.w;
+  x.d[4] = b.x; x.f[0] = b.y; x.f[1] = b.z; x.f[2] = b.w;
+  x.f[3] = c.x; x.f[4] = c.y; x.f[5] = c.z; x.f[6] = c.w;
+  x.f[7] = e.x; x.f[8] = e.y;
+}
+
+__device__ __forceinline__ void quad_store(float4* __restrict__ s, long long np, long long q,
+                                           const float d[5], const float f[9]) {
+  s[q] = make_float4(d[0], d[1], d[2], d[3]);
+  s[np + q] = make_float4(d[4], f[0], f[1], f[2]);
+  s[2 * np + q] = make_float4(f[3], f[4], f[5], f[6]);
+  s[3 * np + q] = make_float4(f[7], f[8], 0.f, 0.f);
+}
+
+// the flux increments of the iterate d of the cell at padded index pn
+template <bool EU>
+__device__ __forceinline__ void point_df32(const float* __restrict__ st, long long pld,
+                                           long long pn, float gam1, float pinfl, int qfix,
+                                           const float d[5], float f[9]) {
+  df_diff<float, EU>(d, st[pn], st[pld + pn], st[2 * pld + pn], st[3 * pld + pn],
+                     st[4 * pld + pn], st[5 * pld + pn], gam1, pinfl, qfix, f);
+}
+
 // spectral radius of the face between cells h (upper side) and l, from their
 // packed inputs q = (u, v, w, c) and (vol, rv); rvh, rvl the viscous factors
 // (zero off the real cells, as the reference's zeroed rv)
@@ -74,14 +106,16 @@ __device__ __forceinline__ float face_coef(const float4 qh, const float4 ql, flo
 // cq32 = (u, v, w, c) and cv32 = (vol, rv) the primitive kernel writes.
 // With d1 given, the cell's first Jacobi iterate too: with a zero previous
 // iterate every face term of the first sweep is zero, so d1 = -u / cd, in
-// the padded layout.
+// the padded layout; with p1 given instead (the point sweeps), the iterate
+// and its increments.
 template <bool EU>
 __global__ void __launch_bounds__(kTile) k_coef32(
     const Blk* __restrict__ blks, Space sp, long long ld, double dtpas,
     const double* __restrict__ dt, const double* __restrict__ vol,
     const float4* __restrict__ cq, const float2* __restrict__ cv,
     const float* __restrict__ sn, float* __restrict__ coefe, float* __restrict__ coefdiag,
-    float4* __restrict__ snc, const float* __restrict__ u32, float* __restrict__ d1) {
+    float4* __restrict__ snc, const float* __restrict__ u32, float* __restrict__ d1,
+    float4* __restrict__ p1, const float* __restrict__ st32, float gam1, float pinfl, int qfix) {
   int b, i, j, k;
   if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
@@ -121,10 +155,18 @@ __global__ void __launch_bounds__(kTile) k_coef32(
   }
   if (!EU && dtpas > 0.) cd = cd + (float)(1.5 * vol[n] / dtpas);
   coefdiag[n] = cd;
-  if (d1) {
-    const long long pn = pad_index(B, i, j, k);
+  if (!d1 && !p1) return;
+  const long long pn = pad_index(B, i, j, k);
+  float d[5];
 #pragma unroll
-    for (int a = 0; a < 5; ++a) d1[a * B.pld + pn] = -u32[a * ld + n] / cd;
+  for (int a = 0; a < 5; ++a) d[a] = -u32[a * ld + n] / cd;
+  if (d1) {
+#pragma unroll
+    for (int a = 0; a < 5; ++a) d1[a * B.pld + pn] = d[a];
+  } else {
+    float f[9];
+    point_df32<EU>(st32, B.pld, pn, gam1, pinfl, qfix, d, f);
+    quad_store(p1, B.pld, pn, d, f);
   }
 }
 
@@ -134,16 +176,18 @@ cudaError_t launch_coefficients32(const Blk* blks, Space cells, int eu, long lon
                                   double dtpas, const double* dt, const double* vol,
                                   const float4* cq32, const float2* cv32, const float* sn32,
                                   float* coefe32, float* coefdiag32, float4* snc32,
-                                  const float* u32, float* d1, cudaStream_t st) {
+                                  const float* u32, float* d1, float4* p1, const float* st32,
+                                  Phys ph, int qfix, cudaStream_t st) {
   if (cells.ntiles == 0) return cudaSuccess;
+  const float g1 = (float)ph.gam1, pi = (float)ph.pinfl;
   if (eu)
     k_coef32<true><<<grid_of(cells), kTile, 0, st>>>(blks, cells, ld, dtpas, dt, vol, cq32,
                                                      cv32, sn32, coefe32, coefdiag32, snc32,
-                                                     u32, d1);
+                                                     u32, d1, p1, st32, g1, pi, qfix);
   else
     k_coef32<false><<<grid_of(cells), kTile, 0, st>>>(blks, cells, ld, dtpas, dt, vol, cq32,
                                                       cv32, sn32, coefe32, coefdiag32, snc32,
-                                                      u32, d1);
+                                                      u32, d1, p1, st32, g1, pi, qfix);
   return cudaGetLastError();
 }
 
@@ -262,26 +306,6 @@ cudaError_t launch_accumulate_t<float>(const Blk* blks, Space sp, const float* G
 // ---------------------------------------------------------------------------
 namespace {
 
-struct Inc {
-  float d[5], f[9];
-};
-
-__device__ __forceinline__ void quad_load(const float4* __restrict__ s, int np, int q, Inc& x) {
-  const float4 a = s[q], b = s[np + q], c = s[2 * np + q], e = s[3 * np + q];
-  x.d[0] = a.x; x.d[1] = a.y; x.d[2] = a.z; x.d[3] = a.w;
-  x.d[4] = b.x; x.f[0] = b.y; x.f[1] = b.z; x.f[2] = b.w;
-  x.f[3] = c.x; x.f[4] = c.y; x.f[5] = c.z; x.f[6] = c.w;
-  x.f[7] = e.x; x.f[8] = e.y;
-}
-
-__device__ __forceinline__ void quad_store(float4* __restrict__ s, int np, int q,
-                                           const float d[5], const float f[9]) {
-  s[q] = make_float4(d[0], d[1], d[2], d[3]);
-  s[np + q] = make_float4(d[4], f[0], f[1], f[2]);
-  s[2 * np + q] = make_float4(f[3], f[4], f[5], f[6]);
-  s[3 * np + q] = make_float4(f[7], f[8], 0.f, 0.f);
-}
-
 // acc += Phi(x) . w + ce * d(x)
 __device__ __forceinline__ void phi_acc(const Inc& x, float w0, float w1, float w2, float ce,
                                         float acc[5]) {
@@ -290,6 +314,67 @@ __device__ __forceinline__ void phi_acc(const Inc& x, float w0, float w1, float 
   acc[2] = fmaf(x.f[1], w0, fmaf(x.f[4], w1, fmaf(x.f[5], w2, fmaf(ce, x.d[2], acc[2]))));
   acc[3] = fmaf(x.f[2], w0, fmaf(x.f[5], w1, fmaf(x.f[7], w2, fmaf(ce, x.d[3], acc[3]))));
   acc[4] = fmaf(x.f[3], w0, fmaf(x.f[6], w1, fmaf(x.f[8], w2, fmaf(ce, x.d[4], acc[4]))));
+}
+
+// The point sweep of the FP32 forms (k_jacobi_point in single precision, the
+// sums of the 2.5D sweep below in its order: the same bits): one thread per
+// cell, (d, f) of the cell and its six neighbours as four quads each from the
+// packed iterate, the new iterate and its increment written for the next
+// sweep, or (LAST) the plain iterate for the update.
+template <bool EU, bool LAST>
+__global__ void __launch_bounds__(kTile) k_sweep_point32(
+    const Blk* __restrict__ blks, Space sp, float gam1, float pinfl, int qfix, long long ld,
+    Sweep32 a, const float4* __restrict__ faces, const float4* __restrict__ p_in,
+    float4* __restrict__ p_out, float* __restrict__ d_out) {
+  int b, i, j, k;
+  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  const Blk& B = blks[b];
+  const long long n = cell_index(B, i, j, k), pn = pad_index(B, i, j, k), pld = B.pld;
+  const float4 fi = faces[3 * n], fj = faces[3 * n + 1], fk = faces[3 * n + 2],
+               fiu = faces[3 * (n + 1)], fju = faces[3 * (n + B.nid) + 1],
+               fku = faces[3 * (n + B.nijd) + 2];
+  float acc[5];
+#pragma unroll
+  for (int c = 0; c < 5; ++c) acc[c] = -a.u[c * ld + n];
+  auto load = [&](long long q, bool in, Inc& x) {
+    if (in) {
+      quad_load(p_in, pld, q, x);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 5; ++c) x.d[c] = 0.f;
+#pragma unroll
+      for (int c = 0; c < 9; ++c) x.f[c] = 0.f;
+    }
+  };
+  Inc c0, il, iu, jl, ju, kl, ku;
+  quad_load(p_in, pld, pn, c0);
+  load(pn - 1, i > 1, il);
+  load(pn + 1, i < B.ni - 1, iu);
+  load(pn - B.pid, j > 1, jl);
+  load(pn + B.pid, j < B.nj - 1, ju);
+  load(pn - B.pnijd, k > 1, kl);
+  load(pn + B.pnijd, k < B.nk - 1, ku);
+  phi_acc(c0, (fi.x - fiu.x) + (fj.x - fju.x) + (fk.x - fku.x),
+          (fi.y - fiu.y) + (fj.y - fju.y) + (fk.y - fku.y),
+          (fi.z - fiu.z) + (fj.z - fju.z) + (fk.z - fku.z), 0.f, acc);
+  phi_acc(il, fi.x, fi.y, fi.z, fi.w, acc);
+  phi_acc(iu, -fiu.x, -fiu.y, -fiu.z, fiu.w, acc);
+  phi_acc(jl, fj.x, fj.y, fj.z, fj.w, acc);
+  phi_acc(ju, -fju.x, -fju.y, -fju.z, fju.w, acc);
+  phi_acc(kl, fk.x, fk.y, fk.z, fk.w, acc);
+  phi_acc(ku, -fku.x, -fku.y, -fku.z, fku.w, acc);
+  const float rc = 1.f / a.coefdiag[n];
+  float d[5];
+#pragma unroll
+  for (int c = 0; c < 5; ++c) d[c] = acc[c] * rc;
+  if (LAST) {
+#pragma unroll
+    for (int c = 0; c < 5; ++c) d_out[c * pld + pn] = d[c];
+  } else {
+    float f[9];
+    point_df32<EU>(a.st, pld, pn, gam1, pinfl, qfix, d, f);
+    quad_store(p_out, pld, pn, d, f);
+  }
 }
 
 // The sweep's staged plane: the padded arrays are read as boxes of
@@ -828,6 +913,28 @@ cudaError_t launch_sweeps32(Tiles tl, const Blk* blks, Phys ph, Scheme sc, int e
     cur = 1 - cur;
   }
   *cur_out = cur;
+  return cudaGetLastError();
+}
+
+cudaError_t launch_point_sweeps32(const Blk* blks, Space cells, Phys ph, Scheme sc, int eu,
+                                  int lmx, long long ld, const Sweep32& a, const float4* faces,
+                                  float4* const pt[2], float* d_out, cudaStream_t st) {
+  if (cells.ntiles == 0) return cudaSuccess;
+  const int g = grid_of(cells), q = eu ? sc.qfix_dfez : 0;
+  const float g1 = (float)ph.gam1, pi = (float)ph.pinfl;
+  auto run = [&](auto kernel, const float4* in, float4* out) {
+    kernel<<<g, kTile, 0, st>>>(blks, cells, g1, pi, q, ld, a, faces, in, out, d_out);
+  };
+  for (int ls = 2; ls <= lmx; ++ls) {
+    const float4* in = pt[ls & 1];
+    float4* out = pt[(ls & 1) ^ 1];
+    if (eu)
+      ls < lmx ? run(k_sweep_point32<true, false>, in, out)
+               : run(k_sweep_point32<true, true>, in, out);
+    else
+      ls < lmx ? run(k_sweep_point32<false, false>, in, out)
+               : run(k_sweep_point32<false, true>, in, out);
+  }
   return cudaGetLastError();
 }
 

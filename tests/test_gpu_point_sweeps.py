@@ -1,0 +1,74 @@
+"""The two forms of the Jacobi sweeps: point sweeps (small layouts) and 2.5D
+tiles (larger ones) give the same bits.  Four independent boxes, each small
+enough for point sweeps, together make a layout of 2.5D tiles: every box of
+the batch must end as it does alone, for every patch shape and precision; and
+a box on each side of the line equals the oracle."""
+import numpy as np
+import pytest
+
+from codens_b200 import cases
+
+from ._helpers import assert_equal_bits, oracle_prepared, real
+
+pytestmark = pytest.mark.gpu
+
+POINT_CELLS = 200000
+
+
+def _run(case, nsteps, precision, tiles=None):
+    from codens_b200.solver import CodeNS
+    case.scheme.precision = precision
+    s = CodeNS(case)
+    s.metric()
+    if tiles:
+        s.set_sweep_tiles(precision, *tiles)
+    s.atsch_num(nsteps)
+    v = s.v.cpu().numpy().reshape(5, case.layout.ld)
+    s.close()
+    return v
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("ns", [0, 1])
+def test_point_equals_tiled(cuda, precision, ns):
+    def batch():
+        bt = cases.batch_case(ncase=4, side=(37, 45), seed=6, qfix_dfez=1 - ns)
+        bt.scheme.ns = ns
+        bt.phys.reynz = 1.0e4
+        return bt
+    bt = batch()
+    assert bt.layout.nreal > POINT_CELLS > max(b.nreal for b in bt.layout.blocks)
+    alone = []
+    for ib in range(4):
+        m = cases.batch_member(bt, ib)
+        alone.append(_run(m, 3, precision)[:, m.layout.blocks[0].real_cells()])
+    for tiles in ((32, 4, 3), (32, 8, 16), (16, 8, 5), (16, 16, 64)):
+        v = _run(batch(), 3, precision, tiles)
+        for ib, want in enumerate(alone):
+            assert_equal_bits(v[:, bt.layout.blocks[ib].real_cells()], want, f"{tiles} box {ib}")
+
+
+# 200000 cells is the last point-sweep size; odd sides, one-cell directions
+@pytest.mark.parametrize("cells", [(50, 50, 80), (67, 53, 57), (129, 2, 3), (1, 33, 5)])
+@pytest.mark.parametrize("ns", [0, 1])
+def test_fused_step_bits_at_the_line(cuda, cells, ns):
+    case = cases.box_case(cells, seed=7, ns=bool(ns), skew=0.01, reynz=1.0e4,
+                          qfix_dfez=1 - ns, lmax=4)
+    orc, st = oracle_prepared(case)
+    for _ in range(2):
+        orc.step(st)
+    rc = real(case)
+    v = _run(case, 2, 0)
+    assert_equal_bits(v[:, rc], np.asarray(st.v).reshape(-1, case.layout.ld)[:5, rc], "state")
+
+
+@pytest.mark.parametrize("lmax", [0, 1, 2, 3])
+def test_few_sweeps(cuda, lmax):
+    case = cases.box_case((9, 7, 5), seed=8, ns=True, skew=0.02, lmax=lmax, reynz=1.0e3)
+    orc, st = oracle_prepared(case)
+    for _ in range(2):
+        orc.step(st)
+    rc = real(case)
+    v = _run(case, 2, 0)
+    assert_equal_bits(v[:, rc], np.asarray(st.v).reshape(-1, case.layout.ld)[:5, rc], "state")
+    assert np.isfinite(_run(case, 2, 1)[:, rc]).all()
