@@ -159,6 +159,53 @@ __device__ __forceinline__ bool space_elem(const Space& sp, int lane, int& b, in
   return space_elem_at(sp, blockIdx.x, lane, b, i, j, k);
 }
 
+// Programmatic dependent launch.  Every kernel launched through pdl() executes
+// pdl_sync() in every thread before it touches memory another kernel writes
+// (the index tables are constant): the next kernel may start its CTAs now, and
+// this one goes on when the kernel before it has completed and its writes are
+// visible.  Launch latency and the index arithmetic of a kernel then overlap
+// the tail of the one before: an iteration of 16x12x8 Euler cells takes 84 ->
+// 77 us, 64x32x32 cells 131 -> 120 (Euler) and 135 -> 118 (Jameson, mixed),
+// a 0.43M-cell HLLC channel 519 -> 503.
+__device__ __forceinline__ void pdl_sync() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// space_elem, then pdl_sync in every thread
+__device__ __forceinline__ bool space_elem_sync(const Space& sp, int lane, int& b, int& i, int& j,
+                                                int& k) {
+  const bool in = space_elem(sp, lane, b, i, j, k);
+  pdl_sync();
+  return in;
+}
+
+template <class... P>
+struct PdlLaunch {
+  void (*kernel)(P...);
+  cudaLaunchConfig_t cfg;
+  template <class... A>
+  void operator()(A&&... args) {  // errors: cudaGetLastError, as after <<< >>>
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  }
+};
+
+// kernel<<<grid, block, smem, st>>> with programmatic serialization
+template <class... P>
+PdlLaunch<P...> pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st) {
+  PdlLaunch<P...> l{kernel, {}};
+  l.cfg.gridDim = grid;
+  l.cfg.blockDim = block;
+  l.cfg.dynamicSmemBytes = smem;
+  l.cfg.stream = st;
+  return l;
+}
+
 __device__ __forceinline__ long long cell_index(const Blk& B, int i, int j, int k) {
   return B.npc + (long long)i + (long long)j * B.nid + (long long)k * B.nijd;
 }

@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(kTile) k_zpres(const Blk* __restrict__ blks,
                                                  double* temp, double* cson,
                                                  double* mu, int* status) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const long long n = cell_index(blks[b], i, j, k);
   double m;
   (void)zpres_cell(ph, with_mu, v, ld, n, ps, temp, cson, mu, status, &m);
@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(kTile) k_zvismo(const Blk* __restrict__ blks,
                                                   const double* __restrict__ temp,
                                                   int* status) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const long long n = cell_index(blks[b], i, j, k);
   const double t = temp[n];
   if (t <= 0.) {
@@ -101,6 +101,7 @@ __global__ void __launch_bounds__(256) k_prim(long long n0, long long n1,
                                              const double* __restrict__ v,
                                              long long ld, double* __restrict__ prim,
                                              const double* __restrict__ ps, PrimShadow sh) {
+  pdl_sync();
   const long long n = n0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= n1) return;
   const double r = v[n];
@@ -200,7 +201,7 @@ __global__ void __launch_bounds__(kTile) k_chronos(
     const double* __restrict__ sn, const double* __restrict__ vol,
     const double* __restrict__ cson) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const long long nc = cell_index(B, i, j, k);
   dt[nc] = chronos_cell(B, ph, sc, t, ld, nc, sn, vol, cson[nc], sc.ns ? mu[nc] : 0.,
@@ -216,7 +217,7 @@ __global__ void __launch_bounds__(kTile) k_zpres_chronos(
     const double* __restrict__ mut, double* dt, const double* __restrict__ sn,
     const double* __restrict__ vol, int* status) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const long long n = cell_index(B, i, j, k);
   double m = 0.;
@@ -234,7 +235,12 @@ __global__ void __launch_bounds__(kTile) k_zpres_chronos(
 // ghost cell depends on interior cells only, so one pass gives the same values.
 __global__ void __launch_bounds__(256) k_rbord(Bnd bd, Phys ph, double* v,
                                               long long ld, double* ps,
-                                              double* temp, double* cson) {
+                                              double* temp, double* cson,
+                                              unsigned* masks) {
+  pdl_sync();
+  // the injection boundaries' sweep masks start empty (k_clidd_mask follows)
+  if (blockIdx.x == 0)
+    for (int q = threadIdx.x; q < bd.nbnd; q += blockDim.x) masks[q] = 0u;
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= bd.nlist) return;
   const int bb = bd.ent_bnd[e];
@@ -352,6 +358,7 @@ __device__ __forceinline__ double idd_sweep(const Phys& ph, IddCell& c) {
 __global__ void __launch_bounds__(256) k_clidd_mask(Bnd bd, Phys ph, const long long* ents,
                                                    long long nent, const double* v,
                                                    long long ld, unsigned* masks) {
+  pdl_sync();
   const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= nent) return;
   const long long e = ents[q];
@@ -369,6 +376,7 @@ __global__ void __launch_bounds__(256) k_clidd_apply(Bnd bd, Phys ph, const long
                                                     long long nent, double* v, long long ld,
                                                     double* ps_, double* temp, double* cson,
                                                     const unsigned* masks) {
+  pdl_sync();
   const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= nent) return;
   const long long e = ents[q], nl = bd.nlist, nc = bd.ncbd[e];
@@ -411,6 +419,7 @@ __global__ void __launch_bounds__(256) k_clidd_apply(Bnd bd, Phys ph, const long
 // rbte.f90:15-31 (non-coincident boundaries: copy of the interior cell) and
 // rbtc.f90:30-100 (coincident: average with the rotated partner)
 __global__ void __launch_bounds__(256) k_tau_ghosts(Bnd bd, double* tau, long long ld) {
+  pdl_sync();
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= bd.nlist) return;
   const int bb = bd.ent_bnd[e];
@@ -455,7 +464,7 @@ __global__ void __launch_bounds__(kTile) k_grad(const Blk* __restrict__ blks,
                                                 const double* __restrict__ temp,
                                                 double* __restrict__ rv) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const long long n = cell_index(B, i, j, k);
   double g[12];
@@ -536,7 +545,7 @@ __global__ void __launch_bounds__(kTile) k_impl_rv(const Blk* __restrict__ blks,
                                                    const double* __restrict__ mu,
                                                    const double* __restrict__ mut, double* rv) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const long long n = cell_index(blks[b], i, j, k);
   rv[n] = ph.gam * (mu[n] / ph.pr + mut[n] / ph.prt) / v[n];
 }
@@ -640,7 +649,7 @@ __global__ void __launch_bounds__(kTile) k_impl_coefs(
     double* __restrict__ d1, double2* __restrict__ p1, const double* __restrict__ ps, Phys ph,
     int qfix) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const long long n = cell_index(B, i, j, k);
   double q0[6];
@@ -706,7 +715,7 @@ __global__ void __launch_bounds__(kTile) k_jacobi_point(
     const double* __restrict__ coefdiag, const double2* __restrict__ p_in,
     double2* __restrict__ p_out, double* __restrict__ d_out) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const long long n = cell_index(B, i, j, k);
   double d0[5], f0[9], w[5];
@@ -752,7 +761,7 @@ __global__ void __launch_bounds__(kTile) k_norm_partials(
     const double* __restrict__ u0, const double* __restrict__ v,
     const double* __restrict__ dt, double* normpart) {
   int b, i, j, k;
-  const bool valid = space_elem(sp, threadIdx.x, b, i, j, k);
+  const bool valid = space_elem_sync(sp, threadIdx.x, b, i, j, k);
   double res[5] = {0., 0., 0., 0., 0.};
   if (valid) {
     const long long n = cell_index(blks[b], i, j, k);
@@ -791,6 +800,7 @@ __global__ void __launch_bounds__(kNormRows * 15) k_norms(
     const Blk* __restrict__ blks, const int* __restrict__ blk_tile0,
     const double* __restrict__ normpart, double* __restrict__ chunksum, int* counter,
     double* norms) {
+  pdl_sync();
   __shared__ double red[kNormRows][15];
   __shared__ int last;
   const int q = threadIdx.x % 15, row = threadIdx.x / 15;
@@ -849,7 +859,7 @@ cudaError_t launch_zpres(const Blk* blks, Space sp, Phys ph, int with_mu,
                          const double* v, long long ld, double* ps, double* temp,
                          double* cson, double* mu, int* status, cudaStream_t st) {
   if (sp.ntiles > 0)
-    k_zpres<<<grid_of(sp), kTile, 0, st>>>(blks, sp, ph, with_mu, v, ld, ps, temp,
+    pdl(k_zpres, grid_of(sp), kTile, 0, st)(blks, sp, ph, with_mu, v, ld, ps, temp,
                                            cson, mu, status);
   return cudaGetLastError();
 }
@@ -857,14 +867,14 @@ cudaError_t launch_zpres(const Blk* blks, Space sp, Phys ph, int with_mu,
 cudaError_t launch_zvismo(const Blk* blks, Space sp, Phys ph, double* mu,
                           const double* temp, int* status, cudaStream_t st) {
   if (sp.ntiles > 0)
-    k_zvismo<<<grid_of(sp), kTile, 0, st>>>(blks, sp, ph, mu, temp, status);
+    pdl(k_zvismo, grid_of(sp), kTile, 0, st)(blks, sp, ph, mu, temp, status);
   return cudaGetLastError();
 }
 
 cudaError_t launch_prim(long long n0, long long n1, const double* v, long long ld,
                         double* prim, cudaStream_t st) {
   if (n1 > n0)
-    k_prim<false><<<(int)((n1 - n0 + 255) / 256), 256, 0, st>>>(n0, n1, v, ld, prim, nullptr,
+    pdl(k_prim<false>, (int)((n1 - n0 + 255) / 256), 256, 0, st)(n0, n1, v, ld, prim, nullptr,
                                                                 PrimShadow{});
   return cudaGetLastError();
 }
@@ -872,7 +882,7 @@ cudaError_t launch_prim(long long n0, long long n1, const double* v, long long l
 cudaError_t launch_prim_shadow(long long ncells, const double* v, long long ld, double* prim,
                                const double* ps, const PrimShadow& sh, cudaStream_t st) {
   if (ncells > 0)
-    k_prim<true><<<(int)((ncells + 255) / 256), 256, 0, st>>>(0, ncells, v, ld, prim, ps, sh);
+    pdl(k_prim<true>, (int)((ncells + 255) / 256), 256, 0, st)(0, ncells, v, ld, prim, ps, sh);
   return cudaGetLastError();
 }
 
@@ -882,6 +892,7 @@ cudaError_t launch_prim_shadow(long long ncells, const double* v, long long ld, 
 __global__ void __launch_bounds__(kTile) k_dt_partials(const Blk* __restrict__ blks, Space sp,
                                                        const double* __restrict__ dt,
                                                        double* __restrict__ part) {
+  pdl_sync();
   int b, i, j, k;
   double x = CUDART_INF;
   if (space_elem(sp, threadIdx.x, b, i, j, k)) x = dt[cell_index(blks[b], i, j, k)];
@@ -900,6 +911,7 @@ __global__ void __launch_bounds__(kTile) k_dt_partials(const Blk* __restrict__ b
 __global__ void __launch_bounds__(256) k_dt_reduce(const double* __restrict__ part, int n,
                                                   double dt1min, double* __restrict__ out,
                                                   int* status) {
+  pdl_sync();
   double x = CUDART_INF;
   for (int q = threadIdx.x; q < n; q += blockDim.x) x = fmin(x, part[q]);
 #pragma unroll
@@ -918,6 +930,7 @@ __global__ void __launch_bounds__(256) k_dt_reduce(const double* __restrict__ pa
 
 __global__ void __launch_bounds__(256) k_dt_set(long long ncells, const double* __restrict__ v,
                                                double* __restrict__ dt) {
+  pdl_sync();
   const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (n < ncells) dt[n] = *v;
 }
@@ -927,7 +940,7 @@ cudaError_t launch_chronos(const Blk* blks, Space sp, Phys ph, Scheme sc,
                            long long ld, double* dt, const double* sn,
                            const double* vol, const double* cson, cudaStream_t st) {
   if (sp.ntiles > 0)
-    k_chronos<<<grid_of(sp), kTile, 0, st>>>(blks, sp, ph, sc, mu, mut, v, ld, dt,
+    pdl(k_chronos, grid_of(sp), kTile, 0, st)(blks, sp, ph, sc, mu, mut, v, ld, dt,
                                              sn, vol, cson);
   return cudaGetLastError();
 }
@@ -938,7 +951,7 @@ cudaError_t launch_zpres_chronos(const Blk* blks, Space sp, Phys ph, Scheme sc,
                                  const double* sn, const double* vol, int* status,
                                  cudaStream_t st) {
   if (sp.ntiles > 0)
-    k_zpres_chronos<<<grid_of(sp), kTile, 0, st>>>(blks, sp, ph, sc, v, ld, ps, temp, cson, mu,
+    pdl(k_zpres_chronos, grid_of(sp), kTile, 0, st)(blks, sp, ph, sc, v, ld, ps, temp, cson, mu,
                                                    mut, dt, sn, vol, status);
   return cudaGetLastError();
 }
@@ -947,9 +960,9 @@ cudaError_t launch_dt_global(const Blk* blks, Space cells, long long ncells, dou
                              double* dt, double* part, double* scalar, int* status,
                              cudaStream_t st) {
   if (cells.ntiles == 0) return cudaSuccess;
-  k_dt_partials<<<grid_of(cells), kTile, 0, st>>>(blks, cells, dt, part);
-  k_dt_reduce<<<1, 256, 0, st>>>(part, cells.ntiles, dt1min, scalar, status);
-  k_dt_set<<<(int)((ncells + 255) / 256), 256, 0, st>>>(ncells, scalar, dt);
+  pdl(k_dt_partials, grid_of(cells), kTile, 0, st)(blks, cells, dt, part);
+  pdl(k_dt_reduce, 1, 256, 0, st)(part, cells.ntiles, dt1min, scalar, status);
+  pdl(k_dt_set, (int)((ncells + 255) / 256), 256, 0, st)(ncells, scalar, dt);
   return cudaGetLastError();
 }
 
@@ -957,13 +970,11 @@ cudaError_t launch_rbord(const Bnd& bd, Phys ph, double* v, long long ld,
                          double* ps, double* temp, double* cson, long long n_idd_ent,
                          const long long* idd_ents, unsigned* masks, cudaStream_t st) {
   if (bd.nlist > 0)
-    k_rbord<<<(int)((bd.nlist + 255) / 256), 256, 0, st>>>(bd, ph, v, ld, ps, temp, cson);
+    pdl(k_rbord, (int)((bd.nlist + 255) / 256), 256, 0, st)(bd, ph, v, ld, ps, temp, cson, masks);
   if (n_idd_ent > 0) {
-    cudaError_t e = cudaMemsetAsync(masks, 0, sizeof(unsigned) * bd.nbnd, st);
-    if (e != cudaSuccess) return e;
     const int g = (int)((n_idd_ent + 255) / 256);
-    k_clidd_mask<<<g, 256, 0, st>>>(bd, ph, idd_ents, n_idd_ent, v, ld, masks);
-    k_clidd_apply<<<g, 256, 0, st>>>(bd, ph, idd_ents, n_idd_ent, v, ld, ps, temp, cson,
+    pdl(k_clidd_mask, g, 256, 0, st)(bd, ph, idd_ents, n_idd_ent, v, ld, masks);
+    pdl(k_clidd_apply, g, 256, 0, st)(bd, ph, idd_ents, n_idd_ent, v, ld, ps, temp, cson,
                                      masks);
   }
   return cudaGetLastError();
@@ -972,7 +983,7 @@ cudaError_t launch_rbord(const Bnd& bd, Phys ph, double* v, long long ld,
 cudaError_t launch_tau_ghosts(const Bnd& bd, double* tau, long long ld,
                               cudaStream_t st) {
   if (bd.nlist > 0)
-    k_tau_ghosts<<<(int)((bd.nlist + 255) / 256), 256, 0, st>>>(bd, tau, ld);
+    pdl(k_tau_ghosts, (int)((bd.nlist + 255) / 256), 256, 0, st)(bd, tau, ld);
   return cudaGetLastError();
 }
 
@@ -982,7 +993,7 @@ cudaError_t launch_grad(const Blk* blks, Space sp, Phys ph, const double* v,
                         const double* vol, const double* temp, double* rv,
                         cudaStream_t st) {
   if (sp.ntiles > 0)
-    k_grad<<<grid_of(sp), kTile, 0, st>>>(blks, sp, ph, v, prim, ld, mu, mut, tau, sn,
+    pdl(k_grad, grid_of(sp), kTile, 0, st)(blks, sp, ph, v, prim, ld, mu, mut, tau, sn,
                                           vol, temp, rv);
   return cudaGetLastError();
 }
@@ -1017,7 +1028,7 @@ cudaError_t launch_accumulate_t<double>(const Blk* blks, Space sp, const double*
                                         long long ld, const double* corr, double* u,
                                         float* u32, cudaStream_t st, const double* V) {
   if (sp.ntiles > 0)
-    k_accumulate<double><<<grid_of(sp), kTile, 0, st>>>(blks, sp, G, ld, corr, u, u32, V);
+    pdl(k_accumulate<double>, grid_of(sp), kTile, 0, st)(blks, sp, G, ld, corr, u, u32, V);
   return cudaGetLastError();
 }
 
@@ -1068,7 +1079,7 @@ cudaError_t launch_update_t<double>(const Blk* blks, Space cells, long long ld,
                                     const double* d, double* v, const double* dt,
                                     double* d_out, double* normpart, cudaStream_t st) {
   if (cells.ntiles > 0)
-    k_update<double><<<grid_of(cells), kTile, 0, st>>>(blks, cells, ld, d, v, dt, d_out,
+    pdl(k_update<double>, grid_of(cells), kTile, 0, st)(blks, cells, ld, d, v, dt, d_out,
                                                        normpart);
   return cudaGetLastError();
 }
@@ -1084,12 +1095,12 @@ cudaError_t launch_implicit_coefficients(const Blk* blks, Space cells, Phys ph, 
   if (cells.ntiles == 0) return cudaSuccess;
   const int g = grid_of(cells);
   if (eu) {
-    k_impl_coefs<true><<<g, kTile, 0, st>>>(blks, cells, dtpas, v, prim, w.ld, sn, vol, cson,
+    pdl(k_impl_coefs<true>, g, kTile, 0, st)(blks, cells, dtpas, v, prim, w.ld, sn, vol, cson,
                                             nullptr, dt, u, w.coefe, w.coefdiag, d1, p1, ps, ph,
                                             qfix);
   } else {
-    if (!rv_done) k_impl_rv<<<g, kTile, 0, st>>>(blks, cells, ph, v, mu, mut, w.rv);
-    k_impl_coefs<false><<<g, kTile, 0, st>>>(blks, cells, dtpas, v, prim, w.ld, sn, vol, cson,
+    if (!rv_done) pdl(k_impl_rv, g, kTile, 0, st)(blks, cells, ph, v, mu, mut, w.rv);
+    pdl(k_impl_coefs<false>, g, kTile, 0, st)(blks, cells, dtpas, v, prim, w.ld, sn, vol, cson,
                                              w.rv, dt, u, w.coefe, w.coefdiag, d1, p1, ps, ph,
                                              qfix);
   }
@@ -1103,7 +1114,7 @@ static cudaError_t point_sweeps64(const Blk* blks, Space cells, Phys ph, int qfi
                                   const double* sn, Work& w, cudaStream_t st) {
   const int g = grid_of(cells);
   auto run = [&](auto kernel, const double2* in, double2* out) {
-    kernel<<<g, kTile, 0, st>>>(blks, cells, ph, qfix, w.ld, u, v, w.prim, ps, sn, w.coefe,
+    pdl(kernel, g, kTile, 0, st)(blks, cells, ph, qfix, w.ld, u, v, w.prim, ps, sn, w.coefe,
                                 w.coefdiag, in, out, w.dpp[0]);
   };
   for (int ls = 2; ls <= lmx; ++ls) {
@@ -1156,7 +1167,7 @@ __global__ void __launch_bounds__(kTile) k_dual(const Blk* __restrict__ blks, Sp
                                                 const double* __restrict__ ptdual,
                                                 double* __restrict__ u, float* __restrict__ u32) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const long long n = cell_index(blks[b], i, j, k);
   const double c0 = vol[n] * dti;
 #pragma unroll
@@ -1178,7 +1189,7 @@ __global__ void __launch_bounds__(kTile) k_dual_update(const Blk* __restrict__ b
                                                        double* ptdual, double* vdual,
                                                        double* vdual1, double* vdual2) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const long long n = cell_index(blks[b], i, j, k);
   const double c13 = 1. / 3.;
 #pragma unroll
@@ -1206,7 +1217,7 @@ cudaError_t launch_dual(const Blk* blks, Space cells, long long ld, double fact,
                         const double* v, const double* vol, const double* ptdual, double* u,
                         float* u32, cudaStream_t st) {
   if (cells.ntiles > 0)
-    k_dual<<<cells.ntiles, kTile, 0, st>>>(blks, cells, ld, fact, dti, v, vol, ptdual, u, u32);
+    pdl(k_dual, cells.ntiles, kTile, 0, st)(blks, cells, ld, fact, dti, v, vol, ptdual, u, u32);
   return cudaGetLastError();
 }
 
@@ -1214,7 +1225,7 @@ cudaError_t launch_dual_update(const Blk* blks, Space cells, long long ld, int m
                                const double* v, double* ptdual, double* vdual, double* vdual1,
                                double* vdual2, cudaStream_t st) {
   if (cells.ntiles > 0)
-    k_dual_update<<<cells.ntiles, kTile, 0, st>>>(blks, cells, ld, mode, v, ptdual, vdual,
+    pdl(k_dual_update, cells.ntiles, kTile, 0, st)(blks, cells, ld, mode, v, ptdual, vdual,
                                                   vdual1, vdual2);
   return cudaGetLastError();
 }
@@ -1224,14 +1235,14 @@ cudaError_t launch_norm_partials(const Blk* blks, Space cells, long long ld,
                                  const double* dt, double* normpart,
                                  cudaStream_t st) {
   if (cells.ntiles > 0)
-    k_norm_partials<<<cells.ntiles, kTile, 0, st>>>(blks, cells, ld, u0, v, dt, normpart);
+    pdl(k_norm_partials, cells.ntiles, kTile, 0, st)(blks, cells, ld, u0, v, dt, normpart);
   return cudaGetLastError();
 }
 
 cudaError_t launch_norm_finalize(const Blk* blks, const int* blk_tile0_dev, int nblk, int chunks,
                                  const double* normpart, double* chunksum, int* counter,
                                  double* norms, cudaStream_t st) {
-  k_norms<<<dim3(chunks, nblk), kNormRows * 15, 0, st>>>(blks, blk_tile0_dev, normpart, chunksum,
+  pdl(k_norms, dim3(chunks, nblk), kNormRows * 15, 0, st)(blks, blk_tile0_dev, normpart, chunksum,
                                                          counter, norms);
   return cudaGetLastError();
 }

@@ -62,6 +62,7 @@ __global__ void __launch_bounds__(kRatioCta) k_ratio(const Blk* __restrict__ blk
                                                      const T* __restrict__ prim, long long ld,
                                                      const T* __restrict__ ps,
                                                      T* __restrict__ R) {
+  pdl_sync();
   constexpr int kSub = kTile / kRatioCta, U = kRatioChunk;
   const int dir = blockIdx.x % 3, sub = blockIdx.x / 3;
   const Space sp = sp3.at(dir);
@@ -116,7 +117,7 @@ cudaError_t ratio_launch(const Blk* blks, const SpaceBuf* lines, int l0, const T
                          const T* prim, long long ld, const T* ps, T* R, cudaStream_t st) {
   const Space3 sp{{lines[0].view(l0), lines[1].view(l0), lines[2].view(l0)}};
   const int g = sp.grid() * (kTile / kRatioCta);
-  if (g > 0) k_ratio<T><<<dim3(g, 5), kRatioCta, 0, st>>>(blks, sp, v, prim, ld, ps, R);
+  if (g > 0) pdl(k_ratio<T>, dim3(g, 5), kRatioCta, 0, st)(blks, sp, v, prim, ld, ps, R);
   return cudaGetLastError();
 }
 
@@ -748,6 +749,7 @@ __global__ void __launch_bounds__(kTile, FL == kFluxRoe ? 4 : 5) k_face_flux(
     const T* __restrict__ v, const T* __restrict__ prim, long long ld,
     const T* __restrict__ ps, const T* __restrict__ tau, const T* __restrict__ sn,
     const T* __restrict__ R, T* __restrict__ G, T* __restrict__ V = nullptr) {
+  pdl_sync();
   const int dir = blockIdx.x % 3, tile = blockIdx.x / 3;
   const Space sp = sp3.at(dir);
   int b, i, j, k;
@@ -789,6 +791,7 @@ __global__ void __launch_bounds__(TI * TJ, MINB) k_residual_25d(
     const T* __restrict__ prim, long long ld, const T* __restrict__ ps,
     const T* __restrict__ tau, const T* __restrict__ sn, const T* __restrict__ R,
     double* __restrict__ u, float* __restrict__ u32) {
+  pdl_sync();
   constexpr int NT = TI * TJ, NFI = (TI + 1) * TJ, NFJ = TI * (TJ + 1);
   constexpr int NF = NFI + NFJ + 2 * NT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -886,7 +889,7 @@ cudaError_t residual_fused_shape(const Blk* blks, Tiles tl, Phys ph, Scheme sc, 
                                  const T* sn, const T* R, double* u, float* u32,
                                  cudaStream_t st) {
   constexpr size_t sm = sizeof(T) * 5 * residual_smem_faces<TI, TJ>();
-  k_residual_25d<T, NS, FL, TI, TJ, MINB><<<tl.ntiles, TI * TJ, sm, st>>>(
+  pdl(k_residual_25d<T, NS, FL, TI, TJ, MINB>, tl.ntiles, TI * TJ, sm, st)(
       blks, tl, ph, sc, v, prim, ld, ps, tau, sn, R, u, u32);
   return cudaGetLastError();
 }
@@ -939,23 +942,21 @@ static inline cudaError_t face_flux_dispatch(const Blk* blks, const SpaceBuf* fa
   const int g = sp.grid();
   if (g == 0) return cudaSuccess;
   if (sc.ischema == 14 && sc.ns)
-    k_face_flux<double, true, kFluxHllc><<<g, kTile, 0, st>>>(blks, sp, ph, sc, v, prim, ld, ps,
+    pdl(k_face_flux<double, true, kFluxHllc>, g, kTile, 0, st)(blks, sp, ph, sc, v, prim, ld, ps,
                                                              tau, sn, R, G, V);
   else if (sc.ischema == 14)
-    k_face_flux<double, false, kFluxHllc><<<g, kTile, 0, st>>>(blks, sp, ph, sc, v, prim, ld, ps,
-                                                              tau, sn, R, G);
+    pdl(k_face_flux<double, false, kFluxHllc>, g, kTile, 0, st)(blks, sp, ph, sc, v, prim, ld, ps,
+                                                              tau, sn, R, G, V);
   else if (sc.ischema == 9)
-    k_face_flux<double, true, kFluxRusanov><<<g, kTile, 0, st>>>(blks, sp, ph, sc, v, prim, ld,
-                                                                ps, tau, sn, R, G);
+    pdl(k_face_flux<double, true, kFluxRusanov>, g, kTile, 0, st)(blks, sp, ph, sc, v, prim, ld,
+                                                                ps, tau, sn, R, G, V);
   else if (sc.ischema == 5)
-    k_face_flux<double, true, kFluxAusm><<<g, kTile, 0, st>>>(blks, sp, ph, sc, v, prim, ld, ps,
-                                                             tau, sn, R, G);
+    pdl(k_face_flux<double, true, kFluxAusm>, g, kTile, 0, st)(blks, sp, ph, sc, v, prim, ld, ps,
+                                                             tau, sn, R, G, V);
   else if (sc.ns)
-    k_face_flux<double, true><<<g, kTile, 0, st>>>(blks, sp, ph, sc, v, prim, ld, ps, tau, sn, R,
-                                                   G);
+    pdl(k_face_flux<double, true>, g, kTile, 0, st)(blks, sp, ph, sc, v, prim, ld, ps, tau, sn, R, G, V);
   else
-    k_face_flux<double, false><<<g, kTile, 0, st>>>(blks, sp, ph, sc, v, prim, ld, ps, tau, sn, R,
-                                                    G);
+    pdl(k_face_flux<double, false>, g, kTile, 0, st)(blks, sp, ph, sc, v, prim, ld, ps, tau, sn, R, G, V);
   return cudaGetLastError();
 }
 
@@ -973,7 +974,7 @@ __global__ void __launch_bounds__(kTile) k_accumulate(const Blk* __restrict__ bl
                                                       float* __restrict__ u32,
                                                       const T* __restrict__ V = nullptr) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const long long n = cell_index(B, i, j, k);
   double acc[5] = {0., 0., 0., 0., 0.};
@@ -1280,6 +1281,7 @@ __global__ void __launch_bounds__(TI * TJ, TI * TJ <= 128 ? 3 : 1) k_jacobi_25d(
     const T* __restrict__ u, const T* __restrict__ v, const T* __restrict__ prim,
     const T* __restrict__ ps, const T* __restrict__ sn, const T* __restrict__ coefe,
     const T* __restrict__ coefdiag, const T* __restrict__ d_in, T* __restrict__ d_out) {
+  pdl_sync();
   constexpr int NX = TI + 2, NY = TJ + 2, NP = NX * NY, NT = TI * TJ;
   constexpr int NR = raw_count<FORM>(EU);
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1533,12 +1535,10 @@ cudaError_t jacobi_25d_shape(const Blk* blks, Tiles tl, Phys ph, int qfix, int e
                              const T* sn, const T* coefe, const T* coefdiag, const T* d_in,
                              T* d_out, cudaStream_t st) {
   if (eu)
-    k_jacobi_25d<T, true, FORM, TI, TJ>
-        <<<tl.ntiles, TI * TJ, jacobi_25d_smem<TI, TJ, T, FORM, true>(), st>>>(
+    pdl(k_jacobi_25d<T, true, FORM, TI, TJ>, tl.ntiles, TI * TJ, jacobi_25d_smem<TI, TJ, T, FORM, true>(), st)(
             blks, tl, ph, qfix, ld, u, v, prim, ps, sn, coefe, coefdiag, d_in, d_out);
   else
-    k_jacobi_25d<T, false, FORM, TI, TJ>
-        <<<tl.ntiles, TI * TJ, jacobi_25d_smem<TI, TJ, T, FORM, false>(), st>>>(
+    pdl(k_jacobi_25d<T, false, FORM, TI, TJ>, tl.ntiles, TI * TJ, jacobi_25d_smem<TI, TJ, T, FORM, false>(), st)(
             blks, tl, ph, qfix, ld, u, v, prim, ps, sn, coefe, coefdiag, d_in, d_out);
   return cudaGetLastError();
 }
@@ -1631,7 +1631,7 @@ __global__ void __launch_bounds__(kTile) k_update(const Blk* __restrict__ blks,
                                                   const double* __restrict__ dt,
                                                   double* d_out, double* normpart) {
   int b, i, j, k;
-  const bool valid = space_elem(sp, threadIdx.x, b, i, j, k);
+  const bool valid = space_elem_sync(sp, threadIdx.x, b, i, j, k);
   double res[5] = {0., 0., 0., 0., 0.};
   if (valid) {
     const Blk& B = blks[b];

@@ -25,6 +25,7 @@ inline int grid_of(const Space& s) { return s.ntiles; }
 __global__ void __launch_bounds__(256) k_ghost_refresh(Bnd bd, int mode, double* v,
                                                       long long ld, double* ps, double* temp,
                                                       double* cson) {
+  pdl_sync();
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= bd.nlist) return;
   const int bb = bd.ent_bnd[e];
@@ -70,7 +71,7 @@ __global__ void __launch_bounds__(kTile) k_dissip_face(const Blk* __restrict__ b
                                                        const double* __restrict__ sn,
                                                        double* __restrict__ G) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const double ck2 = B.ki2, ck4 = B.ki4;  // ki2(lm), ki4(lm)
   const long long n = cell_index(B, i, j, k);
@@ -154,7 +155,7 @@ __global__ void __launch_bounds__(kTile) k_jam_face(const Blk* __restrict__ blks
                                                     const double* __restrict__ sn,
                                                     double* __restrict__ G) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const long long n = cell_index(B, i, j, k);
   const long long inc = ninc_of(B, dir);
@@ -197,7 +198,7 @@ __global__ void __launch_bounds__(kTile) k_jam_accumulate(const Blk* __restrict_
                                                           double* __restrict__ out,
                                                           float* __restrict__ out32) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const long long n = cell_index(B, i, j, k);
   double acc[5] = {0., 0., 0., 0., 0.};
@@ -233,7 +234,7 @@ __global__ void __launch_bounds__(kTile) k_jam_accumulate(const Blk* __restrict_
 cudaError_t launch_ghost_refresh(const Bnd& bd, int mode, double* v, long long ld, double* ps,
                                  double* temp, double* cson, cudaStream_t st) {
   if (bd.nlist > 0)
-    k_ghost_refresh<<<(int)((bd.nlist + 255) / 256), 256, 0, st>>>(bd, mode, v, ld, ps, temp,
+    pdl(k_ghost_refresh, (int)((bd.nlist + 255) / 256), 256, 0, st)(bd, mode, v, ld, ps, temp,
                                                                   cson);
   return cudaGetLastError();
 }
@@ -245,11 +246,11 @@ cudaError_t launch_dissip_jameson(const Blk* blks, const SpaceBuf* faces, Space 
   for (int dir = 0; dir < 3; ++dir) {
     const Space sp = faces[dir].view(l0);
     if (sp.ntiles > 0)
-      k_dissip_face<<<grid_of(sp), kTile, 0, st>>>(blks, sp, dir, v, ld, ps, cson,
+      pdl(k_dissip_face, grid_of(sp), kTile, 0, st)(blks, sp, dir, v, ld, ps, cson,
                                                    sn, G);
   }
   if (cells.ntiles > 0)
-    k_jam_accumulate<<<grid_of(cells), kTile, 0, st>>>(blks, cells, G, ld, nullptr, d,
+    pdl(k_jam_accumulate, grid_of(cells), kTile, 0, st)(blks, cells, G, ld, nullptr, d,
                                                        nullptr);
   return cudaGetLastError();
 }
@@ -263,14 +264,14 @@ cudaError_t launch_sch_jameson(const Blk* blks, const SpaceBuf* faces, Space cel
     const Space sp = faces[dir].view(l0);
     if (sp.ntiles == 0) continue;
     if (ns)
-      k_jam_face<true><<<grid_of(sp), kTile, 0, st>>>(blks, sp, dir, pinfl, v, ld, ps, tau, sn,
+      pdl(k_jam_face<true>, grid_of(sp), kTile, 0, st)(blks, sp, dir, pinfl, v, ld, ps, tau, sn,
                                                       G);
     else
-      k_jam_face<false><<<grid_of(sp), kTile, 0, st>>>(blks, sp, dir, pinfl, v, ld, ps, tau,
+      pdl(k_jam_face<false>, grid_of(sp), kTile, 0, st)(blks, sp, dir, pinfl, v, ld, ps, tau,
                                                        sn, G);
   }
   if (cells.ntiles > 0)
-    k_jam_accumulate<<<grid_of(cells), kTile, 0, st>>>(blks, cells, G, ld, dis, u, u32);
+    pdl(k_jam_accumulate, grid_of(cells), kTile, 0, st)(blks, cells, G, ld, dis, u, u32);
   return cudaGetLastError();
 }
 

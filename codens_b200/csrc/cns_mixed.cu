@@ -32,6 +32,7 @@ inline int grid_of(const Space& s) { return s.ntiles; }
 
 __global__ void __launch_bounds__(256) k_to_float(const double* __restrict__ a,
                                                  float* __restrict__ b, long long n) {
+  pdl_sync();
   const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (q < n) b[q] = (float)a[q];
 }
@@ -42,7 +43,7 @@ __global__ void __launch_bounds__(kTile) k_defect(const Blk* __restrict__ blks, 
                                                   const double* __restrict__ ur32,
                                                   double* __restrict__ corr) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const long long n = cell_index(blks[b], i, j, k);
 #pragma unroll
   for (int a = 0; a < 5; ++a) corr[a * ld + n] = u64[a * ld + n] - ur32[a * ld + n];
@@ -117,7 +118,7 @@ __global__ void __launch_bounds__(kTile) k_coef32(
     float4* __restrict__ snc, const float* __restrict__ u32, float* __restrict__ d1,
     float4* __restrict__ p1, const float* __restrict__ st32, float gam1, float pinfl, int qfix) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const long long n = cell_index(B, i, j, k);
   const float4 q0 = cq[n];
@@ -181,11 +182,11 @@ cudaError_t launch_coefficients32(const Blk* blks, Space cells, int eu, long lon
   if (cells.ntiles == 0) return cudaSuccess;
   const float g1 = (float)ph.gam1, pi = (float)ph.pinfl;
   if (eu)
-    k_coef32<true><<<grid_of(cells), kTile, 0, st>>>(blks, cells, ld, dtpas, dt, vol, cq32,
+    pdl(k_coef32<true>, grid_of(cells), kTile, 0, st)(blks, cells, ld, dtpas, dt, vol, cq32,
                                                      cv32, sn32, coefe32, coefdiag32, snc32,
                                                      u32, d1, p1, st32, g1, pi, qfix);
   else
-    k_coef32<false><<<grid_of(cells), kTile, 0, st>>>(blks, cells, ld, dtpas, dt, vol, cq32,
+    pdl(k_coef32<false>, grid_of(cells), kTile, 0, st)(blks, cells, ld, dtpas, dt, vol, cq32,
                                                       cv32, sn32, coefe32, coefdiag32, snc32,
                                                       u32, d1, p1, st32, g1, pi, qfix);
   return cudaGetLastError();
@@ -197,6 +198,7 @@ __global__ void __launch_bounds__(256) k_pack_faces32(const Blk* __restrict__ bl
                                                      long long ncells,
                                                      const float* __restrict__ sn,
                                                      float4* __restrict__ snc) {
+  pdl_sync();
   const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= ncells) return;
   int b = 0;
@@ -213,19 +215,19 @@ __global__ void __launch_bounds__(256) k_pack_faces32(const Blk* __restrict__ bl
 cudaError_t launch_pack_faces32(const Blk* blks, int nblk, long long ncells, const float* sn32,
                                 float4* snc32, cudaStream_t st) {
   if (ncells > 0)
-    k_pack_faces32<<<(int)((ncells + 255) / 256), 256, 0, st>>>(blks, nblk, ncells, sn32, snc32);
+    pdl(k_pack_faces32, (int)((ncells + 255) / 256), 256, 0, st)(blks, nblk, ncells, sn32, snc32);
   return cudaGetLastError();
 }
 
 cudaError_t launch_to_float(const double* a, float* b, long long n, cudaStream_t st) {
-  if (n > 0) k_to_float<<<(int)((n + 255) / 256), 256, 0, st>>>(a, b, n);
+  if (n > 0) pdl(k_to_float, (int)((n + 255) / 256), 256, 0, st)(a, b, n);
   return cudaGetLastError();
 }
 
 cudaError_t launch_defect(const Blk* blks, Space cells, long long ld, const double* u64,
                           const double* ur32, double* corr, cudaStream_t st) {
   if (cells.ntiles > 0)
-    k_defect<<<grid_of(cells), kTile, 0, st>>>(blks, cells, ld, u64, ur32, corr);
+    pdl(k_defect, grid_of(cells), kTile, 0, st)(blks, cells, ld, u64, ur32, corr);
   return cudaGetLastError();
 }
 
@@ -247,11 +249,11 @@ cudaError_t launch_face_flux_t<float>(const Blk* blks, const SpaceBuf* faces, in
   const int g = sp.grid();
   if (g == 0) return cudaSuccess;
   if (sc.ns)
-    k_face_flux<float, true><<<g, kTile, 0, st>>>(blks, sp, ph, sc, v, prim, ld, ps, tau, sn, R,
-                                                  G);
+    pdl(k_face_flux<float, true>, g, kTile, 0, st)(blks, sp, ph, sc, v, prim, ld, ps, tau, sn, R,
+                                                  G, nullptr);
   else
-    k_face_flux<float, false><<<g, kTile, 0, st>>>(blks, sp, ph, sc, v, prim, ld, ps, tau, sn, R,
-                                                   G);
+    pdl(k_face_flux<float, false>, g, kTile, 0, st)(blks, sp, ph, sc, v, prim, ld, ps, tau, sn, R,
+                                                   G, nullptr);
   return cudaGetLastError();
 }
 
@@ -282,7 +284,7 @@ cudaError_t launch_accumulate_t<float>(const Blk* blks, Space sp, const float* G
                                        long long ld, const double* corr, double* u,
                                        float* u32, cudaStream_t st, const float* V) {
   if (sp.ntiles > 0)
-    k_accumulate<float><<<grid_of(sp), kTile, 0, st>>>(blks, sp, G, ld, corr, u, u32, V);
+    pdl(k_accumulate<float>, grid_of(sp), kTile, 0, st)(blks, sp, G, ld, corr, u, u32, V);
   return cudaGetLastError();
 }
 
@@ -327,7 +329,7 @@ __global__ void __launch_bounds__(kTile) k_sweep_point32(
     Sweep32 a, const float4* __restrict__ faces, const float4* __restrict__ p_in,
     float4* __restrict__ p_out, float* __restrict__ d_out) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const long long n = cell_index(B, i, j, k), pn = pad_index(B, i, j, k), pld = B.pld;
   const float4 fi = faces[3 * n], fj = faces[3 * n + 1], fk = faces[3 * n + 2],
@@ -698,6 +700,7 @@ __global__ void __launch_bounds__(TI * TJ) k_sweep_f32(const Blk* __restrict__ b
                                                       Sweep32 a, const float* __restrict__ d_in,
                                                       float* __restrict__ d_out,
                                                       const CUtensorMap* __restrict__ map_d) {
+  pdl_sync();
   extern __shared__ unsigned char smem_dyn[];
   __shared__ __align__(8) unsigned long long bar[2];
   __shared__ int s_next;
@@ -758,10 +761,10 @@ cudaError_t sweep_f32_launch(const Blk* blks, Tiles tl, Phys ph, int qfix, int e
   const int grid = tl.sched ? min(tl.grid, tl.ntiles) : tl.ntiles;
   if (grid <= 0 || !tl.faces) return cudaErrorInvalidValue;
   if (eu)
-    k_sweep_f32<true, TI, TJ, BOX><<<grid, TI * TJ, sm, st>>>(blks, tl, ph, qfix, ld, a, d_in,
+    pdl(k_sweep_f32<true, TI, TJ, BOX>, grid, TI * TJ, sm, st)(blks, tl, ph, qfix, ld, a, d_in,
                                                                d_out, map_d);
   else
-    k_sweep_f32<false, TI, TJ, BOX><<<grid, TI * TJ, sm, st>>>(blks, tl, ph, qfix, ld, a, d_in,
+    pdl(k_sweep_f32<false, TI, TJ, BOX>, grid, TI * TJ, sm, st)(blks, tl, ph, qfix, ld, a, d_in,
                                                                 d_out, map_d);
   return cudaGetLastError();
 }
@@ -923,7 +926,7 @@ cudaError_t launch_point_sweeps32(const Blk* blks, Space cells, Phys ph, Scheme 
   const int g = grid_of(cells), q = eu ? sc.qfix_dfez : 0;
   const float g1 = (float)ph.gam1, pi = (float)ph.pinfl;
   auto run = [&](auto kernel, const float4* in, float4* out) {
-    kernel<<<g, kTile, 0, st>>>(blks, cells, g1, pi, q, ld, a, faces, in, out, d_out);
+    pdl(kernel, g, kTile, 0, st)(blks, cells, g1, pi, q, ld, a, faces, in, out, d_out);
   };
   for (int ls = 2; ls <= lmx; ++ls) {
     const float4* in = pt[ls & 1];
@@ -941,7 +944,7 @@ cudaError_t launch_point_sweeps32(const Blk* blks, Space cells, Phys ph, Scheme 
 cudaError_t launch_update32(const Blk* blks, Space cells, long long ld, const float* d,
                             double* v, const double* dt, double* normpart, cudaStream_t st) {
   if (cells.ntiles > 0)
-    k_update<float, true><<<grid_of(cells), kTile, 0, st>>>(blks, cells, ld, d, v, dt, nullptr,
+    pdl(k_update<float, true>, grid_of(cells), kTile, 0, st)(blks, cells, ld, d, v, dt, nullptr,
                                                             normpart);
   return cudaGetLastError();
 }

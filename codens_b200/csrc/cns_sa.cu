@@ -51,6 +51,7 @@ template <int NSC>
 __global__ void __launch_bounds__(256) k_teq_scalars(int mode, const double* __restrict__ v,
                                                     long long ld, long long n0, long long n1,
                                                     double* __restrict__ sc) {
+  pdl_sync();
   const long long n = n0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= n1) return;
 #pragma unroll
@@ -73,7 +74,7 @@ __global__ void __launch_bounds__(kTile) k_teq_cell(const Blk* __restrict__ blks
                                                     const double* __restrict__ vol,
                                                     double* __restrict__ out) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const long long n = cell_index(B, i, j, k);
   double s0[NSC];
@@ -131,7 +132,7 @@ __global__ void __launch_bounds__(kTile) k_smsa(
     const double* __restrict__ fd5y, const double* __restrict__ fd5z,
     double* __restrict__ ts6, double* __restrict__ ts7, double* __restrict__ cfke, int fix) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const long long n = cell_index(B, i, j, k);
   const long long m = n - B.npc;  // met_smsa.f90:177 reads txxf5x.. at this index
@@ -216,7 +217,7 @@ __global__ void __launch_bounds__(kTile) k_i2_cell(const Blk* __restrict__ blks,
                                                    double* __restrict__ rv,
                                                    double* __restrict__ cd) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const long long n = cell_index(blks[b], i, j, k);
   rv[n] = (mu[n] + mut[n] / cmt) / v[n];
   cd[n] = vol[n] / dt[n] + cfke[n] * vol[n];
@@ -232,7 +233,7 @@ __global__ void __launch_bounds__(kTile) k_i2_face(const Blk* __restrict__ blks,
                                                    double* __restrict__ uf,
                                                    double* __restrict__ ce) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const long long n = cell_index(B, i, j, k);
   const long long inc = ninc_of(B, dir), nl = n - inc;
@@ -252,7 +253,7 @@ __global__ void __launch_bounds__(kTile) k_i2_diag(const Blk* __restrict__ blks,
                                                    long long ld, const double* __restrict__ ce,
                                                    double* __restrict__ cd) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const long long m = cell_index(B, i, j, k);
   cd[m] = cd[m] + ce[m] + ce[m + 1] + ce[ld + m] + ce[ld + m + B.nid] + ce[2 * ld + m] +
@@ -276,7 +277,7 @@ __global__ void __launch_bounds__(kTile) k_i2_rhs(
     double* __restrict__ tb, double* __restrict__ tc, double* __restrict__ d6,
     double* __restrict__ d7) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const int oa = dir == 0 ? 1 : 0, ob = dir == 2 ? 1 : 2;
   const long long inc = ninc_of(B, dir), inca = ninc_of(B, oa), incb = ninc_of(B, ob);
@@ -325,6 +326,7 @@ __global__ void __launch_bounds__(kLineCta, 1) k_i2_line(const Blk* __restrict__
                                                       double* __restrict__ b7,
                                                       double* __restrict__ n6,
                                                       double* __restrict__ n7) {
+  pdl_sync();
   int b, i, j, k;
   constexpr int kSub = kTile / kLineCta;
   if (!space_elem_at(sp, blockIdx.x / kSub, (blockIdx.x % kSub) * kLineCta + threadIdx.x, b, i,
@@ -450,7 +452,7 @@ __global__ void __launch_bounds__(kTile) k_i2_update(const Blk* __restrict__ blk
                                                      const double* __restrict__ w7,
                                                      double* __restrict__ v) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const long long n = cell_index(blks[b], i, j, k);
   v[5 * ld + n] = v[5 * ld + n] + w6[n];
   v[6 * ld + n] = v[6 * ld + n] + w7[n];
@@ -470,6 +472,7 @@ __global__ void __launch_bounds__(256) k_wall_facets(Bnd bd, const Blk* __restri
                                                     const double* __restrict__ y,
                                                     const double* __restrict__ z,
                                                     double* __restrict__ par) {
+  pdl_sync();
   const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= nw) return;
   const long long e = went[q];
@@ -494,7 +497,7 @@ __global__ void __launch_bounds__(kTile) k_wall_dist(const Blk* __restrict__ blk
                                                      long long nw, double* __restrict__ dist) {
   __shared__ double sx[kWallChunk], sy[kWallChunk], sz[kWallChunk];
   int b, i, j, k;
-  const bool live = space_elem(sp, threadIdx.x, b, i, j, k);
+  const bool live = space_elem_sync(sp, threadIdx.x, b, i, j, k);
   double xcc = 0., ycc = 0., zcc = 0.;
   long long n = 0;
   if (live) {
@@ -532,6 +535,7 @@ __global__ void __launch_bounds__(kTile) k_wall_dist(const Blk* __restrict__ blk
 // (rokinf, roeinf), walls 0, extrapolation and outlet the interior cell
 __global__ void __launch_bounds__(256) k_turb_bord(Bnd bd, double* v, long long ld,
                                                   double rokinf, double roeinf) {
+  pdl_sync();
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= bd.nlist) return;
   const int bb = bd.ent_bnd[e];
@@ -632,6 +636,7 @@ __global__ void __launch_bounds__(128) k_lpsa1(Bnd bd, long long e0, int cnt, Ph
                                               const double* __restrict__ mu, double* mut,
                                               const double* __restrict__ dist,
                                               const double* __restrict__ temp) {
+  pdl_sync();
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= cnt) return;
   const long long e = e0 + m, ni = bd.ncin[e], nc = bd.ncbd[e];
@@ -670,6 +675,7 @@ __global__ void __launch_bounds__(128) k_lparoi1(Bnd bd, long long e0, int cnt, 
                                                 const double* __restrict__ mut,
                                                 const double* __restrict__ dist,
                                                 const double* __restrict__ temp, double* tau) {
+  pdl_sync();
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= cnt) return;
   const long long e = e0 + m, ni = bd.ncin[e], nc = bd.ncbd[e];
@@ -697,6 +703,7 @@ __global__ void __launch_bounds__(128) k_lparoi1(Bnd bd, long long e0, int cnt, 
 // variable vanish in the first cell of every wall-law wall
 __global__ void __launch_bounds__(256) k_i2_wall_freeze(const long long* __restrict__ ni,
                                                        long long cnt, double* w6, double* w7) {
+  pdl_sync();
   const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= cnt) return;
   w6[ni[q]] = 0.;
@@ -711,6 +718,7 @@ struct Fd6 {
 };
 
 __global__ void __launch_bounds__(256) k_fd_ghosts(Bnd bd, Fd6 fd) {
+  pdl_sync();
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= bd.nlist) return;
   const int bb = bd.ent_bnd[e];
@@ -729,7 +737,7 @@ __global__ void __launch_bounds__(256) k_fd_ghosts(Bnd bd, Fd6 fd) {
 __global__ void __launch_bounds__(kTile) k_cutsa(const Blk* __restrict__ blks, Space sp,
                                                  double* v, long long ld, double epsk) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const long long n = cell_index(blks[b], i, j, k);
   if (v[5 * ld + n] < 0.) v[5 * ld + n] = epsk;
   v[6 * ld + n] = 0.;
@@ -742,29 +750,29 @@ cudaError_t launch_wall_dist(const Bnd& bd, const Blk* blks, Space cells,
                              const double* y, const double* z, double* par, double* dist,
                              cudaStream_t st) {
   if (nw <= 0) return cudaErrorInvalidValue;
-  k_wall_facets<<<(int)((nw + 255) / 256), 256, 0, st>>>(bd, blks, went, nw, x, y, z, par);
+  pdl(k_wall_facets, (int)((nw + 255) / 256), 256, 0, st)(bd, blks, went, nw, x, y, z, par);
   if (cells.ntiles > 0)
-    k_wall_dist<<<grid_of(cells), kTile, 0, st>>>(blks, cells, x, y, z, par, nw, dist);
+    pdl(k_wall_dist, grid_of(cells), kTile, 0, st)(blks, cells, x, y, z, par, nw, dist);
   return cudaGetLastError();
 }
 
 cudaError_t launch_turb_bord(const Bnd& bd, double* v, long long ld, double rokinf,
                              double roeinf, cudaStream_t st) {
   if (bd.nlist > 0)
-    k_turb_bord<<<(int)((bd.nlist + 255) / 256), 256, 0, st>>>(bd, v, ld, rokinf, roeinf);
+    pdl(k_turb_bord, (int)((bd.nlist + 255) / 256), 256, 0, st)(bd, v, ld, rokinf, roeinf);
   return cudaGetLastError();
 }
 
 cudaError_t launch_fd_ghosts(const Bnd& bd, double* const fd[6], cudaStream_t st) {
   Fd6 f;
   for (int q = 0; q < 6; ++q) f.p[q] = fd[q];
-  if (bd.nlist > 0) k_fd_ghosts<<<(int)((bd.nlist + 255) / 256), 256, 0, st>>>(bd, f);
+  if (bd.nlist > 0) pdl(k_fd_ghosts, (int)((bd.nlist + 255) / 256), 256, 0, st)(bd, f);
   return cudaGetLastError();
 }
 
 cudaError_t launch_cutsa(const Blk* blks, Space cells, double* v, long long ld, double epsk,
                          cudaStream_t st) {
-  if (cells.ntiles > 0) k_cutsa<<<grid_of(cells), kTile, 0, st>>>(blks, cells, v, ld, epsk);
+  if (cells.ntiles > 0) pdl(k_cutsa, grid_of(cells), kTile, 0, st)(blks, cells, v, ld, epsk);
   return cudaGetLastError();
 }
 
@@ -776,21 +784,21 @@ cudaError_t launch_teq_grads(const Blk* blks, Space cells, int mode, int nsc,
   if (mode != 1) {
     const int g = (int)((n1 - n0 + 255) / 256);
     if (nsc == 3)
-      k_teq_scalars<3><<<g, 256, 0, st>>>(mode, v, ld, n0, n1, sc);
+      pdl(k_teq_scalars<3>, g, 256, 0, st)(mode, v, ld, n0, n1, sc);
     else if (nsc == 2)
-      k_teq_scalars<2><<<g, 256, 0, st>>>(mode, v, ld, n0, n1, sc);
+      pdl(k_teq_scalars<2>, g, 256, 0, st)(mode, v, ld, n0, n1, sc);
     else
-      k_teq_scalars<1><<<g, 256, 0, st>>>(mode, v, ld, n0, n1, sc);
+      pdl(k_teq_scalars<1>, g, 256, 0, st)(mode, v, ld, n0, n1, sc);
     mode = 1;
     f = sc;
   }
   {
     if (nsc == 3)
-      k_teq_cell<3><<<grid_of(cells), kTile, 0, st>>>(blks, cells, mode, v, f, ld, sn, vol, out);
+      pdl(k_teq_cell<3>, grid_of(cells), kTile, 0, st)(blks, cells, mode, v, f, ld, sn, vol, out);
     else if (nsc == 2)
-      k_teq_cell<2><<<grid_of(cells), kTile, 0, st>>>(blks, cells, mode, v, f, ld, sn, vol, out);
+      pdl(k_teq_cell<2>, grid_of(cells), kTile, 0, st)(blks, cells, mode, v, f, ld, sn, vol, out);
     else
-      k_teq_cell<1><<<grid_of(cells), kTile, 0, st>>>(blks, cells, mode, v, f, ld, sn, vol, out);
+      pdl(k_teq_cell<1>, grid_of(cells), kTile, 0, st)(blks, cells, mode, v, f, ld, sn, vol, out);
   }
   return cudaGetLastError();
 }
@@ -815,34 +823,34 @@ cudaError_t launch_impli2(const Blk* blks, const SpaceBuf* faces, const SpaceBuf
   if (e == cudaSuccess) e = cudaMemsetAsync(w + 11 * ld, 0, sizeof(double) * 4 * ld, st);
   if (e != cudaSuccess) return e;
   if (cells.ntiles == 0) return cudaSuccess;
-  k_i2_cell<<<grid_of(cells), kTile, 0, st>>>(blks, cells, v, mu, mut, dt, cfke, vol, cmt, rv,
+  pdl(k_i2_cell, grid_of(cells), kTile, 0, st)(blks, cells, v, mu, mut, dt, cfke, vol, cmt, rv,
                                               cd);
   for (int dir = 0; dir < 3; ++dir) {
     const Space sp = faces[dir].view(l0);
     if (sp.ntiles > 0)
-      k_i2_face<<<grid_of(sp), kTile, 0, st>>>(blks, sp, dir, v, ld, sn, vol, rv, uf, ce);
+      pdl(k_i2_face, grid_of(sp), kTile, 0, st)(blks, sp, dir, v, ld, sn, vol, rv, uf, ce);
   }
-  k_i2_diag<<<grid_of(cells), kTile, 0, st>>>(blks, cells, ld, ce, cd);
+  pdl(k_i2_diag, grid_of(cells), kTile, 0, st)(blks, cells, ld, ce, cd);
   int cur = 0;
   for (int dir = 0; dir < 3; ++dir) {
     const Space sp = lines[dir].view(l0);
     for (int sw = 0; sw < 2; ++sw) {
-      k_i2_rhs<<<grid_of(cells), kTile, 0, st>>>(blks, cells, dir, ld, u, uf, ce, cd,
+      pdl(k_i2_rhs, grid_of(cells), kTile, 0, st)(blks, cells, dir, ld, u, uf, ce, cd,
                                                  it[cur][0], it[cur][1], ta, tb, tc, d6, d7);
       const int lg = grid_of(sp) * (kTile / kLineCta);
       if (sp.ntiles > 0 && rcp)
-        k_i2_line<true><<<lg, kLineCta, 0, st>>>(blks, sp, dir, ta, tb, tc, d6, d7, al, b6, b7,
+        pdl(k_i2_line<true>, lg, kLineCta, 0, st)(blks, sp, dir, ta, tb, tc, d6, d7, al, b6, b7,
                                                  it[1 - cur][0], it[1 - cur][1]);
       else if (sp.ntiles > 0)
-        k_i2_line<false><<<lg, kLineCta, 0, st>>>(blks, sp, dir, ta, tb, tc, d6, d7, al, b6,
+        pdl(k_i2_line<false>, lg, kLineCta, 0, st)(blks, sp, dir, ta, tb, tc, d6, d7, al, b6,
                                                   b7, it[1 - cur][0], it[1 - cur][1]);
       cur = 1 - cur;
     }
   }
   if (nwall > 0)
-    k_i2_wall_freeze<<<(unsigned)((nwall + 255) / 256), 256, 0, st>>>(wall_ni, nwall,
+    pdl(k_i2_wall_freeze, (unsigned)((nwall + 255) / 256), 256, 0, st)(wall_ni, nwall,
                                                                      it[cur][0], it[cur][1]);
-  k_i2_update<<<grid_of(cells), kTile, 0, st>>>(blks, cells, ld, it[cur][0], it[cur][1], v);
+  pdl(k_i2_update, grid_of(cells), kTile, 0, st)(blks, cells, ld, it[cur][0], it[cur][1], v);
   return cudaGetLastError();
 }
 
@@ -850,7 +858,7 @@ cudaError_t launch_lpsa1(const Bnd& bd, long long e0, int cnt, Phys ph, WallLaw 
                          long long ld, double* v, const double* mu, double* mut,
                          const double* dist, const double* temp, cudaStream_t st) {
   if (cnt > 0)
-    k_lpsa1<<<(cnt + 127) / 128, 128, 0, st>>>(bd, e0, cnt, ph, wl, ld, v, mu, mut, dist, temp);
+    pdl(k_lpsa1, (cnt + 127) / 128, 128, 0, st)(bd, e0, cnt, ph, wl, ld, v, mu, mut, dist, temp);
   return cudaGetLastError();
 }
 
@@ -859,7 +867,7 @@ cudaError_t launch_lparoi1(const Bnd& bd, long long e0, int cnt, Phys ph, WallLa
                            const double* dist, const double* temp, double* tau,
                            cudaStream_t st) {
   if (cnt > 0)
-    k_lparoi1<<<(cnt + 127) / 128, 128, 0, st>>>(bd, e0, cnt, ph, wl, ld, v, mu, mut, dist,
+    pdl(k_lparoi1, (cnt + 127) / 128, 128, 0, st)(bd, e0, cnt, ph, wl, ld, v, mu, mut, dist,
                                                  temp, tau);
   return cudaGetLastError();
 }
@@ -869,7 +877,7 @@ cudaError_t launch_smsa(const Blk* blks, Space cells, long long ld, const double
                         const double* grt, const double* grr, const double* const fd5[3],
                         double* ts6, double* ts7, double* cfke, int fix, cudaStream_t st) {
   if (cells.ntiles > 0)
-    k_smsa<<<grid_of(cells), kTile, 0, st>>>(blks, cells, ld, v, mu, dist, dv, grt, grr,
+    pdl(k_smsa, grid_of(cells), kTile, 0, st)(blks, cells, ld, v, mu, dist, dv, grt, grr,
                                              fd5[0], fd5[1], fd5[2], ts6, ts7, cfke, fix);
   return cudaGetLastError();
 }

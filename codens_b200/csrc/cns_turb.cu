@@ -23,6 +23,7 @@ __global__ void __launch_bounds__(256) k_fludc(long long n0, long long n1,
                                               double* fd5y, double* fd5z, double* fd6x,
                                               double* fd6y, double* fd6z, double alfak,
                                               double alfae) {
+  pdl_sync();
   const long long n = n0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (n > n1) return;
   const double m = mu[n], mt = mut[n];
@@ -40,6 +41,7 @@ __global__ void __launch_bounds__(256) k_fludcsa(long long n0, long long n1,
                                                 const double* __restrict__ mu, double* fd5x,
                                                 double* fd5y, double* fd5z, double* fd6x,
                                                 double* fd6y, double* fd6z, double sigma1) {
+  pdl_sync();
   const long long n = n0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (n > n1) return;
   const double smutot = sigma1 * (mu[n] + s6[n]);
@@ -84,7 +86,7 @@ __global__ void __launch_bounds__(kTile) k_roe2o_face(const Blk* __restrict__ bl
                                                       const double* __restrict__ sn,
                                                       double* __restrict__ G) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const long long n = cell_index(B, i, j, k);
   const long long inc = ninc_of(B, dir);
@@ -127,7 +129,7 @@ __global__ void __launch_bounds__(kTile) k_roe2o_acc(const Blk* __restrict__ blk
                                                      const double* __restrict__ G,
                                                      long long ld, double* __restrict__ d) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   --i;
   --j;
@@ -160,7 +162,7 @@ __global__ void __launch_bounds__(kTile) k_samut(const Blk* __restrict__ blks, S
                                                  const double* __restrict__ mu,
                                                  double* __restrict__ mut, double cv13) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const long long n = cell_index(blks[b], i, j, k);
   const double xkhi = v6[n] / mu[n];
   const double xkhi3 = xkhi * xkhi * xkhi;
@@ -194,7 +196,7 @@ __global__ void __launch_bounds__(kTile) k_turb_face(const Blk* __restrict__ blk
                                                      const double* __restrict__ sn,
                                                      double* __restrict__ G) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const long long n = cell_index(B, i, j, k);
   const long long inc = ninc_of(B, dir);
@@ -229,7 +231,7 @@ __global__ void __launch_bounds__(kTile) k_turb_acc(const Blk* __restrict__ blks
                                                     const double* __restrict__ d,
                                                     double* __restrict__ u) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const long long n = cell_index(B, i, j, k);
   double acc[2] = {0., 0.};
@@ -261,7 +263,7 @@ __global__ void __launch_bounds__(kTile) k_turb_acc(const Blk* __restrict__ blks
 cudaError_t launch_fludc(long long n0, long long n1, const double* mu, const double* mut,
                          double* const fd[6], double alfak, double alfae, cudaStream_t st) {
   if (n1 >= n0)
-    k_fludc<<<(int)((n1 - n0 + 256) / 256), 256, 0, st>>>(n0, n1, mu, mut, fd[0], fd[1], fd[2],
+    pdl(k_fludc, (int)((n1 - n0 + 256) / 256), 256, 0, st)(n0, n1, mu, mut, fd[0], fd[1], fd[2],
                                                           fd[3], fd[4], fd[5], alfak, alfae);
   return cudaGetLastError();
 }
@@ -270,7 +272,7 @@ cudaError_t launch_fludcsa(long long n0, long long n1, const double* s6, const d
                            double* const fd[6], double sigma, cudaStream_t st) {
   const double sigma1 = 1. / sigma;
   if (n1 >= n0)
-    k_fludcsa<<<(int)((n1 - n0 + 256) / 256), 256, 0, st>>>(n0, n1, s6, mu, fd[0], fd[1],
+    pdl(k_fludcsa, (int)((n1 - n0 + 256) / 256), 256, 0, st)(n0, n1, s6, mu, fd[0], fd[1],
                                                             fd[2], fd[3], fd[4], fd[5], sigma1);
   return cudaGetLastError();
 }
@@ -279,7 +281,7 @@ cudaError_t launch_samut(const Blk* blks, Space cells, const double* v6, const d
                          double* mut, cudaStream_t st) {
   const double cv1 = 7.1;  // atlecdon.f90:200
   if (cells.ntiles > 0)
-    k_samut<<<grid_of(cells), kTile, 0, st>>>(blks, cells, v6, mu, mut, cv1 * cv1 * cv1);
+    pdl(k_samut, grid_of(cells), kTile, 0, st)(blks, cells, v6, mu, mut, cv1 * cv1 * cv1);
   return cudaGetLastError();
 }
 
@@ -293,10 +295,10 @@ cudaError_t launch_sch_turb(const Blk* blks, const SpaceBuf* faces, Space cells,
   for (int dir = 0; dir < 3; ++dir) {
     const Space sp = faces[dir].view(l0);
     if (sp.ntiles > 0)
-      k_turb_face<<<grid_of(sp), kTile, 0, st>>>(blks, sp, dir, v, ld, fdp, sn, G);
+      pdl(k_turb_face, grid_of(sp), kTile, 0, st)(blks, sp, dir, v, ld, fdp, sn, G);
   }
   if (cells.ntiles > 0)
-    k_turb_acc<<<grid_of(cells), kTile, 0, st>>>(blks, cells, G, ld, vol, ts6, ts7, d, u);
+    pdl(k_turb_acc, grid_of(cells), kTile, 0, st)(blks, cells, G, ld, vol, ts6, ts7, d, u);
   return cudaGetLastError();
 }
 
@@ -307,11 +309,11 @@ cudaError_t launch_roe2o(const Blk* blks, const SpaceBuf* faces, Space cells_ext
   for (int dir = 0; dir < 3; ++dir) {
     const Space sp = faces[dir].view(l0);
     if (sp.ntiles > 0)
-      k_roe2o_face<<<grid_of(sp), kTile, 0, st>>>(blks, sp, dir, harten, epsroe, gam, gam1, t,
+      pdl(k_roe2o_face, grid_of(sp), kTile, 0, st)(blks, sp, dir, harten, epsroe, gam, gam1, t,
                                                   ld, sn, G);
   }
   if (cells_ext.ntiles > 0)
-    k_roe2o_acc<<<grid_of(cells_ext), kTile, 0, st>>>(blks, cells_ext, G, ld, d);
+    pdl(k_roe2o_acc, grid_of(cells_ext), kTile, 0, st)(blks, cells_ext, G, ld, d);
   return cudaGetLastError();
 }
 

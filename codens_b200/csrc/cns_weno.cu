@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(kTile) k_weno_face(const Blk* __restrict__ blk
                                                      double* __restrict__ G,
                                                      double* __restrict__ V) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const int p = DIR == 0 ? i : (DIR == 1 ? j : k);
   if (p > nd_of(B, DIR) - 2) return;
@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(kTile) k_weno_acc(const Blk* __restrict__ blks
                                                     double* __restrict__ u,
                                                     float* __restrict__ u32) {
   int b, i, j, k;
-  if (!space_elem(sp, threadIdx.x, b, i, j, k)) return;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const long long n = cell_index(B, i, j, k);
   double acc[5] = {0., 0., 0., 0., 0.};
@@ -391,13 +391,13 @@ cudaError_t launch_weno5(const Blk* blks, Space cells, Phys ph, int fix, const d
                          const double* ps, const double* tau, const double* sn, double* G,
                          double* V, double* u, float* u32, cudaStream_t st) {
   if (cells.ntiles == 0) return cudaSuccess;
-  k_weno_face<0><<<cells.ntiles, kTile, 0, st>>>(blks, cells, ph, fix, v, ld, ps, tau, sn, G,
+  pdl(k_weno_face<0>, cells.ntiles, kTile, 0, st)(blks, cells, ph, fix, v, ld, ps, tau, sn, G,
                                                   V);
-  k_weno_face<1><<<cells.ntiles, kTile, 0, st>>>(blks, cells, ph, fix, v, ld, ps, tau, sn, G,
+  pdl(k_weno_face<1>, cells.ntiles, kTile, 0, st)(blks, cells, ph, fix, v, ld, ps, tau, sn, G,
                                                   V);
-  k_weno_face<2><<<cells.ntiles, kTile, 0, st>>>(blks, cells, ph, fix, v, ld, ps, tau, sn, G,
+  pdl(k_weno_face<2>, cells.ntiles, kTile, 0, st)(blks, cells, ph, fix, v, ld, ps, tau, sn, G,
                                                   V);
-  k_weno_acc<<<cells.ntiles, kTile, 0, st>>>(blks, cells, ph, v, ld, ps, tau, sn, G, V, u,
+  pdl(k_weno_acc, cells.ntiles, kTile, 0, st)(blks, cells, ph, v, ld, ps, tau, sn, G, V, u,
                                               u32);
   return cudaGetLastError();
 }
