@@ -74,7 +74,7 @@ struct cns_ctx {
   std::vector<int> h_btype;
   long long n_idd_ent = 0;
   long long* d_idd_ents = nullptr;  // list entries of injection boundaries
-  unsigned* d_idd_masks = nullptr;  // per boundary sweep masks
+  unsigned* d_idd_work = nullptr;  // the injection condition's sweep counts and flags
   // scratch
   Work w;
   std::vector<void*> allocs;
@@ -738,7 +738,7 @@ cudaError_t enqueue_step(cns_ctx* c, bool first, bool dt_on) {
   if (e == cudaSuccess && jameson(c)) e = jameson_dissipation(c, first);
   if (e == cudaSuccess)
     e = launch_rbord(c->bd, c->ph, s.v, ld, s.pression, s.ztemp, s.cson, c->n_idd_ent,
-                     c->d_idd_ents, c->d_idd_masks, c->st);
+                     c->d_idd_ents, c->d_idd_work, c->st);
   if (e == cudaSuccess && (c->sa_on || c->ke_on)) e = enqueue_met_num(c);
   if (e == cudaSuccess) e = launch_prim(0, c->lay.ncells, s.v, ld, c->w.prim, c->st);
   if (e == cudaSuccess && c->sc.ns) {
@@ -849,7 +849,7 @@ cudaError_t enqueue_step_mixed(cns_ctx* c, MixedMode mode, bool first, bool dt_o
   if (e == cudaSuccess && jameson(c)) e = jameson_dissipation(c, first);
   if (e == cudaSuccess)
     e = launch_rbord(c->bd, c->ph, s.v, ld, s.pression, s.ztemp, s.cson, c->n_idd_ent,
-                     c->d_idd_ents, c->d_idd_masks, c->st);
+                     c->d_idd_ents, c->d_idd_work, c->st);
   if (e == cudaSuccess && (c->sa_on || c->ke_on)) e = enqueue_met_num(c);
   if (e == cudaSuccess) {
     PrimShadow sh{};
@@ -1340,7 +1340,7 @@ int cns_create(const cns_layout_t* layout, const cns_phys_t* phys,
     if (e == cudaSuccess) e = upload(c, &c->d_wall_ents, wall_ents.data(), wall_ents.size());
     if (e == cudaSuccess) e = upload(c, &c->d_lp2_ni, lp2_ni.data(), lp2_ni.size());
     c->n_lp2_ni = (long long)lp2_ni.size();
-    if (e == cudaSuccess) e = dev_alloc(c, &c->d_idd_masks, (size_t)nb);
+    if (e == cudaSuccess) e = dev_alloc(c, &c->d_idd_work, (size_t)(2 * nb + 1));
     if (e == cudaSuccess) e = dev_alloc(c, &c->bd.nxn, (size_t)nl);
     if (e == cudaSuccess) e = dev_alloc(c, &c->bd.nyn, (size_t)nl);
     if (e == cudaSuccess) e = dev_alloc(c, &c->bd.nzn, (size_t)nl);
@@ -1609,7 +1609,7 @@ int cns_rbord(cns_ctx* c, double* v, double* ps, double* temp, double* cson) {
   double* dcson = sg.inout(cson, ld);
   CK(sg.err);
   CK(launch_rbord(c->bd, c->ph, dv, ld, dps, dtemp, dcson, c->n_idd_ent, c->d_idd_ents,
-                  c->d_idd_masks, c->st));
+                  c->d_idd_work, c->st));
   CK(sg.finish());
   return CNS_OK;
 }
@@ -2197,7 +2197,7 @@ int cns_adjoint_prepare(cns_ctx* c) {
                     s.cson, c->st));
   CK(global_dt(c));
   CK(launch_rbord(c->bd, c->ph, s.v, ld, s.pression, s.ztemp, s.cson, c->n_idd_ent,
-                  c->d_idd_ents, c->d_idd_masks, c->st));
+                  c->d_idd_ents, c->d_idd_work, c->st));
   CK(launch_prim(0, c->lay.ncells, s.v, ld, c->w.prim, c->st));
   CK(launch_implicit_coefficients(c->d_blks, all, c->ph, 1, 0., s.dt, s.v, c->w.prim, s.mu,
                                   s.mut, s.sn, s.vol, s.cson, nullptr, 0, nullptr, nullptr,

@@ -189,7 +189,7 @@ cudaError_t launch_chronos(const Blk* blks, Space sp, Phys ph, Scheme sc,
 // rbord: every list entry, then the injection entries (two passes)
 cudaError_t launch_rbord(const Bnd& bd, Phys ph, double* v, long long ld,
                          double* ps, double* temp, double* cson, long long n_idd_ent,
-                         const long long* idd_ents, unsigned* masks, cudaStream_t st);
+                         const long long* idd_ents, unsigned* idd_work, cudaStream_t st);
 
 cudaError_t launch_tau_ghosts(const Bnd& bd, double* tau, long long ld,
                               cudaStream_t st);
