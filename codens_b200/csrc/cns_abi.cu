@@ -1,6 +1,7 @@
 // cns_abi.cu -- C ABI of the CodeNS hot path: context (the reference's module
 // state), tile work lists, per-routine entry points and the graph-captured
 // fused pseudo-time step.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -187,17 +188,46 @@ cudaError_t build_space(cns_ctx* c, SpaceBuf& s, F ext_of) {
   return e;
 }
 
-// the 2.5D sweep tiles: patches of ti x tj columns, kc planes deep, block by
-// block
-cudaError_t build_tiles(cns_ctx* c, TileBuf& t, int ti, int tj, int kc) {
+// The depth the sweep tiles are cut to: at most kc planes, such that the last
+// wave of CTAs is not nearly empty.  A CTA's time is its planes plus about
+// kTilePrologue planes of start-up (two planes staged and evaluated before
+// the first result), and the launch takes as many such times as there are
+// waves of `slots` resident CTAs.  Sixteen planes asked: 1.07M cells in three
+// blocks (640 CTAs for 444 slots) go to fewer planes and 2.14 -> 2.00 ms an
+// iteration, a batch of 24 uneven boxes 1.56 -> 1.52 ms.
+constexpr double kTilePrologue = 2.5;
+
+int sweep_depth(const HostLayout& lay, int ti, int tj, int kc, int slots) {
+  int best = kc;
+  double cost = 1e300;
+  for (int d = kc; d >= 1 && slots > 0; --d) {
+    long long n = 0;
+    int deep = 0;
+    for (const Blk& B : lay.blks) {
+      n += (long long)((B.ni - 2 + ti) / ti) * ((B.nj - 2 + tj) / tj) * ((B.nk - 2 + d) / d);
+      deep = std::max(deep, std::min(d, B.nk - 1));
+    }
+    const double x = (double)((n + slots - 1) / slots) * (deep + kTilePrologue);
+    if (x < cost) {
+      cost = x;
+      best = d;
+    }
+  }
+  return best;
+}
+
+// the 2.5D sweep tiles: patches of ti x tj columns, at most kc planes deep
+// (slots > 0: cut to sweep_depth), block by block
+cudaError_t build_tiles(cns_ctx* c, TileBuf& t, int ti, int tj, int kc, int slots = 0) {
   dev_free(c, t.d_tile);
   t.d_tile = nullptr;
+  const int depth = sweep_depth(c->lay, ti, tj, kc, slots);
   std::vector<int4> tl;
   t.blk_tile0.assign(c->lay.blks.size() + 1, 0);
   for (size_t b = 0; b < c->lay.blks.size(); ++b) {
     const Blk& B = c->lay.blks[b];
     t.blk_tile0[b] = (int)tl.size();
-    for (int k0 = 1; k0 <= B.nk - 1; k0 += kc)
+    for (int k0 = 1; k0 <= B.nk - 1; k0 += depth)
       for (int j0 = 1; j0 <= B.nj - 1; j0 += tj)
         for (int i0 = 1; i0 <= B.ni - 1; i0 += ti) tl.push_back(make_int4((int)b, i0, j0, k0));
   }
@@ -206,7 +236,19 @@ cudaError_t build_tiles(cns_ctx* c, TileBuf& t, int ti, int tj, int kc) {
   t.ti = ti;
   t.tj = tj;
   t.kc = kc;
+  t.depth = depth;
   return upload(c, &t.d_tile, tl.data(), tl.size());
+}
+
+// resident CTAs of the sweep kernel of a patch shape on the whole GPU
+int sweep_slots(cns_ctx* c, bool fp32, int ti, int tj) {
+  const int per_sm = fp32 ? sweep_f32_blocks_per_sm(ti, tj, !c->sc.ns, c->staging32 == 0)
+                          : jacobi_25d_blocks_per_sm(ti, tj, !c->sc.ns);
+  return per_sm * c->nsm;
+}
+
+cudaError_t build_sweep_tiles(cns_ctx* c, bool fp32, TileBuf& t, int ti, int tj, int kc) {
+  return build_tiles(c, t, ti, tj, kc, sweep_slots(c, fp32, ti, tj));
 }
 
 // the FP32 sweep tiles run as a persistent launch: one CTA per resident slot
@@ -1052,7 +1094,7 @@ cudaError_t tune_sweeps(cns_ctx* c, bool fp32) {
   {
     int cti, ctj, ckc;
     if (!key.empty() && tune_cache_lookup(c, key, &cti, &ctj, &ckc)) {
-      cudaError_t e = build_tiles(c, best, cti, ctj, ckc);
+      cudaError_t e = build_sweep_tiles(c, fp32, best, cti, ctj, ckc);
       if (e == cudaSuccess && fp32) persistent_sweep32(c);
       if (e == cudaSuccess) {
         (fp32 ? c->tuned32 : c->tuned64) = true;
@@ -1069,7 +1111,12 @@ cudaError_t tune_sweeps(cns_ctx* c, bool fp32) {
   TileBuf cand;
   for (int sh = 0; sh < kSweepShapes && e == cudaSuccess; ++sh)
     for (int kc : kTuneKc) {
-      e = build_tiles(c, cand, kSweepShape[sh][0], kSweepShape[sh][1], kc);
+      const int ti = kSweepShape[sh][0], tj = kSweepShape[sh][1];
+      // plane counts cut to the same depth are one tiling
+      if (cand.ti == ti && cand.tj == tj &&
+          cand.depth == sweep_depth(c->lay, ti, tj, kc, sweep_slots(c, fp32, ti, tj)))
+        continue;
+      e = build_sweep_tiles(c, fp32, cand, ti, tj, kc);
       if (e != cudaSuccess) break;
       if (fp32) {  // timed as it runs: the persistent launch
         const int per_sm =
@@ -1095,7 +1142,7 @@ cudaError_t tune_sweeps(cns_ctx* c, bool fp32) {
   dev_free(c, cand.d_tile);
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
-  if (e == cudaSuccess) e = build_tiles(c, best, bti, btj, bkc);
+  if (e == cudaSuccess) e = build_sweep_tiles(c, fp32, best, bti, btj, bkc);
   if (e == cudaSuccess && fp32) persistent_sweep32(c);
   if (e == cudaSuccess) {
     (fp32 ? c->tuned32 : c->tuned64) = true;
@@ -1250,13 +1297,15 @@ int cns_create(const cns_layout_t* layout, const cns_phys_t* phys,
   if (e == cudaSuccess)
     e = build_space(c, c->cells_ext, [](const Blk& B, int x[3]) {
       x[0] = B.ni + 1; x[1] = B.nj + 1; x[2] = B.nk + 1; });
-  if (e == cudaSuccess) e = build_tiles(c, c->tiles64, 32, 8, 8);
-  if (e == cudaSuccess) e = build_tiles(c, c->tiles32, 32, 8, 8);
-  if (e == cudaSuccess) e = dev_alloc(c, &c->sched32, 2);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, c->device);
+  if (e == cudaSuccess) e = init_jacobi_25d();
+  // until tuned or set: three FP64 CTAs of 16x8 per SM (one of 32x8), two
+  // FP32 ones of 32x8
+  if (e == cudaSuccess) e = build_sweep_tiles(c, false, c->tiles64, 16, 8, 16);
+  if (e == cudaSuccess) e = build_sweep_tiles(c, true, c->tiles32, 32, 8, 16);
+  if (e == cudaSuccess) e = dev_alloc(c, &c->sched32, 2);
   if (e == cudaSuccess) persistent_sweep32(c);
   if (e == cudaSuccess) e = build_tiles(c, c->tiles_res, kResTI, kResTJ, kResKC);
-  if (e == cudaSuccess) e = init_jacobi_25d();
   for (int dir = 0; dir < 3 && e == cudaSuccess; ++dir) {
     e = build_space(c, c->faces[dir], [dir](const Blk& B, int x[3]) {
       x[0] = dir == 0 ? B.ni : B.ni - 1;
@@ -2468,7 +2517,7 @@ int cns_set_sweep_tiles(cns_ctx* c, int precision, int ti, int tj, int kc) {
     ok = ok || (kSweepShape[sh][0] == ti && kSweepShape[sh][1] == tj);
   if (!ok) return fail(c, CNS_EINVAL, "sweep patch shape not one of 32x4, 32x8, 16x8, 16x16");
   CK(cudaStreamSynchronize(c->st));
-  CK(build_tiles(c, precision == 0 ? c->tiles64 : c->tiles32, ti, tj, kc));
+  CK(build_sweep_tiles(c, precision != 0, precision == 0 ? c->tiles64 : c->tiles32, ti, tj, kc));
   if (precision != 0) persistent_sweep32(c);
   (precision == 0 ? c->tuned64 : c->tuned32) = true;
   (precision == 0 ? c->tune_src64 : c->tune_src32) = 0;

@@ -1096,6 +1096,26 @@ cudaError_t launch_jacobi_25d_t<double>(const Blk* blks, Tiles tl, Phys ph, int 
                                         coefdiag, d_in, d_out, st);
 }
 
+int jacobi_25d_blocks_per_sm(int ti, int tj, int eu) {
+  int n = 0;
+#define CNS_OCC1(A, B, E)                                                                   \
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_jacobi_25d<double, E, 0, A, B>, A * B, \
+                                                jacobi_25d_smem<A, B, double, 0, E>())
+#define CNS_OCC(A, B)                                  \
+  if (ti == A && tj == B) {                            \
+    if (eu) CNS_OCC1(A, B, true);                      \
+    else CNS_OCC1(A, B, false);                        \
+    return n;                                          \
+  }
+  CNS_OCC(32, 4)
+  CNS_OCC(32, 8)
+  CNS_OCC(16, 8)
+  CNS_OCC(16, 16)
+#undef CNS_OCC
+#undef CNS_OCC1
+  return 0;
+}
+
 cudaError_t init_jacobi_25d() {
   cudaError_t e = jacobi_25d_attr<double, 0>();
   if (e == cudaSuccess) e = init_jacobi_25d_float();

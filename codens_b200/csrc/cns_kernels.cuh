@@ -90,6 +90,7 @@ cudaError_t launch_dual_update(const Blk* blks, Space cells, long long ld, int m
 // the 2.5D tile list of one sweep configuration
 struct TileBuf {
   int ti = 0, tj = 0, kc = 0, ntiles = 0;
+  int depth = 0;  // planes of a tile, at most kc (sweep_depth)
   std::vector<int> blk_tile0;  // first tile of each block, size nblk+1
   int4* d_tile = nullptr;
   int* sched = nullptr;  // persistent launch: tile counter pair (device), else null
@@ -98,7 +99,7 @@ struct TileBuf {
   Tiles view(int l0 = -1) const {
     Tiles t;
     t.tile = d_tile;
-    t.kc = kc;
+    t.kc = depth;
     t.ti = ti;
     t.tj = tj;
     t.sched = sched;
@@ -456,6 +457,8 @@ cudaError_t launch_cutsa(const Blk* blks, Space cells, double* v, long long ld, 
 // raise the dynamic shared-memory limit of every 2.5D instantiation (once
 // per device, before the first launch)
 cudaError_t init_jacobi_25d();
+// resident CTAs per SM of the FP64 2.5D sweep kernel of patch ti x tj
+int jacobi_25d_blocks_per_sm(int ti, int tj, int eu);
 // resident CTAs per SM of the FP32 sweep kernel of patch ti x tj (persistent launch size)
 int sweep_f32_blocks_per_sm(int ti, int tj, int eu, int box);
 cudaError_t init_jacobi_25d_float();
