@@ -585,7 +585,7 @@ cudaError_t ensure_sa_step(cns_ctx* c) {
   cudaError_t e = cudaSuccess;
   if (!c->sa_gr) e = dev_alloc(c, &c->sa_gr, 6 * ld, false);
   if (e == cudaSuccess && !c->sa_sc) e = dev_alloc(c, &c->sa_sc, 3 * ld, false);
-  if (e == cudaSuccess && !c->sa_w) e = dev_alloc(c, &c->sa_w, 20 * ld, false);
+  if (e == cudaSuccess && !c->sa_w) e = dev_alloc(c, &c->sa_w, 20 * ld);
   if (e == cudaSuccess && !c->sa_dv) e = dev_alloc(c, &c->sa_dv, 9 * ld);
   if (e == cudaSuccess && !c->sa_fd) e = dev_alloc(c, &c->sa_fd, 6 * ld);
   if (e == cudaSuccess && !c->sa_ts) e = dev_alloc(c, &c->sa_ts, 2 * ld);
@@ -658,6 +658,7 @@ cudaError_t enqueue_met_num_ke(cns_ctx* c) {
   double* ts6 = c->sa_ts;
   double* ts7 = c->sa_ts + ld;
   cudaError_t e = launch_turb_bord(c->bd, s.v, ld, c->ke_rokinf, c->ke_roeinf, c->st);
+  if (e == cudaSuccess) e = launch_prim(0, c->lay.ncells, s.v, ld, c->w.prim, c->st);
   for (int b = 0; b < nb && e == cudaSuccess; ++b) {
     const Space cb = c->cells.view(b);
     long long b0, b1, n0, n1;
@@ -681,17 +682,17 @@ cudaError_t enqueue_met_num_ke(cns_ctx* c) {
   if (e == cudaSuccess) e = launch_fd_ghosts(c->bd, fdw, c->st);
   const Space all = c->cells.view(-1);
   if (e == cudaSuccess)
-    e = launch_roe2o(c->d_blks, c->faces, c->cells_ext.view(-1), -1, sa_harten(c), c->epsroe,
-                     c->ph.gam, c->ph.gam1, s.v, ld, s.sn, c->w.G, s.d, c->st);
+    e = launch_roe2o(c->d_blks, c->cells_ext.view(-1), sa_harten(c), c->epsroe, c->ph.gam,
+                     c->ph.gam1, s.v, c->w.prim, ld, s.sn, s.d, c->st);
   if (e == cudaSuccess)
     e = cudaMemsetAsync(s.u + 5 * ld, 0, sizeof(double) * c->lay.ncells, c->st);
   if (e == cudaSuccess)
     e = cudaMemsetAsync(s.u + 6 * ld, 0, sizeof(double) * c->lay.ncells, c->st);
   if (e == cudaSuccess)
-    e = launch_sch_turb(c->d_blks, c->faces, all, -1, s.v, ld, fdr, ts6, ts7, s.d, s.sn, s.vol,
-                        c->w.G, s.u, c->st);
+    e = launch_sch_turb(c->d_blks, all, s.v, c->w.prim, ld, fdr, ts6, ts7, s.d, s.sn, s.vol, s.u,
+                        c->st);
   if (e == cudaSuccess)
-    e = launch_impli2(c->d_blks, c->faces, c->lines, all, -1, ld, s.u, s.dt, s.v, s.mu, s.mut,
+    e = launch_impli2(c->d_blks, c->lines, all, -1, ld, s.u, s.dt, s.v, c->w.prim, s.mu, s.mut,
                       c->sa_cfke, s.sn, s.vol, 1.0, c->sa_w, c->sc.precision != 0, nullptr, 0,
                       c->st);
   if (e == cudaSuccess) e = launch_cutke(c->d_blks, all, ld, s.v, c->ke_epsk, c->ke_epse, c->st);
@@ -710,6 +711,7 @@ cudaError_t enqueue_met_num(cns_ctx* c) {
   double* ts6 = c->sa_ts;
   double* ts7 = c->sa_ts + ld;
   cudaError_t e = launch_turb_bord(c->bd, s.v, ld, c->sa_rokinf, c->sa_roeinf, c->st);
+  if (e == cudaSuccess) e = launch_prim(0, c->lay.ncells, s.v, ld, c->w.prim, c->st);
   for (int b = 0; b < nb && e == cudaSuccess; ++b) {
     const Space cb = c->cells.view(b);
     long long b0, b1;
@@ -743,18 +745,18 @@ cudaError_t enqueue_met_num(cns_ctx* c) {
   if (e == cudaSuccess) e = launch_fd_ghosts(c->bd, fdw, c->st);
   const Space all = c->cells.view(-1);
   if (e == cudaSuccess)
-    e = launch_roe2o(c->d_blks, c->faces, c->cells_ext.view(-1), -1, sa_harten(c), c->epsroe,
-                     c->ph.gam, c->ph.gam1, s.v, ld, s.sn, c->w.G, s.d, c->st);
+    e = launch_roe2o(c->d_blks, c->cells_ext.view(-1), sa_harten(c), c->epsroe, c->ph.gam,
+                     c->ph.gam1, s.v, c->w.prim, ld, s.sn, s.d, c->st);
   // sch_turb.f90:59-66 zeroes u(:,6:7) over every block
   if (e == cudaSuccess)
     e = cudaMemsetAsync(s.u + 5 * ld, 0, sizeof(double) * c->lay.ncells, c->st);
   if (e == cudaSuccess)
     e = cudaMemsetAsync(s.u + 6 * ld, 0, sizeof(double) * c->lay.ncells, c->st);
   if (e == cudaSuccess)
-    e = launch_sch_turb(c->d_blks, c->faces, all, -1, s.v, ld, fdr, ts6, ts7, s.d, s.sn, s.vol,
-                        c->w.G, s.u, c->st);
+    e = launch_sch_turb(c->d_blks, all, s.v, c->w.prim, ld, fdr, ts6, ts7, s.d, s.sn, s.vol, s.u,
+                        c->st);
   if (e == cudaSuccess)
-    e = launch_impli2(c->d_blks, c->faces, c->lines, all, -1, ld, s.u, s.dt, s.v, s.mu, s.mut,
+    e = launch_impli2(c->d_blks, c->lines, all, -1, ld, s.u, s.dt, s.v, c->w.prim, s.mu, s.mut,
                       c->sa_cfke, s.sn, s.vol, 1.0, c->sa_w, c->sc.precision != 0,
                       c->d_lp2_ni, c->n_lp2_ni, c->st);
   if (e == cudaSuccess) e = launch_cutsa(c->d_blks, all, s.v, ld, c->sa_epsk, c->st);
@@ -1922,8 +1924,9 @@ static int met_roe2o_common(cns_ctx* c, int l, const double* t, double* d, const
   double* dd = sg.inout(d, 7 * ld);
   const double* dsn = sg.in(sn, sn_elems(c, l));
   CK(sg.err);
-  CK(launch_roe2o(c->d_blks, c->faces, c->cells_ext.view(l - 1), l - 1, harten, c->epsroe,
-                  c->ph.gam, c->ph.gam1, dt7, ld, sn_base(c, l, dsn), c->w.G, dd, c->st));
+  CK(prim_of(c, l, dt7));
+  CK(launch_roe2o(c->d_blks, c->cells_ext.view(l - 1), harten, c->epsroe, c->ph.gam, c->ph.gam1,
+                  dt7, c->w.prim, ld, sn_base(c, l, dsn), dd, c->st));
   CK(sg.finish());
   return CNS_OK;
 }
@@ -1955,8 +1958,9 @@ int cns_sch_turb(cns_ctx* c, int l, double* u, const double* v, const double* d,
   CK(cudaMemsetAsync(u + 5 * ld + n0, 0, sizeof(double) * (n1 - n0), c->st));
   CK(cudaMemsetAsync(u + 6 * ld + n0, 0, sizeof(double) * (n1 - n0), c->st));
   const double* fd[6] = {fd5x, fd5y, fd5z, fd6x, fd6y, fd6z};
-  CK(launch_sch_turb(c->d_blks, c->faces, c->cells.view(l - 1), l - 1, v, ld, fd, ts6, ts7, d,
-                     sn, vol, c->w.G, u, c->st));
+  CK(prim_of(c, l, v));
+  CK(launch_sch_turb(c->d_blks, c->cells.view(l - 1), v, c->w.prim, ld, fd, ts6, ts7, d, sn, vol,
+                     u, c->st));
   return CNS_OK;
 }
 
@@ -2005,9 +2009,10 @@ int cns_impli2_eqt_3d(cns_ctx* c, int l, const double* u, const double* dt, doub
   if (!c || bad_block(c, l) || !u || !dt || !v || !mu || !mut || !cfke || !sn || !vol ||
       !(cmt != 0.))
     return CNS_EINVAL;
-  if (!c->sa_w) CK(dev_alloc(c, &c->sa_w, (size_t)20 * c->lay.ld, false));
-  CK(launch_impli2(c->d_blks, c->faces, c->lines, c->cells.view(l - 1), l - 1, c->lay.ld, u, dt,
-                   v, mu, mut, cfke, sn, vol, cmt, c->sa_w, 0, c->d_lp2_ni, c->n_lp2_ni,
+  if (!c->sa_w) CK(dev_alloc(c, &c->sa_w, (size_t)20 * c->lay.ld));
+  CK(prim_of(c, l, v));
+  CK(launch_impli2(c->d_blks, c->lines, c->cells.view(l - 1), l - 1, c->lay.ld, u, dt, v,
+                   c->w.prim, mu, mut, cfke, sn, vol, cmt, c->sa_w, 0, c->d_lp2_ni, c->n_lp2_ni,
                    c->st));
   return CNS_OK;
 }

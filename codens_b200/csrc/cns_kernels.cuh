@@ -341,10 +341,9 @@ cudaError_t launch_fludcsa(long long n0, long long n1, const double* s6, const d
                            double* const fd[6], double sigma, cudaStream_t st);
 // met_roe2o / met_roe2oh (harten) of block l0 (all: -1): t, d are (ld, 7);
 // cells_ext covers i 0..ni, j 0..nj, k 0..nk
-cudaError_t launch_roe2o(const Blk* blks, const SpaceBuf* faces, Space cells_ext, int l0,
-                         int harten, double epsroe, double gam, double gam1, const double* t,
-                         long long ld, const double* sn, double* G, double* d,
-                         cudaStream_t st);
+cudaError_t launch_roe2o(const Blk* blks, Space cells_ext, int harten, double epsroe, double gam,
+                         double gam1, const double* t, const double* prim, long long ld,
+                         const double* sn, double* d, cudaStream_t st);
 
 // discrete adjoint of the FP64 Euler Roe iteration (cns_adjoint.cu)
 // face-flux Jacobians J[3 dirs][27 seeds][5][ld] (4 stencil cells x (W, p),
@@ -371,11 +370,10 @@ cudaError_t launch_precond_ta(const Blk* blks, Space cells, long long ld, const 
 // met_samut (real cells of block l0's space) and sch_turb (u, v, d: (ld, 7))
 cudaError_t launch_samut(const Blk* blks, Space cells, const double* v6, const double* mu,
                          double* mut, cudaStream_t st);
-cudaError_t launch_sch_turb(const Blk* blks, const SpaceBuf* faces, Space cells, int l0,
-                            const double* v, long long ld, const double* const fd[6],
-                            const double* ts6, const double* ts7, const double* d,
-                            const double* sn, const double* vol, double* G, double* u,
-                            cudaStream_t st);
+cudaError_t launch_sch_turb(const Blk* blks, Space cells, const double* v, const double* prim,
+                            long long ld, const double* const fd[6], const double* ts6,
+                            const double* ts7, const double* d, const double* sn,
+                            const double* vol, double* u, cudaStream_t st);
 
 // teq_grads over the cells of the space into out[3 nsc][ld]: mode 0 = the
 // velocity (nsc 3), mode 1 = the fields f[q][ld], mode 2 = the transport
@@ -397,11 +395,12 @@ cudaError_t launch_smsa(const Blk* blks, Space cells, long long ld, const double
 // reduced-precision forms; not bit-exact)
 // wall_ni: the first cells of the wall-law walls (nwall of them), whose
 // increments are zeroed before the update (impli2_eqt_3d.f90:384-405)
-cudaError_t launch_impli2(const Blk* blks, const SpaceBuf* faces, const SpaceBuf* lines,
-                          Space cells, int l0, long long ld, const double* u, const double* dt,
-                          double* v, const double* mu, const double* mut, const double* cfke,
-                          const double* sn, const double* vol, double cmt, double* w, int rcp,
-                          const long long* wall_ni, long long nwall, cudaStream_t st);
+cudaError_t launch_impli2(const Blk* blks, const SpaceBuf* lines, Space cells, int l0,
+                          long long ld, const double* u, const double* dt, double* v,
+                          const double* prim, const double* mu, const double* mut,
+                          const double* cfke, const double* sn, const double* vol, double cmt,
+                          double* w, int rcp, const long long* wall_ni, long long nwall,
+                          cudaStream_t st);
 
 // wall laws of the adiabatic wall-law walls 'lp2' (rbord.f90:377-379: vkar,
 // cllog, yp0; the SA cv1 and the nu~ floor epsk) on the cnt list entries

@@ -206,7 +206,8 @@ __global__ void __launch_bounds__(kTile) k_smsa(
   cfke[n] = fabs(dsm1 + dsm2 + dsdif);
 }
 
-// impli2_eqt_3d.f90:93-103: rv and the time-step part of the diagonal
+// impli2_eqt_3d.f90:93-103: rv and the time-step part of the diagonal; the
+// first iterate of the line sweeps is zero
 __global__ void __launch_bounds__(kTile) k_i2_cell(const Blk* __restrict__ blks, Space sp,
                                                    const double* __restrict__ v,
                                                    const double* __restrict__ mu,
@@ -215,49 +216,62 @@ __global__ void __launch_bounds__(kTile) k_i2_cell(const Blk* __restrict__ blks,
                                                    const double* __restrict__ cfke,
                                                    const double* __restrict__ vol, double cmt,
                                                    double* __restrict__ rv,
-                                                   double* __restrict__ cd) {
+                                                   double* __restrict__ cd,
+                                                   double* __restrict__ w6,
+                                                   double* __restrict__ w7) {
   int b, i, j, k;
   if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const long long n = cell_index(blks[b], i, j, k);
   rv[n] = (mu[n] + mut[n] / cmt) / v[n];
   cd[n] = vol[n] / dt[n] + cfke[n] * vol[n];
+  w6[n] = 0.;
+  w7[n] = 0.;
 }
 
-// impli2_eqt_3d.f90:104-160: face velocity flux u_dir and coefficient of one
-// face (boundary faces included)
-__global__ void __launch_bounds__(kTile) k_i2_face(const Blk* __restrict__ blks, Space sp,
-                                                   int dir, const double* __restrict__ v,
-                                                   long long ld, const double* __restrict__ sn,
-                                                   const double* __restrict__ vol,
-                                                   const double* __restrict__ rv,
-                                                   double* __restrict__ uf,
-                                                   double* __restrict__ ce) {
+// impli2_eqt_3d.f90:104-171 per real cell: the velocity fluxes and
+// coefficients of the six faces (the lower ones stored, and the upper one at
+// the end of each line) and the diagonal in the reference's order.  Interior
+// faces are evaluated by both their cells from stored velocities, in place of
+// a launch per direction, their divisions, and the diagonal's re-read:
+// 206 -> 100 us on a 2.1M-cell plate (cold).
+__global__ void __launch_bounds__(kTile) k_i2_coefs(const Blk* __restrict__ blks, Space sp,
+                                                    const double* __restrict__ prim,
+                                                    long long ld,
+                                                    const double* __restrict__ sn,
+                                                    const double* __restrict__ vol,
+                                                    const double* __restrict__ rv,
+                                                    double* __restrict__ uf,
+                                                    double* __restrict__ ce,
+                                                    double* __restrict__ cd) {
   int b, i, j, k;
   if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const long long n = cell_index(B, i, j, k);
-  const long long inc = ninc_of(B, dir), nl = n - inc;
-  const double s1 = sn_ptr(sn, B, dir, 0)[n], s2 = sn_ptr(sn, B, dir, 1)[n],
-               s3 = sn_ptr(sn, B, dir, 2)[n];
-  const double cnds = s1 * s1 + s2 * s2 + s3 * s3;
-  const double uu = 0.5 * (v[ld + n] / v[n] + v[ld + nl] / v[nl]);
-  const double vv = 0.5 * (v[2 * ld + n] / v[n] + v[2 * ld + nl] / v[nl]);
-  const double ww = 0.5 * (v[3 * ld + n] / v[n] + v[3 * ld + nl] / v[nl]);
-  const double u = 0.5 * (uu * s1 + vv * s2 + ww * s3);
-  uf[(long long)dir * ld + n] = u;
-  ce[(long long)dir * ld + n] = fabs(u) + (rv[n] + rv[nl]) * cnds / (vol[n] + vol[nl]);
-}
-
-// impli2_eqt_3d.f90:161-171
-__global__ void __launch_bounds__(kTile) k_i2_diag(const Blk* __restrict__ blks, Space sp,
-                                                   long long ld, const double* __restrict__ ce,
-                                                   double* __restrict__ cd) {
-  int b, i, j, k;
-  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
-  const Blk& B = blks[b];
-  const long long m = cell_index(B, i, j, k);
-  cd[m] = cd[m] + ce[m] + ce[m + 1] + ce[ld + m] + ce[ld + m + B.nid] + ce[2 * ld + m] +
-          ce[2 * ld + m + B.nijd];
+  double c = cd[n];
+#pragma unroll
+  for (int dir = 0; dir < 3; ++dir) {
+    const long long inc = ninc_of(B, dir);
+    const int p = dir == 0 ? i : (dir == 1 ? j : k);
+    const double *s0 = sn_ptr(sn, B, dir, 0), *s1 = sn_ptr(sn, B, dir, 1),
+                 *s2 = sn_ptr(sn, B, dir, 2);
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {  // face between h - inc and h
+      const long long h = n + (side ? inc : 0), l = h - inc;
+      const double x = s0[h], y = s1[h], z = s2[h];
+      const double cnds = x * x + y * y + z * z;
+      const double uu = 0.5 * (prim[h] + prim[l]);
+      const double vv = 0.5 * (prim[ld + h] + prim[ld + l]);
+      const double ww = 0.5 * (prim[2 * ld + h] + prim[2 * ld + l]);
+      const double u = 0.5 * (uu * x + vv * y + ww * z);
+      const double e = fabs(u) + (rv[h] + rv[l]) * cnds / (vol[h] + vol[l]);
+      if (side == 0 || p == nd_of(B, dir) - 1) {
+        uf[(long long)dir * ld + h] = u;
+        ce[(long long)dir * ld + h] = e;
+      }
+      c = c + e;
+    }
+  }
+  cd[n] = c;
 }
 
 // one alternating-line sweep of direction dir (impli2_eqt_3d.f90:172-291),
@@ -803,46 +817,41 @@ cudaError_t launch_teq_grads(const Blk* blks, Space cells, int mode, int nsc,
   return cudaGetLastError();
 }
 
-cudaError_t launch_impli2(const Blk* blks, const SpaceBuf* faces, const SpaceBuf* lines,
-                          Space cells, int l0, long long ld, const double* u, const double* dt,
-                          double* v, const double* mu, const double* mut, const double* cfke,
-                          const double* sn, const double* vol, double cmt, double* w,
-                          int rcp, const long long* wall_ni, long long nwall,
+cudaError_t launch_impli2(const Blk* blks, const SpaceBuf* lines, Space cells, int l0,
+                          long long ld, const double* u, const double* dt, double* v,
+                          const double* prim, const double* mu, const double* mut,
+                          const double* cfke, const double* sn, const double* vol, double cmt,
+                          double* w, int rcp, const long long* wall_ni, long long nwall,
                           cudaStream_t st) {
-  // scratch w: rv, cd, uf[3], ce[3], al, b6, b7, two iterates x (6, 7),
-  // the tridiagonal coefficients ta, tb, tc and right-hand sides d6, d7 of
-  // a sweep = 20 ld.  rv and the iterates start at zero (their ghost
-  // entries are the reference's zeroed rv and never-written neighbours);
-  // every other entry read is written first.
+  // scratch w, zeroed when allocated: rv, cd, uf[3], ce[3], al, b6, b7, two
+  // iterates x (6, 7), the tridiagonal coefficients ta, tb, tc and right-hand
+  // sides d6, d7 of a sweep = 20 ld.  The ghost entries of rv and of the
+  // iterates are never written (the reference's zeroed rv and never-written
+  // neighbours); every other entry read is written first.
   double *rv = w, *cd = w + ld, *uf = w + 2 * ld, *ce = w + 5 * ld, *al = w + 8 * ld,
          *b6 = w + 9 * ld, *b7 = w + 10 * ld;
   double* it[2][2] = {{w + 11 * ld, w + 12 * ld}, {w + 13 * ld, w + 14 * ld}};
   double *ta = w + 15 * ld, *tb = w + 16 * ld, *tc = w + 17 * ld, *d6 = w + 18 * ld,
          *d7 = w + 19 * ld;
-  cudaError_t e = cudaMemsetAsync(rv, 0, sizeof(double) * ld, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(w + 11 * ld, 0, sizeof(double) * 4 * ld, st);
-  if (e != cudaSuccess) return e;
   if (cells.ntiles == 0) return cudaSuccess;
   pdl(k_i2_cell, grid_of(cells), kTile, 0, st)(blks, cells, v, mu, mut, dt, cfke, vol, cmt, rv,
-                                              cd);
-  for (int dir = 0; dir < 3; ++dir) {
-    const Space sp = faces[dir].view(l0);
-    if (sp.ntiles > 0)
-      pdl(k_i2_face, grid_of(sp), kTile, 0, st)(blks, sp, dir, v, ld, sn, vol, rv, uf, ce);
-  }
-  pdl(k_i2_diag, grid_of(cells), kTile, 0, st)(blks, cells, ld, ce, cd);
+                                               cd, it[0][0], it[0][1]);
+  pdl(k_i2_coefs, grid_of(cells), kTile, 0, st)(blks, cells, prim, ld, sn, vol, rv, uf, ce, cd);
   int cur = 0;
   for (int dir = 0; dir < 3; ++dir) {
     const Space sp = lines[dir].view(l0);
     for (int sw = 0; sw < 2; ++sw) {
       pdl(k_i2_rhs, grid_of(cells), kTile, 0, st)(blks, cells, dir, ld, u, uf, ce, cd,
                                                  it[cur][0], it[cur][1], ta, tb, tc, d6, d7);
+      // launched only when the chip is empty: placed while the kernel before
+      // drains, the few one-warp CTAs crowd on the first free SMs (an iteration
+      // of the 2.1M-cell plate 3.64 against 3.43 ms)
       const int lg = grid_of(sp) * (kTile / kLineCta);
       if (sp.ntiles > 0 && rcp)
-        pdl(k_i2_line<true>, lg, kLineCta, 0, st)(blks, sp, dir, ta, tb, tc, d6, d7, al, b6, b7,
+        k_i2_line<true><<<lg, kLineCta, 0, st>>>(blks, sp, dir, ta, tb, tc, d6, d7, al, b6, b7,
                                                  it[1 - cur][0], it[1 - cur][1]);
       else if (sp.ntiles > 0)
-        pdl(k_i2_line<false>, lg, kLineCta, 0, st)(blks, sp, dir, ta, tb, tc, d6, d7, al, b6,
+        k_i2_line<false><<<lg, kLineCta, 0, st>>>(blks, sp, dir, ta, tb, tc, d6, d7, al, b6,
                                                   b7, it[1 - cur][0], it[1 - cur][1]);
       cur = 1 - cur;
     }
