@@ -65,6 +65,7 @@ struct cns_ctx {
   int nsm = 0;                 // streaming multiprocessors of the device
   bool adj_fp32 = false;     // L^T of the prepared adjoint in FP32 (precision != 0)
   TileBuf tiles64, tiles32;   // 2.5D tiles of the FP64 and the FP32 Jacobi sweeps
+  TileBuf tiles64_blk;        // the FP64 tiles of one-block launches
   TileBuf tiles_res;          // 2.5D tiles of the fused residual
   bool res_fused = false;     // residual: fused kernel (tiles_res) or face kernels + accumulate
   bool tuned64 = false, tuned32 = false;
@@ -197,13 +198,14 @@ cudaError_t build_space(cns_ctx* c, SpaceBuf& s, F ext_of) {
 // iteration, a batch of 24 uneven boxes 1.56 -> 1.52 ms.
 constexpr double kTilePrologue = 2.5;
 
-int sweep_depth(const HostLayout& lay, int ti, int tj, int kc, int slots) {
+int sweep_depth(const Blk* b0, const Blk* b1, int ti, int tj, int kc, int slots) {
   int best = kc;
   double cost = 1e300;
   for (int d = kc; d >= 1 && slots > 0; --d) {
     long long n = 0;
     int deep = 0;
-    for (const Blk& B : lay.blks) {
+    for (const Blk* p = b0; p < b1; ++p) {
+      const Blk& B = *p;
       n += (long long)((B.ni - 2 + ti) / ti) * ((B.nj - 2 + tj) / tj) * ((B.nk - 2 + d) / d);
       deep = std::max(deep, std::min(d, B.nk - 1));
     }
@@ -216,17 +218,25 @@ int sweep_depth(const HostLayout& lay, int ti, int tj, int kc, int slots) {
   return best;
 }
 
+int sweep_depth(const HostLayout& lay, int ti, int tj, int kc, int slots) {
+  return sweep_depth(lay.blks.data(), lay.blks.data() + lay.blks.size(), ti, tj, kc, slots);
+}
+
 // the 2.5D sweep tiles: patches of ti x tj columns, at most kc planes deep
-// (slots > 0: cut to sweep_depth), block by block
-cudaError_t build_tiles(cns_ctx* c, TileBuf& t, int ti, int tj, int kc, int slots = 0) {
+// (slots > 0: cut to sweep_depth for a launch of all blocks, or, alone, for
+// launches of one block), block by block
+cudaError_t build_tiles(cns_ctx* c, TileBuf& t, int ti, int tj, int kc, int slots = 0,
+                        bool alone = false) {
   dev_free(c, t.d_tile);
   t.d_tile = nullptr;
-  const int depth = sweep_depth(c->lay, ti, tj, kc, slots);
+  int depth = sweep_depth(c->lay, ti, tj, kc, slots);
+  t.blk_depth.assign(c->lay.blks.size(), depth);
   std::vector<int4> tl;
   t.blk_tile0.assign(c->lay.blks.size() + 1, 0);
   for (size_t b = 0; b < c->lay.blks.size(); ++b) {
     const Blk& B = c->lay.blks[b];
     t.blk_tile0[b] = (int)tl.size();
+    if (alone) depth = t.blk_depth[b] = sweep_depth(&B, &B + 1, ti, tj, kc, slots);
     for (int k0 = 1; k0 <= B.nk - 1; k0 += depth)
       for (int j0 = 1; j0 <= B.nj - 1; j0 += tj)
         for (int i0 = 1; i0 <= B.ni - 1; i0 += ti) tl.push_back(make_int4((int)b, i0, j0, k0));
@@ -248,7 +258,14 @@ int sweep_slots(cns_ctx* c, bool fp32, int ti, int tj) {
 }
 
 cudaError_t build_sweep_tiles(cns_ctx* c, bool fp32, TileBuf& t, int ti, int tj, int kc) {
-  return build_tiles(c, t, ti, tj, kc, sweep_slots(c, fp32, ti, tj));
+  const int slots = sweep_slots(c, fp32, ti, tj);
+  cudaError_t e = build_tiles(c, t, ti, tj, kc, slots);
+  // the per-routine calls go block by block: a block of 250k cells cut for a
+  // launch of two is 210 CTAs on 444 slots (the driver's iteration 1.58 ms
+  // against 1.21 with its own cut)
+  if (e == cudaSuccess && &t == &c->tiles64)
+    e = build_tiles(c, c->tiles64_blk, ti, tj, kc, slots, true);
+  return e;
 }
 
 // the FP32 sweep tiles run as a persistent launch: one CTA per resident slot
@@ -2359,7 +2376,8 @@ static int implimf(cns_ctx* c, int l, int eu, const double* u, const double* dt,
   CK(prim_of(c, l, dv));
   Scheme sc = c->sc;
   if (sc.kfmg == 3) sc.dt1min = dtpas;
-  CK(launch_implicit(c->d_blks, c->cells.view(l - 1), c->tiles64.view(l - 1), c->ph, sc, eu,
+  const Tiles tl = l == 0 ? c->tiles64.view() : c->tiles64_blk.view(l - 1);
+  CK(launch_implicit(c->d_blks, c->cells.view(l - 1), tl, c->ph, sc, eu,
                      lmx, du, ddt, dv, dd, dmu, dmut, sn_base(c, l, dsn), dvol, dps, dcson, 0,
                      c->w, 0, c->st));
   CK(sg.finish());

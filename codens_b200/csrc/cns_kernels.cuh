@@ -91,6 +91,7 @@ cudaError_t launch_dual_update(const Blk* blks, Space cells, long long ld, int m
 struct TileBuf {
   int ti = 0, tj = 0, kc = 0, ntiles = 0;
   int depth = 0;  // planes of a tile, at most kc (sweep_depth)
+  std::vector<int> blk_depth;  // and of the tiles of a block in a one-block launch
   std::vector<int> blk_tile0;  // first tile of each block, size nblk+1
   int4* d_tile = nullptr;
   int* sched = nullptr;  // persistent launch: tile counter pair (device), else null
@@ -111,6 +112,7 @@ struct TileBuf {
     } else {
       t.tile0 = blk_tile0[l0];
       t.ntiles = blk_tile0[l0 + 1] - blk_tile0[l0];
+      t.kc = blk_depth[l0];
     }
     return t;
   }
