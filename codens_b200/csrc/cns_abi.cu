@@ -882,8 +882,8 @@ cudaError_t ensure_mixed(cns_ctx* c) {
 cudaError_t refresh_sn32(cns_ctx* c, const double* sn) {
   cudaError_t e = launch_to_float(sn, c->w.sn32, 9 * c->lay.ld, c->st);
   if (e == cudaSuccess)
-    e = launch_pack_faces32(c->d_blks, (int)c->lay.blks.size(), c->lay.ncells, c->w.sn32,
-                            c->w.snc32, c->st);
+    e = launch_pack_faces32(c->d_blks, (int)c->lay.blks.size(), c->lay.ncells, c->lay.ld,
+                            c->w.sn32, c->w.snc32, c->st);
   c->tiles32.faces = c->w.snc32;
   return e;
 }
@@ -992,7 +992,7 @@ cudaError_t enqueue_step_mixed(cns_ctx* c, MixedMode mode, bool first, bool dt_o
   if (e == cudaSuccess)
     e = launch_coefficients32(c->d_blks, all, !c->sc.ns, ld,
                               c->sc.kfmg == 3 ? c->sc.dt1min : 0., s.dt, s.vol, w.cq32,
-                              w.cv32, w.sn32, w.coefe32, w.coefdiag32, w.snc32, w.u32,
+                              w.cv32, w.sn32, w.coefdiag32, w.snc32, w.u32,
                               c->sc.lmax >= 1 && !point ? w.d32pp[0] : nullptr,
                               point ? w.pt32[0] : nullptr, w.st32, c->ph,
                               c->sc.ns ? 0 : c->sc.qfix_dfez, c->st);

@@ -161,7 +161,7 @@ struct Work {
   float2* cv32 = nullptr;     // and (vol, rv) [ld]
   void* sweep_maps = nullptr; // the box staging's tensor maps (device)
   double *corr = nullptr, *ur32 = nullptr;
-  float4* snc32 = nullptr;  // [ld][3]: half lower-face areas and their coefficients
+  float4* snc32 = nullptr;  // [3][ld]: half lower-face areas and their coefficients
 };
 
 cudaError_t launch_metric(const HostLayout& lay, const Blk* dblks, const Bnd& bd,
@@ -558,20 +558,20 @@ cudaError_t launch_to_float(const double* a, float* b, long long n, cudaStream_t
 // corr = u64 - u_r32 on the real cells (defect correction)
 cudaError_t launch_defect(const Blk* blks, Space cells, long long ld, const double* u64,
                           const double* ur32, double* corr, cudaStream_t st);
-// the FP32 implicit coefficients (coefe32 per face, coefdiag32 per cell) of
+// the FP32 implicit coefficients (snc32 per face, coefdiag32 per cell) of
 // the mixed sweeps in one pass over the real cells
 // (the per-cell inputs cq32, cv32 of PrimShadow); the first iterate in d1, or
 // with its increments in p1
 cudaError_t launch_coefficients32(const Blk* blks, Space cells, int eu, long long ld,
                                   double dtpas, const double* dt, const double* vol,
                                   const float4* cq32, const float2* cv32, const float* sn32,
-                                  float* coefe32, float* coefdiag32, float4* snc32,
+                                  float* coefdiag32, float4* snc32,
                                   const float* u32, float* d1, float4* p1, const float* st32,
                                   Phys ph, int qfix, cudaStream_t st);
-// the face lanes of the FP32 sweep's pack: snc[3n + dir].xyz = S/2 of cell n's
+// the face lanes of the FP32 sweep's pack: snc[dir * ld + n].xyz = S/2 of cell n's
 // lower face in dir (exact halves of sn32), .w = 0 until k_coef32 writes it
-cudaError_t launch_pack_faces32(const Blk* blks, int nblk, long long ncells, const float* sn32,
-                                float4* snc32, cudaStream_t st);
+cudaError_t launch_pack_faces32(const Blk* blks, int nblk, long long ncells, long long ld,
+                                const float* sn32, float4* snc32, cudaStream_t st);
 // FP64 face fluxes with FMA contraction (the mixed form's residual; agrees
 // with launch_face_flux_t<double> to FP64 rounding, not bit for bit)
 cudaError_t launch_face_flux_fma(const Blk* blks, const SpaceBuf* faces, int l0, Phys ph,

@@ -101,7 +101,7 @@ __device__ __forceinline__ float face_coef(const float4 qh, const float4 ql, flo
 // the implicit coefficients of the FP32 sweeps in one pass (the FP32 form of
 // implimf_3d.f90:111-203 / implimf_eu.f90:124-170): each real cell evaluates
 // the spectral radii of its six faces, stores the lower faces (and the upper
-// one at the end of each line) and sums the diagonal in the reference order.
+// one at the end of each line) in the sweep's face pack and sums the diagonal in the reference order.
 // Every interior face is evaluated by both its cells (cheaper than a second
 // pass over memory); a neighbour's inputs are two vector loads of the packed
 // cq32 = (u, v, w, c) and cv32 = (vol, rv) the primitive kernel writes.
@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(kTile) k_coef32(
     const Blk* __restrict__ blks, Space sp, long long ld, double dtpas,
     const double* __restrict__ dt, const double* __restrict__ vol,
     const float4* __restrict__ cq, const float2* __restrict__ cv,
-    const float* __restrict__ sn, float* __restrict__ coefe, float* __restrict__ coefdiag,
+    const float* __restrict__ sn, float* __restrict__ coefdiag,
     float4* __restrict__ snc, const float* __restrict__ u32, float* __restrict__ d1,
     float4* __restrict__ p1, const float* __restrict__ st32, float gam1, float pinfl, int qfix) {
   int b, i, j, k;
@@ -141,17 +141,13 @@ __global__ void __launch_bounds__(kTile) k_coef32(
     const float rvu = (EU || p >= nd - 1) ? 0.f : cu.y;
     const float cel = face_coef<EU>(q0, ql, c0.x, cl.x, s0[n], s1[n], s2[n], rv0, rvl);
     const float ceu = face_coef<EU>(qu, q0, cu.x, c0.x, s0[nu], s1[nu], s2[nu], rvu, rv0);
-    coefe[(long long)dir * ld + n] = cel;
-    if (p == nd - 1) coefe[(long long)dir * ld + nu] = ceu;
-    if (snc) {
-      // the sweep's face pack, whole 16-byte entries (half the face's area
-      // vector, as k_pack_faces32 writes it, and its coefficient): a store of
-      // the coefficient lane alone would make the memory system fetch the
-      // rest of each entry first
-      snc[3 * n + dir] = make_float4(0.5f * s0[n], 0.5f * s1[n], 0.5f * s2[n], cel);
-      if (p == nd - 1)
-        snc[3 * nu + dir] = make_float4(0.5f * s0[nu], 0.5f * s1[nu], 0.5f * s2[nu], ceu);
-    }
+    // the sweep's face pack, whole 16-byte entries (half the face's area
+    // vector, as k_pack_faces32 writes it, and its coefficient): a store of
+    // the coefficient lane alone would make the memory system fetch the rest
+    // of each entry first
+    float4* sd = snc + (long long)dir * ld;
+    sd[n] = make_float4(0.5f * s0[n], 0.5f * s1[n], 0.5f * s2[n], cel);
+    if (p == nd - 1) sd[nu] = make_float4(0.5f * s0[nu], 0.5f * s1[nu], 0.5f * s2[nu], ceu);
     cd = cd + cel + ceu;
   }
   if (!EU && dtpas > 0.) cd = cd + (float)(1.5 * vol[n] / dtpas);
@@ -176,18 +172,18 @@ __global__ void __launch_bounds__(kTile) k_coef32(
 cudaError_t launch_coefficients32(const Blk* blks, Space cells, int eu, long long ld,
                                   double dtpas, const double* dt, const double* vol,
                                   const float4* cq32, const float2* cv32, const float* sn32,
-                                  float* coefe32, float* coefdiag32, float4* snc32,
+                                  float* coefdiag32, float4* snc32,
                                   const float* u32, float* d1, float4* p1, const float* st32,
                                   Phys ph, int qfix, cudaStream_t st) {
   if (cells.ntiles == 0) return cudaSuccess;
   const float g1 = (float)ph.gam1, pi = (float)ph.pinfl;
   if (eu)
     pdl(k_coef32<true>, grid_of(cells), kTile, 0, st)(blks, cells, ld, dtpas, dt, vol, cq32,
-                                                     cv32, sn32, coefe32, coefdiag32, snc32,
+                                                     cv32, sn32, coefdiag32, snc32,
                                                      u32, d1, p1, st32, g1, pi, qfix);
   else
     pdl(k_coef32<false>, grid_of(cells), kTile, 0, st)(blks, cells, ld, dtpas, dt, vol, cq32,
-                                                      cv32, sn32, coefe32, coefdiag32, snc32,
+                                                      cv32, sn32, coefdiag32, snc32,
                                                       u32, d1, p1, st32, g1, pi, qfix);
   return cudaGetLastError();
 }
@@ -195,7 +191,7 @@ cudaError_t launch_coefficients32(const Blk* blks, Space cells, int eu, long lon
 namespace {
 // the face lanes of the sweep's pack for every cell of every block
 __global__ void __launch_bounds__(256) k_pack_faces32(const Blk* __restrict__ blks, int nblk,
-                                                     long long ncells,
+                                                     long long ncells, long long ld,
                                                      const float* __restrict__ sn,
                                                      float4* __restrict__ snc) {
   pdl_sync();
@@ -207,15 +203,15 @@ __global__ void __launch_bounds__(256) k_pack_faces32(const Blk* __restrict__ bl
   if (q >= B.npc + B.nnn) return;
 #pragma unroll
   for (int dir = 0; dir < 3; ++dir)
-    snc[3 * q + dir] = make_float4(0.5f * sn_ptr(sn, B, dir, 0)[q], 0.5f * sn_ptr(sn, B, dir, 1)[q],
+    snc[(long long)dir * ld + q] = make_float4(0.5f * sn_ptr(sn, B, dir, 0)[q], 0.5f * sn_ptr(sn, B, dir, 1)[q],
                                    0.5f * sn_ptr(sn, B, dir, 2)[q], 0.f);
 }
 }  // namespace
 
-cudaError_t launch_pack_faces32(const Blk* blks, int nblk, long long ncells, const float* sn32,
-                                float4* snc32, cudaStream_t st) {
+cudaError_t launch_pack_faces32(const Blk* blks, int nblk, long long ncells, long long ld,
+                                const float* sn32, float4* snc32, cudaStream_t st) {
   if (ncells > 0)
-    pdl(k_pack_faces32, (int)((ncells + 255) / 256), 256, 0, st)(blks, nblk, ncells, sn32, snc32);
+    pdl(k_pack_faces32, (int)((ncells + 255) / 256), 256, 0, st)(blks, nblk, ncells, ld, sn32, snc32);
   return cudaGetLastError();
 }
 
@@ -332,9 +328,8 @@ __global__ void __launch_bounds__(kTile) k_sweep_point32(
   if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const long long n = cell_index(B, i, j, k), pn = pad_index(B, i, j, k), pld = B.pld;
-  const float4 fi = faces[3 * n], fj = faces[3 * n + 1], fk = faces[3 * n + 2],
-               fiu = faces[3 * (n + 1)], fju = faces[3 * (n + B.nid) + 1],
-               fku = faces[3 * (n + B.nijd) + 2];
+  const float4 fi = faces[n], fj = faces[ld + n], fk = faces[2 * ld + n], fiu = faces[n + 1],
+               fju = faces[ld + n + B.nid], fku = faces[2 * ld + n + B.nijd];
   float acc[5];
 #pragma unroll
   for (int c = 0; c < 5; ++c) acc[c] = -a.u[c * ld + n];
@@ -620,7 +615,7 @@ __device__ __forceinline__ bool sweep_f32_tile(const int4 t, const Blk* __restri
   const int q0 = (ty + 1) * NX + tx + 1;
   // the lower k face of the own cell, carried from plane to plane (the
   // upper k face of plane k is the lower one of plane k+1)
-  float4 fkc = own ? tl.faces[3 * cell_index(B, i, j, kbeg) + 2]
+  float4 fkc = own ? tl.faces[2 * ld + cell_index(B, i, j, kbeg)]
                    : make_float4(0.f, 0.f, 0.f, 0.f);
   for (int k = kbeg; k < kend; ++k) {
     // this cell's own inputs, in flight across the barrier
@@ -636,11 +631,11 @@ __device__ __forceinline__ bool sweep_f32_tile(const int4 t, const Blk* __restri
     if (own) {
 #pragma unroll
       for (int c = 0; c < 5; ++c) uu[c] = u[c * ld + n];
-      fi = tl.faces[3 * n];
-      fj = tl.faces[3 * n + 1];
-      fiu = tl.faces[3 * (n + 1)];
-      fju = tl.faces[3 * (n + B.nid) + 1];
-      fku = tl.faces[3 * (n + B.nijd) + 2];
+      fi = tl.faces[n];
+      fj = tl.faces[ld + n];
+      fiu = tl.faces[n + 1];
+      fju = tl.faces[ld + n + B.nid];
+      fku = tl.faces[2 * ld + n + B.nijd];
       cd = a.coefdiag[n];
     }
     fkc = fku;
