@@ -861,7 +861,7 @@ cudaError_t ensure_mixed(cns_ctx* c) {
   if (e == cudaSuccess) e = dev_alloc(c, &w.st32, (size_t)(6 * ldp));
   if (e == cudaSuccess) e = dev_alloc(c, &w.cq32, (size_t)ld);
   if (e == cudaSuccess) e = dev_alloc(c, &w.cv32, (size_t)ld);
-  for (int q = 0; q < 2 && e == cudaSuccess && point_sweeps(c->lay); ++q)
+  for (int q = 0; q < 2 && e == cudaSuccess && c->lay.nreal <= kPoint32; ++q)
     e = dev_alloc(c, &w.pt32[q], (size_t)(4 * ldp), false);
   if (e == cudaSuccess) {
     std::vector<unsigned char> maps;
@@ -1437,9 +1437,11 @@ int cns_create(const cns_layout_t* layout, const cns_phys_t* phys,
   if (e == cudaSuccess) e = dev_alloc(c, &c->w.coefe, (size_t)(3 * ld));
   if (e == cudaSuccess) e = dev_alloc(c, &c->w.coefdiag, (size_t)ld);
   if (e == cudaSuccess) e = dev_alloc(c, &c->w.rv, (size_t)ld);
+  c->w.point_eu = c->lay.nreal <= kPointEuler64;
+  c->w.point_ns = c->lay.nreal <= kPointNs64;
   for (int q = 0; q < 2 && e == cudaSuccess; ++q) {
     e = dev_alloc(c, &c->w.dpp[q], (size_t)(5 * ld));
-    if (e == cudaSuccess && point_sweeps(c->lay))
+    if (e == cudaSuccess && (c->w.point_eu || c->w.point_ns))
       e = dev_alloc(c, &c->w.pt[q], (size_t)(7 * ld), false);
   }
   if (e == cudaSuccess) e = dev_alloc(c, &c->w.normpart, (size_t)(15 * c->cells.ntiles));

@@ -747,7 +747,7 @@ __global__ void __launch_bounds__(kTile) k_impl_coefs(
 
 // ---------------------------------------------------------------------------
 // Point sweep: the Jacobi sweep of grids small enough for every array of the
-// sweeps to stay in L2 (point_sweeps() in cns_kernels.cuh has the line and
+// sweeps to stay in L2 (kPointEuler64 in cns_kernels.cuh has the lines and
 // both sides' figures).  One thread per cell reads its own and its six
 // neighbours' iterate and flux increment (d, f), evaluates the six faces and
 // the new iterate with the expressions and order of the 2.5D sweep, then the
@@ -1213,7 +1213,7 @@ cudaError_t launch_implicit(const Blk* blks, Space cells, Tiles tl, Phys ph, Sch
   const long long ld = w.ld;
   if (cells.ntiles == 0) return cudaSuccess;
   const int qfix = eu ? sc.qfix_dfez : 0;
-  const bool point = w.pt[0] && lmx >= 2;
+  const bool point = (eu ? w.point_eu : w.point_ns) && lmx >= 2;
   // dtpas > 0: dual time stepping with physical step dtpas
   cudaError_t e = launch_implicit_coefficients(
       blks, cells, ph, eu, sc.kfmg == 3 ? sc.dt1min : 0., dt, v, w.prim, mu, mut, sn, vol, cson,

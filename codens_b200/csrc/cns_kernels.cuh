@@ -118,15 +118,17 @@ struct TileBuf {
   }
 };
 
-// Whether a layout's Jacobi sweeps run as point sweeps (one thread per cell
-// from stored increments) instead of 2.5D tiles: while all that the sweeps
-// touch stays in the 126 MB L2.  Whole iterations of ten sweeps, tiles
-// against points: 64x32x32 cells 161 -> 113 us (Euler), 197 -> 135
-// (Navier-Stokes), mixed 131 -> 89 and 145 -> 105; 131k cells 241 -> 189,
-// 313 -> 226, 150 -> 132, 178 -> 158; at 196k FP64 is even (289 and 306, 355
-// and 351).
-constexpr long long kPointCells = 200000;
-inline bool point_sweeps(const HostLayout& lay) { return lay.nreal <= kPointCells; }
+// The layouts (real cells) whose Jacobi sweeps run as point sweeps (one thread
+// per cell from stored increments) instead of 2.5D tiles: while most of what
+// the sweeps touch stays in the 126 MB L2; the Navier-Stokes increments cost
+// the tiles six divisions a cell and ring cell, so their line lies higher, and
+// FP32 has half the bytes.  Whole iterations of ten sweeps, tiles against
+// points, Euler and Navier-Stokes: 64x32x32 cells 161 -> 113 us, 197 -> 135;
+// 131k 241 -> 189, 313 -> 226; 196k 289 and 305, 355 and 350; 262k 397 and
+// 419, 514 -> 479; 393k 553 and 610, 674 and 685.  FP32: 65k 131 -> 89, 145 ->
+// 105; 196k 235 -> 171, 266 -> 201; 262k 261 -> 222, 296 -> 261; 393k 348 ->
+// 338, 400 -> 397; 524k 428 and 449, 496 and 526.
+constexpr long long kPointEuler64 = 180000, kPointNs64 = 300000, kPoint32 = 400000;
 
 // per-step scratch (device)
 struct Work {
@@ -143,6 +145,7 @@ struct Work {
   double* rv = nullptr;       // [ld]
   double* dpp[2] = {nullptr, nullptr};   // Jacobi iterates, [5][ld] each
   double2* pt[2] = {nullptr, nullptr};   // point sweeps: (d, f) packed, [7][ld] each
+  bool point_eu = false, point_ns = false;  // FP64 point sweeps by equations
   float4* pt32[2] = {nullptr, nullptr};  // and in FP32, padded [4][ldp] each
   double* normpart = nullptr; // per tile partial norms [ntiles][15]
   double* norms = nullptr;    // [16]
@@ -279,7 +282,7 @@ struct Sweep32 {
   int nblk;
   int* status;         // bit 4: a box wait gave up
 };
-// sweeps 2..lmx of a small grid (point_sweeps): the first iterate with its
+// sweeps 2..lmx of a small grid (kPoint32): the first iterate with its
 // increments in pt[0], the final iterate in d_out
 cudaError_t launch_point_sweeps32(const Blk* blks, Space cells, Phys ph, Scheme sc, int eu,
                                   int lmx, long long ld, const Sweep32& a, const float4* faces,

@@ -557,8 +557,10 @@ int cns_sch_dual(cns_ctx *ctx, int l, double *u, const double *v, int icycle,
                  const double *vol, const double *ptdual);
 
 /* Jacobi sweep tiling (no counterpart in the reference).  Every sweep after
- * the first runs 2.5D-blocked over patches of ti x tj cell columns, kc
- * planes deep.  The first fused iteration of each precision tunes the tiling
+ * the first runs 2.5D-blocked over patches of ti x tj cell columns, at most kc
+ * planes deep (fewer where that fills the last wave of CTAs better); layouts
+ * small enough for the L2 cache run one thread per cell instead and use no
+ * tiles (the same bits).  The first fused iteration of each precision tunes the tiling
  * on its own data (no result depends on it: the FP32 sweeps round every
  * operation explicitly).  cns_sweep_tiles returns {ti, tj, kc, source} of
  * precision 0 (FP64) or 1/2 (FP32 sweeps), source 0 = the default or a tiling

@@ -1,8 +1,8 @@
 """The two forms of the Jacobi sweeps: point sweeps (small layouts) and 2.5D
-tiles (larger ones) give the same bits.  Four independent boxes, each small
+tiles (larger ones) give the same bits.  Six independent boxes, each small
 enough for point sweeps, together make a layout of 2.5D tiles: every box of
 the batch must end as it does alone, for every patch shape and precision; and
-a box on each side of the line equals the oracle."""
+boxes at the lines equal the oracle."""
 import numpy as np
 import pytest
 
@@ -12,7 +12,8 @@ from ._helpers import assert_equal_bits, oracle_prepared, real
 
 pytestmark = pytest.mark.gpu
 
-POINT_CELLS = 200000
+# the largest layouts of point sweeps: FP64 Euler, FP64 Navier-Stokes, FP32
+POINT_EULER64, POINT_NS64, POINT_32 = 180000, 300000, 400000
 
 
 def _run(case, nsteps, precision, tiles=None):
@@ -32,14 +33,14 @@ def _run(case, nsteps, precision, tiles=None):
 @pytest.mark.parametrize("ns", [0, 1])
 def test_point_equals_tiled(cuda, precision, ns):
     def batch():
-        bt = cases.batch_case(ncase=4, side=(37, 45), seed=6, qfix_dfez=1 - ns)
+        bt = cases.batch_case(ncase=6, side=(40, 47), seed=6, qfix_dfez=1 - ns)
         bt.scheme.ns = ns
         bt.phys.reynz = 1.0e4
         return bt
     bt = batch()
-    assert bt.layout.nreal > POINT_CELLS > max(b.nreal for b in bt.layout.blocks)
+    assert bt.layout.nreal > POINT_32 and max(b.nreal for b in bt.layout.blocks) < POINT_EULER64
     alone = []
-    for ib in range(4):
+    for ib in range(bt.layout.nblk):
         m = cases.batch_member(bt, ib)
         alone.append(_run(m, 3, precision)[:, m.layout.blocks[0].real_cells()])
     for tiles in ((32, 4, 3), (32, 8, 16), (16, 8, 5), (16, 16, 64)):
@@ -48,10 +49,11 @@ def test_point_equals_tiled(cuda, precision, ns):
             assert_equal_bits(v[:, bt.layout.blocks[ib].real_cells()], want, f"{tiles} box {ib}")
 
 
-# 200000 cells is the last point-sweep size; odd sides, one-cell directions
-@pytest.mark.parametrize("cells", [(50, 50, 80), (67, 53, 57), (129, 2, 3), (1, 33, 5)])
-@pytest.mark.parametrize("ns", [0, 1])
-def test_fused_step_bits_at_the_line(cuda, cells, ns):
+# the last point-sweep size and the first tiled one; odd sides, one-cell directions
+@pytest.mark.parametrize("ns,cells", [
+    (0, (60, 50, 60)), (0, (61, 59, 51)), (1, (100, 60, 50)), (1, (67, 67, 67)),
+    (0, (129, 2, 3)), (1, (129, 2, 3)), (0, (1, 33, 5)), (1, (1, 33, 5))])
+def test_fused_step_bits_at_the_line(cuda, ns, cells):
     case = cases.box_case(cells, seed=7, ns=bool(ns), skew=0.01, reynz=1.0e4,
                           qfix_dfez=1 - ns, lmax=4)
     orc, st = oracle_prepared(case)
