@@ -367,7 +367,8 @@ cudaError_t prim_of(cns_ctx* c, int l, const double* v) {
 // the residual of one block set: (optional) limiter ratios, face fluxes,
 // accumulation into u; the primitive velocities must be current
 cudaError_t residual(cns_ctx* c, int l0, double* u, const double* v,
-                     const double* tau, const double* sn, const double* ps) {
+                     const double* tau, const double* sn, const double* ps,
+                     bool faces_only = false) {
   const long long ld = c->lay.ld;
   cudaError_t e = cudaSuccess;
   // WENO5 (no limiter) reads the stresses whatever the equations
@@ -382,7 +383,7 @@ cudaError_t residual(cns_ctx* c, int l0, double* u, const double* v,
   if (e == cudaSuccess)
     e = launch_face_flux(c->d_blks, c->faces, l0, c->ph, c->sc, v, c->w.prim, ld, ps, tau,
                          sn, c->w.R, c->w.G, c->st, c->w.V);
-  if (e == cudaSuccess)
+  if (e == cudaSuccess && !faces_only)
     e = launch_accumulate(c->d_blks, c->cells.view(l0), c->w.G, ld, u, c->st, c->w.V);
   return e;
 }
@@ -567,6 +568,14 @@ cudaError_t ensure_dis(cns_ctx* c) {
 }
 
 bool jameson(const cns_ctx* c) { return c->sc.ischema <= 4; }
+
+// whether the FP64 iteration's coefficient kernel sums the face fluxes into
+// the residual: the families with a face buffer and nothing between the
+// residual and the implicit phase (dual time's term)
+bool sum_in_coefs(const cns_ctx* c) {
+  return !jameson(c) && c->sc.ischema != 12 && c->sc.kfmg != 3 &&
+         !(c->res_fused && residual_fused_ok(c->sc));
+}
 
 cudaError_t ensure_dtpart(cns_ctx* c) {
   if (c->w.dtpart) return cudaSuccess;
@@ -809,17 +818,18 @@ cudaError_t enqueue_step(cns_ctx* c, bool first, bool dt_on) {
     if (e == cudaSuccess)
       e = enqueue_cllparoi1(c, s.v, s.mu, s.mut, c->sa_dist, s.ztemp, s.tau);
   }
+  const bool sum = sum_in_coefs(c);
   if (e == cudaSuccess) {
     if (jameson(c))
       e = launch_sch_jameson(c->d_blks, c->faces, all, -1, c->sc.ns, c->ph.pinfl, s.v, ld,
                              s.pression, s.tau, s.sn, c->w.dis, c->w.G, s.u, nullptr, c->st);
     else
-      e = residual(c, -1, s.u, s.v, weno_euler(c) ? c->w.tau0 : s.tau, s.sn, s.pression);
+      e = residual(c, -1, s.u, s.v, weno_euler(c) ? c->w.tau0 : s.tau, s.sn, s.pression, sum);
   }
   if (e == cudaSuccess && c->sc.kfmg == 3) e = enqueue_dual(c, nullptr);
   if (e == cudaSuccess)
     e = launch_implicit(c->d_blks, all, c->tiles64.view(-1), c->ph, c->sc, !c->sc.ns,
-                        c->sc.lmax, s.u, s.dt, s.v, nullptr, s.mu, s.mut, s.sn, s.vol,
+                        c->sc.lmax, s.u, sum, s.dt, s.v, nullptr, s.mu, s.mut, s.sn, s.vol,
                         s.pression, s.cson, 1, c->w, 1, c->st);
   if (e == cudaSuccess)
     e = finalize_norms(c);
@@ -2273,9 +2283,8 @@ int cns_adjoint_prepare(cns_ctx* c) {
                   c->d_idd_ents, c->d_idd_work, c->st));
   CK(launch_prim(0, c->lay.ncells, s.v, ld, c->w.prim, c->st));
   CK(launch_implicit_coefficients(c->d_blks, all, c->ph, 1, 0., s.dt, s.v, c->w.prim, s.mu,
-                                  s.mut, s.sn, s.vol, s.cson, nullptr, 0, nullptr, nullptr,
-                                  nullptr, 0,
-                                  c->w, c->st));
+                                  s.mut, s.sn, s.vol, s.cson, nullptr, 0, 0, nullptr, nullptr,
+                                  nullptr, 0, c->w, c->st));
   CK(launch_face_jac(c->d_blks, c->faces, c->ph, c->sc, s.v, s.pression, ld, s.sn, c->adj_J,
                      c->st));
   if (c->sc.precision != 0) {
@@ -2379,9 +2388,9 @@ static int implimf(cns_ctx* c, int l, int eu, const double* u, const double* dt,
   Scheme sc = c->sc;
   if (sc.kfmg == 3) sc.dt1min = dtpas;
   const Tiles tl = l == 0 ? c->tiles64.view() : c->tiles64_blk.view(l - 1);
-  CK(launch_implicit(c->d_blks, c->cells.view(l - 1), tl, c->ph, sc, eu,
-                     lmx, du, ddt, dv, dd, dmu, dmut, sn_base(c, l, dsn), dvol, dps, dcson, 0,
-                     c->w, 0, c->st));
+  CK(launch_implicit(c->d_blks, c->cells.view(l - 1), tl, c->ph, sc, eu, lmx,
+                     const_cast<double*>(du), 0, ddt, dv, dd, dmu, dmut, sn_base(c, l, dsn), dvol,
+                     dps, dcson, 0, c->w, 0, c->st));
   CK(sg.finish());
   return CNS_OK;
 }

@@ -691,8 +691,14 @@ __device__ __forceinline__ void radius_cell(const double* __restrict__ v,
 // 64x32x32 Euler cells, 13 us less of 263 us with Navier-Stokes, 15 us less
 // of 2.33 ms on a 1.07M-cell Navier-Stokes channel.
 // With p1 given (the point sweeps) the iterate goes there together with its
-// flux increments instead.
-template <bool EU>
+// flux increments instead.  ACC (the FP64 iteration): u is formed here from
+// the face fluxes G, V (accumulate_cell) and stored, in place of a launch and a
+// re-read: an iteration of 16x12x8 Euler cells 77.1 -> 74.6 us, of 64x32x32
+// cells 121.0 -> 117.7 (Euler) and 159.1 -> 155.7 (limited Navier-Stokes), of
+// 1.07M cells 2025 -> 2023.  The FP32 coefficient kernel does not: the sums'
+// loads lengthen it by more than the launch costs (4.4M cells 3.41 -> 3.44 ms
+// an iteration).
+template <bool EU, bool ACC>
 __global__ void __launch_bounds__(kTile) k_impl_coefs(
     const Blk* __restrict__ blks, Space sp, double dtpas, const double* __restrict__ v,
     const double* __restrict__ prim, long long ld, const double* __restrict__ sn,
@@ -700,7 +706,8 @@ __global__ void __launch_bounds__(kTile) k_impl_coefs(
     const double* __restrict__ rv, const double* __restrict__ dt,
     const double* __restrict__ u, double* __restrict__ coefe, double* __restrict__ coefdiag,
     double* __restrict__ d1, double2* __restrict__ p1, const double* __restrict__ ps, Phys ph,
-    int qfix) {
+    int qfix, const double* __restrict__ G, const double* __restrict__ V,
+    double* __restrict__ u_out) {
   int b, i, j, k;
   if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
@@ -731,10 +738,15 @@ __global__ void __launch_bounds__(kTile) k_impl_coefs(
   }
   if (!EU && dtpas > 0.) c = c + 1.5 * vn / dtpas;
   coefdiag[n] = c;
-  if (!d1 && !p1) return;
   double d[5];
+  if (ACC) {
+    accumulate_cell(B, i, j, k, n, G, V, ld, d);
 #pragma unroll
-  for (int a = 0; a < 5; ++a) d[a] = (-u[a * ld + n] + 0.) / c;
+    for (int a = 0; a < 5; ++a) u_out[a * ld + n] = d[a];
+  }
+  if (!d1 && !p1) return;
+#pragma unroll
+  for (int a = 0; a < 5; ++a) d[a] = (-(ACC ? d[a] : u[a * ld + n]) + 0.) / c;
   if (d1) {
 #pragma unroll
     for (int a = 0; a < 5; ++a) d1[a * ld + n] = d[a];
@@ -1162,22 +1174,21 @@ cudaError_t launch_implicit_coefficients(const Blk* blks, Space cells, Phys ph, 
                                          double dtpas, const double* dt, const double* v,
                                          const double* prim, const double* mu,
                                          const double* mut, const double* sn,
-                                         const double* vol, const double* cson,
-                                         const double* u, int rv_done, double* d1,
-                                         double2* p1, const double* ps, int qfix, Work& w,
+                                         const double* vol, const double* cson, double* u,
+                                         int sum_faces, int rv_done, double* d1, double2* p1,
+                                         const double* ps, int qfix, Work& w,
                                          cudaStream_t st) {
   if (cells.ntiles == 0) return cudaSuccess;
   const int g = grid_of(cells);
-  if (eu) {
-    pdl(k_impl_coefs<true>, g, kTile, 0, st)(blks, cells, dtpas, v, prim, w.ld, sn, vol, cson,
-                                            nullptr, dt, u, w.coefe, w.coefdiag, d1, p1, ps, ph,
-                                            qfix);
-  } else {
-    if (!rv_done) pdl(k_impl_rv, g, kTile, 0, st)(blks, cells, ph, v, mu, mut, w.rv);
-    pdl(k_impl_coefs<false>, g, kTile, 0, st)(blks, cells, dtpas, v, prim, w.ld, sn, vol, cson,
-                                             w.rv, dt, u, w.coefe, w.coefdiag, d1, p1, ps, ph,
-                                             qfix);
-  }
+  if (!eu && !rv_done) pdl(k_impl_rv, g, kTile, 0, st)(blks, cells, ph, v, mu, mut, w.rv);
+  auto run = [&](auto kernel) {
+    pdl(kernel, g, kTile, 0, st)(blks, cells, dtpas, v, prim, w.ld, sn, vol, cson, w.rv, dt, u,
+                                 w.coefe, w.coefdiag, d1, p1, ps, ph, qfix, w.G, w.V, u);
+  };
+  if (sum_faces)
+    eu ? run(k_impl_coefs<true, true>) : run(k_impl_coefs<false, true>);
+  else
+    eu ? run(k_impl_coefs<true, false>) : run(k_impl_coefs<false, false>);
   return cudaGetLastError();
 }
 
@@ -1205,7 +1216,7 @@ static cudaError_t point_sweeps64(const Blk* blks, Space cells, Phys ph, int qfi
 }
 
 cudaError_t launch_implicit(const Blk* blks, Space cells, Tiles tl, Phys ph, Scheme sc, int eu,
-                            int lmx, const double* u, const double* dt, double* v,
+                            int lmx, double* u, int sum_faces, const double* dt, double* v,
                             double* d_out, const double* mu, const double* mut,
                             const double* sn, const double* vol, const double* ps,
                             const double* cson, int rv_done, Work& w, int want_norms,
@@ -1217,8 +1228,8 @@ cudaError_t launch_implicit(const Blk* blks, Space cells, Tiles tl, Phys ph, Sch
   // dtpas > 0: dual time stepping with physical step dtpas
   cudaError_t e = launch_implicit_coefficients(
       blks, cells, ph, eu, sc.kfmg == 3 ? sc.dt1min : 0., dt, v, w.prim, mu, mut, sn, vol, cson,
-      u, rv_done, lmx >= 1 && !point ? w.dpp[0] : nullptr, point ? w.pt[0] : nullptr, ps, qfix, w,
-      st);
+      u, sum_faces, rv_done, lmx >= 1 && !point ? w.dpp[0] : nullptr,
+      point ? w.pt[0] : nullptr, ps, qfix, w, st);
   int cur = 0;
   if (e == cudaSuccess && point)
     e = point_sweeps64(blks, cells, ph, qfix, eu, lmx, u, v, ps, sn, w, st);

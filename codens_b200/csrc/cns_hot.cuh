@@ -961,23 +961,15 @@ static inline cudaError_t face_flux_dispatch(const Blk* blks, const SpaceBuf* fa
 }
 
 // u(n) from the six faces of the cell, summed in FP64 in the reference's
-// order; with corr (defect correction, FP64) u = that sum + corr; with u32 a
-// single-precision copy of u is written too
-// V (HLLC with the stresses): the halves 0.5*fv of the interior faces'
+// order.  V (HLLC with the stresses): the halves 0.5*fv of the interior faces'
 // viscous flux, applied after each face's fc as sch_hllc.f90:376-385 does
 template <class T>
-__global__ void __launch_bounds__(kTile) k_accumulate(const Blk* __restrict__ blks,
-                                                      Space sp, const T* __restrict__ G,
-                                                      long long ld,
-                                                      const double* __restrict__ corr,
-                                                      double* __restrict__ u,
-                                                      float* __restrict__ u32,
-                                                      const T* __restrict__ V = nullptr) {
-  int b, i, j, k;
-  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
-  const Blk& B = blks[b];
-  const long long n = cell_index(B, i, j, k);
-  double acc[5] = {0., 0., 0., 0., 0.};
+__device__ __forceinline__ void accumulate_cell(const Blk& B, int i, int j, int k, long long n,
+                                                const T* __restrict__ G,
+                                                const T* __restrict__ V, long long ld,
+                                                double acc[5]) {
+#pragma unroll
+  for (int a = 0; a < 5; ++a) acc[a] = 0.;
 #pragma unroll
   for (int dir = 0; dir < 3; ++dir) {
     const long long inc = ninc_of(B, dir);
@@ -1002,6 +994,25 @@ __global__ void __launch_bounds__(kTile) k_accumulate(const Blk* __restrict__ bl
       }
     }
   }
+}
+
+// the residual of each cell; with corr (defect correction, FP64) u = the sum +
+// corr; with u32 a single-precision copy of u is written too.  (The FP64
+// iteration's coefficient kernel sums the cell's faces itself.)
+template <class T>
+__global__ void __launch_bounds__(kTile) k_accumulate(const Blk* __restrict__ blks,
+                                                      Space sp, const T* __restrict__ G,
+                                                      long long ld,
+                                                      const double* __restrict__ corr,
+                                                      double* __restrict__ u,
+                                                      float* __restrict__ u32,
+                                                      const T* __restrict__ V = nullptr) {
+  int b, i, j, k;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
+  const Blk& B = blks[b];
+  const long long n = cell_index(B, i, j, k);
+  double acc[5];
+  accumulate_cell(B, i, j, k, n, G, V, ld, acc);
 #pragma unroll
   for (int a = 0; a < 5; ++a) {
     const double r = corr ? acc[a] + corr[a * ld + n] : acc[a];
