@@ -839,79 +839,76 @@ __global__ void __launch_bounds__(kTile) k_norm_partials(
 // Sums of the tile partials in a fixed order, and the rscpsv.f90:79-150
 // combination over blocks, in one launch.  CTA (x, y) sums the tiles
 // x * kNormChunk .. of block y: 32 rows of 15 lanes walk the partials
-// [tile][15] (consecutive threads read consecutive values), then a tree over
-// the rows; the last CTA to finish combines the blocks the same way and
-// resets the counter.  Latency bound (a megabyte of partials on a million
-// cells): 13 -> 8.5 us on 64x32x32 cells, 30 -> 10 us on 1.07M cells in three
-// blocks, against one CTA a block and a combining kernel (cold).
+// [tile][15] (consecutive threads read consecutive values), then, turned round
+// in shared memory, a tree over the rows of column q in warp q; the last CTA to
+// finish combines the blocks the same way and resets the counter.  Latency
+// bound (a megabyte of partials on a million cells): 13 -> 8.5 us on 64x32x32
+// cells, 30 -> 10 us on 1.07M cells in three blocks, against one CTA a block
+// and a combining kernel (cold).  The trees are shuffles: with one barrier in
+// place of eighteen and the partials' own tree (norm_tile_reduce) an iteration
+// of 16x12x8 cells takes 74.6 -> 71.5 us.
 constexpr int kNormRows = 32;
 
-__device__ __forceinline__ double norm_add(int q, double a, double b) {
-  return q >= 10 ? fmax(a, b) : a + b;
-}
-
-// tree over the rows of red; the result of column q is in red[0][q]
-__device__ __forceinline__ void norm_tree(double (*red)[15], int row, int q, double x) {
-  red[row][q] = x;
-  __syncthreads();
+// tree over the lanes (rows) of column q; the result is lane 0's
+__device__ __forceinline__ double norm_tree(int q, double x) {
 #pragma unroll
-  for (int s = kNormRows / 2; s > 0; s >>= 1) {
-    if (row < s) red[row][q] = norm_add(q, red[row][q], red[row + s][q]);
-    __syncthreads();
-  }
+  for (int s = kNormRows / 2; s > 0; s >>= 1)
+    x = norm_add(q, x, __shfl_down_sync(0xffffffffu, x, s));
+  return x;
 }
 
 __global__ void __launch_bounds__(kNormRows * 15) k_norms(
     const Blk* __restrict__ blks, const int* __restrict__ blk_tile0,
     const double* __restrict__ normpart, double* __restrict__ chunksum, int* counter,
     double* norms) {
-  pdl_sync();
-  __shared__ double red[kNormRows][15];
+  __shared__ double red[kNormRows * 15];
   __shared__ int last;
-  const int q = threadIdx.x % 15, row = threadIdx.x / 15;
   const int t1 = blk_tile0[blockIdx.y + 1];
   const int c0 = blk_tile0[blockIdx.y] + (int)blockIdx.x * kNormChunk;
   const int c1 = min(c0 + kNormChunk, t1);
+  pdl_sync();
   double x = 0.;
 #pragma unroll 8
-  for (int t = c0 + row; t < c1; t += kNormRows)
-    x = norm_add(q, x, normpart[(long long)t * 15 + q]);
-  norm_tree(red, row, q, x);
-  const long long chunk = (long long)blockIdx.y * gridDim.x + blockIdx.x;
-  if (row == 0) {
-    chunksum[chunk * 15 + q] = red[0][q];
+  for (int t = c0 + (int)threadIdx.x / 15; t < c1; t += kNormRows)
+    x = norm_add(threadIdx.x % 15, x, normpart[(long long)t * 15 + threadIdx.x % 15]);
+  red[threadIdx.x] = x;
+  __syncthreads();
+  const int q = threadIdx.x / 32, row = threadIdx.x % 32;
+  x = norm_tree(q, red[row * 15 + q]);
+  const int ctas = gridDim.x * gridDim.y;
+  if (ctas > 1) {
+    const long long chunk = (long long)blockIdx.y * gridDim.x + blockIdx.x;
+    if (row == 0) {
+      chunksum[chunk * 15 + q] = x;
+      __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(counter, 1) == ctas - 1;
+    __syncthreads();
+    if (!last) return;
     __threadfence();
+    if (threadIdx.x == 0) *counter = 0;
   }
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(counter, 1) == (int)(gridDim.x * gridDim.y) - 1;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
   // blocks row, row + 32, ... (rscpsv.f90: nmax * norm1, nmax * norm2^2, max)
-  double g = 0.;
-  long long npts = 0;
+  double g = 0., npts = 0.;
   for (int b = row; b < (int)gridDim.y; b += kNormRows) {
     const Blk& B = blks[b];
-    const long long nmax = (long long)(B.ni - 1) * (B.nj - 1) * (B.nk - 1);
-    const double coef = 1. / (double)nmax;
+    const double nmax = (double)((long long)(B.ni - 1) * (B.nj - 1) * (B.nk - 1));
+    const double coef = 1. / nmax;
     double s = 0.;
-    for (int c = 0; c < (int)gridDim.x; ++c)
-      s = norm_add(q, s, __ldcg(chunksum + ((long long)b * gridDim.x + c) * 15 + q));
+    if (ctas == 1) s = x;
+    else
+      for (int c = 0; c < (int)gridDim.x; ++c)
+        s = norm_add(q, s, __ldcg(chunksum + ((long long)b * gridDim.x + c) * 15 + q));
     if (q < 5)
-      s = (double)nmax * (coef * s);
+      s = nmax * (coef * s);
     else if (q < 10)
-      s = (double)nmax * sq(sqrt(coef * s));
+      s = nmax * sq(sqrt(coef * s));
     g = norm_add(q, g, s);
     npts += nmax;
   }
-  __syncthreads();
-  norm_tree(red, row, q, g);
-  const double tot = red[0][q];
-  __syncthreads();
-  norm_tree(red, row, q, q == 0 ? (double)npts : 0.);
-  if (row == 0)
-    norms[q] = q < 5 ? tot / red[0][0] : (q < 10 ? sqrt(tot / red[0][0]) : tot);
-  if (threadIdx.x == 0) *counter = 0;
+  const double tot = norm_tree(q, g), n = norm_tree(0, npts);
+  if (row == 0) norms[q] = q < 5 ? tot / n : (q < 10 ? sqrt(tot / n) : tot);
 }
 
 }  // namespace

