@@ -286,8 +286,8 @@ cudaError_t launch_accumulate_t<float>(const Blk* blks, Space sp, const float* G
 
 // ---------------------------------------------------------------------------
 // FP32 2.5D point-Jacobi sweep of the mixed forms (every sweep after the
-// first).  The tiling, the cp.async staging of plane k+2 and the one-cell
-// ring are those of k_jacobi_25d; two things differ from its FP64 form:
+// first).  The tiling, the staging of plane k+2 and the one-cell ring are
+// those of k_jacobi_25d; two things differ from its FP64 form:
 //
 // * shared layout: the increment (d, f) of a staged cell is packed as four
 //   float4 quads [d0 d1 d2 d3] [d4 f0 f1 f2] [f3 f4 f5 f6] [f7 f8 - -] in
@@ -301,6 +301,13 @@ cudaError_t launch_accumulate_t<float>(const Blk* blks, Space sp, const float* G
 //   over the directions: 20 fused multiply-adds per neighbour instead of the
 //   two face evaluations.  The same sum in exact arithmetic (FP32 rounding
 //   differs; the sweep only shapes the increment).
+// A thread fills its own cell and at most one of the ring, so its own column
+// (planes k-1, k, k+1) stays in registers, it reads the four in-plane
+// neighbours only, and a plane needs one barrier (the boxes' arrival) instead
+// of two: bound by shared-memory reads and barriers more than by DRAM, an
+// iteration of 4.4M cells takes 3.47 -> 3.31 ms, of 1.5M Euler cells in 24
+// boxes 1.50 -> 1.40 ms.  (128 registers, four CTAs of 128 threads a SM;
+// capped at 96 for five it is no faster.)
 // ---------------------------------------------------------------------------
 namespace {
 
@@ -483,20 +490,20 @@ __device__ __forceinline__ bool sweep_f32_tile(const int4 t, const Blk* __restri
   const float gam1 = (float)ph64.gam1, pinfl = (float)ph64.pinfl;
   const int x0 = t.y - 1, y0 = t.z - 1;
 
-  // the patch-and-ring points this thread fills (at most two for every
-  // shape: NP <= 2 NT): whether the column is inside the block's real cells
-  // and its offset in a component's box
-  constexpr int NQ = (NP + NT - 1) / NT;
-  static_assert(NQ <= 2, "a thread fills at most two ring points");
-  bool colin[NQ];
-  int boxo[NQ];
+  // the points this thread fills: its own cell (r = 0) and one of the ring
+  // (r = 1; the corners are not used): whether the column is inside the
+  // block's real cells, its quad point and its offset in a component's box
+  constexpr int NR = 2 * (TI + TJ);
+  static_assert(NR <= NT, "a thread fills at most one ring point");
+  const int e = threadIdx.x, es = e - 2 * TI;
+  const int rx = es < 0 ? e % TI + 1 : (es & 1) * (TI + 1);
+  const int ry = es < 0 ? (e < TI ? 0 : TJ + 1) : es / 2 + 1;
+  const int qx[2] = {tx + 1, rx}, qy[2] = {ty + 1, ry};
+  bool colin[2];
 #pragma unroll
-  for (int r = 0; r < NQ; ++r) {
-    const int q = threadIdx.x + r * NT;
-    const int qx = q % NX, qy = q / NX;
-    const int ii = x0 + qx, jj = y0 + qy;
-    colin[r] = q < NP && ii >= 1 && ii <= B.ni - 1 && jj >= 1 && jj <= B.nj - 1;
-    boxo[r] = qy * NXP + qx;
+  for (int r = 0; r < 2; ++r) {
+    const int ii = x0 + qx[r], jj = y0 + qy[r];
+    colin[r] = (r == 0 || e < NR) && ii >= 1 && ii <= B.ni - 1 && jj >= 1 && jj <= B.nj - 1;
   }
   if (BOX && threadIdx.x == 0) {
     map_acquire(map_d + t.x);
@@ -523,12 +530,11 @@ __device__ __forceinline__ bool sweep_f32_tile(const int4 t, const Blk* __restri
       float* rs = raw_s(b);
       const bool kin = kk >= 1 && kk <= B.nk - 1;
 #pragma unroll
-      for (int rr = 0; rr < NQ; ++rr) {
-        const int q = threadIdx.x + rr * NT;
-        if (q >= NP) break;
-        const bool in = colin[rr] && kin;
-        const long long m = in ? pad_index(B, x0 + q % NX, y0 + q / NX, kk) : B.ppc;
-        const int o = boxo[rr];
+      for (int r = 0; r < 2; ++r) {
+        if (r == 1 && e >= NR) break;
+        const bool in = colin[r] && kin;
+        const long long m = in ? pad_index(B, x0 + qx[r], y0 + qy[r], kk) : B.ppc;
+        const int o = qy[r] * NXP + qx[r];
 #pragma unroll
         for (int c = 0; c < 5; ++c) cp_async_elem(rd + c * PL + o, d_in + c * pld + m, in);
 #pragma unroll
@@ -552,30 +558,28 @@ __device__ __forceinline__ bool sweep_f32_tile(const int4 t, const Blk* __restri
     }
     return !__syncthreads_or(!ok);
   };
-  // increments of the staged plane in raw plane b into quad plane b; cells
-  // outside the block's real cells are zero
-  auto fill = [&](int kk, int b) {
+  // increments of the staged plane in raw plane b into quad plane b, the own
+  // cell's into x too; cells outside the block's real cells are zero
+  auto fill = [&](int kk, int b, Inc& x) {
     const float* rd = raw_d(b);
     const float* rs = raw_s(b);
     float4* s = sm.sq + b * 4 * NP;
     const bool kin = kk >= 1 && kk <= B.nk - 1;
 #pragma unroll
-    for (int rr = 0; rr < NQ; ++rr) {
-      const int q = threadIdx.x + rr * NT;
-      if (q >= NP) break;
-      const bool in = colin[rr] && kin;
-      const int o = boxo[rr];
-      float dd[5], f[9];
+    for (int r = 1; r >= 0; --r) {
+      if (r == 1 && e >= NR) continue;
+      const bool in = colin[r] && kin;
+      const int o = qy[r] * NXP + qx[r];
 #pragma unroll
-      for (int c = 0; c < 5; ++c) dd[c] = in ? rd[c * PL + o] : 0.f;
+      for (int c = 0; c < 5; ++c) x.d[c] = in ? rd[c * PL + o] : 0.f;
       if (in) {
-        df_diff<float, EU>(dd, rs[o], rs[PL + o], rs[2 * PL + o], rs[3 * PL + o],
-                           rs[4 * PL + o], rs[5 * PL + o], gam1, pinfl, qfix, f);
+        df_diff<float, EU>(x.d, rs[o], rs[PL + o], rs[2 * PL + o], rs[3 * PL + o],
+                           rs[4 * PL + o], rs[5 * PL + o], gam1, pinfl, qfix, x.f);
       } else {
 #pragma unroll
-        for (int c = 0; c < 9; ++c) f[c] = 0.f;
+        for (int c = 0; c < 9; ++c) x.f[c] = 0.f;
       }
-      quad_store(s, NP, q, dd, f);
+      quad_store(s, NP, qy[r] * NX + qx[r], x.d, x.f);
     }
   };
   // a failed wait: the boxes still in flight are waited for (bounded) before
@@ -591,7 +595,7 @@ __device__ __forceinline__ bool sweep_f32_tile(const int4 t, const Blk* __restri
   };
 
   // the own column's plane kbeg-1 (registers), read from global memory
-  Inc pk;
+  Inc pk, c0, up;
   if (own && kbeg >= 2) {
     const long long pm = pad_index(B, i, j, kbeg - 1);
 #pragma unroll
@@ -610,8 +614,7 @@ __device__ __forceinline__ bool sweep_f32_tile(const int4 t, const Blk* __restri
     drain(1u << ((kbeg + 1) & 1));
     return false;
   }
-  fill(kbeg, kbeg & 1);
-  __syncthreads();
+  fill(kbeg, kbeg & 1, c0);
   const int q0 = (ty + 1) * NX + tx + 1;
   // the lower k face of the own cell, carried from plane to plane (the
   // upper k face of plane k is the lower one of plane k+1)
@@ -639,20 +642,18 @@ __device__ __forceinline__ bool sweep_f32_tile(const int4 t, const Blk* __restri
       cd = a.coefdiag[n];
     }
     fkc = fku;
-    // plane k+1 has landed; plane k's raw plane is free
+    // plane k+1 has landed; plane k's increments are in its quad plane, and
+    // its raw plane and the other quad plane are free
     if (!arrived((k + 1) & 1, true)) {
       drain(0u);
       return false;
     }
     // plane k+2's inputs go into the raw plane that plane k used
     stage(k + 2, k & 1);
-    fill(k + 1, (k + 1) & 1);
-    __syncthreads();
+    fill(k + 1, (k + 1) & 1, up);
     const float4* s = sm.sq + (k & 1) * 4 * NP;
-    const float4* su = sm.sq + ((k + 1) & 1) * 4 * NP;
-    Inc c0, x;
-    quad_load(s, NP, q0, c0);
     if (own) {
+      Inc x;
       float acc[5];
 #pragma unroll
       for (int c = 0; c < 5; ++c) acc[c] = -uu[c];
@@ -669,14 +670,14 @@ __device__ __forceinline__ bool sweep_f32_tile(const int4 t, const Blk* __restri
       quad_load(s, NP, q0 + NX, x);
       phi_acc(x, -fju.x, -fju.y, -fju.z, fju.w, acc);
       phi_acc(pk, fk.x, fk.y, fk.z, fk.w, acc);
-      quad_load(su, NP, q0, x);
-      phi_acc(x, -fku.x, -fku.y, -fku.z, fku.w, acc);
+      phi_acc(up, -fku.x, -fku.y, -fku.z, fku.w, acc);
       const float rc = 1.f / cd;
       const long long pn = pad_index(B, i, j, k);
 #pragma unroll
       for (int c = 0; c < 5; ++c) d_out[c * pld + pn] = acc[c] * rc;
     }
     pk = c0;
+    c0 = up;
   }
   // plane kend+1 (staged by the last plane) is still in flight
   if (!arrived((kend + 1) & 1, true)) return false;
