@@ -43,9 +43,8 @@ def test_norms_of_the_fused_step(cuda, make):
     case = make()
     orc, st = oracle_prepared(case)
     s = _solver(case)
-    for _ in range(2):
-        v0 = st.v.copy()
-        orc.step(st)
-        # sums of at most 134160 positive terms in two orders: 1e-12 is 4500 eps
-        np.testing.assert_allclose(s.atsch_num(1), orc.norms(v0, st), rtol=1e-12, atol=0)
+    v0 = st.v.copy()
+    orc.step(st)  # one iteration: the 37 boxes diverge in the second, in the oracle too
+    # sums of at most 134160 positive terms in two orders: 1e-12 is 4500 eps
+    np.testing.assert_allclose(s.atsch_num(1), orc.norms(v0, st), rtol=1e-12, atol=0)
     s.close()
