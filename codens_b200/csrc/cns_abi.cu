@@ -27,7 +27,7 @@ struct cns_ctx {
   double alfak = 1.0, alfae = 1.3, sigma = 2.0 / 3.0, epsroe = 0.0;  // modeleturb, schemanum
   double* sa_gr = nullptr;   // gradients of rho nu~ and rho [6][ld]
   double* sa_sc = nullptr;   // gradient scalars (velocity, s6/s1, s7/s1) [3][ld]
-  double* sa_w = nullptr;    // impli2_eqt_3d scratch [20][ld]
+  double* sa_w = nullptr;    // impli2_eqt_3d scratch [17][ld]
   // Spalart-Allmaras transport step of the fused iteration (cns_set_sa)
   bool sa_on = false;
   double sa_rokinf = 0., sa_roeinf = 0., sa_epsk = 1e-8;
@@ -611,7 +611,7 @@ cudaError_t ensure_sa_step(cns_ctx* c) {
   cudaError_t e = cudaSuccess;
   if (!c->sa_gr) e = dev_alloc(c, &c->sa_gr, 6 * ld, false);
   if (e == cudaSuccess && !c->sa_sc) e = dev_alloc(c, &c->sa_sc, 3 * ld, false);
-  if (e == cudaSuccess && !c->sa_w) e = dev_alloc(c, &c->sa_w, 20 * ld);
+  if (e == cudaSuccess && !c->sa_w) e = dev_alloc(c, &c->sa_w, 17 * ld);
   if (e == cudaSuccess && !c->sa_dv) e = dev_alloc(c, &c->sa_dv, 9 * ld);
   if (e == cudaSuccess && !c->sa_fd) e = dev_alloc(c, &c->sa_fd, 6 * ld);
   if (e == cudaSuccess && !c->sa_ts) e = dev_alloc(c, &c->sa_ts, 2 * ld);
@@ -2038,7 +2038,7 @@ int cns_impli2_eqt_3d(cns_ctx* c, int l, const double* u, const double* dt, doub
   if (!c || bad_block(c, l) || !u || !dt || !v || !mu || !mut || !cfke || !sn || !vol ||
       !(cmt != 0.))
     return CNS_EINVAL;
-  if (!c->sa_w) CK(dev_alloc(c, &c->sa_w, (size_t)20 * c->lay.ld));
+  if (!c->sa_w) CK(dev_alloc(c, &c->sa_w, (size_t)17 * c->lay.ld));
   CK(prim_of(c, l, v));
   CK(launch_impli2(c->d_blks, c->lines, c->cells.view(l - 1), l - 1, c->lay.ld, u, dt, v,
                    c->w.prim, mu, mut, cfke, sn, vol, cmt, c->sa_w, 0, c->d_lp2_ni, c->n_lp2_ni,

@@ -395,7 +395,7 @@ cudaError_t launch_smsa(const Blk* blks, Space cells, long long ld, const double
                         const double* mu, const double* dist, const double* dv,
                         const double* grt, const double* grr, const double* const fd5[3],
                         double* ts6, double* ts7, double* cfke, int fix, cudaStream_t st);
-// impli2_eqt_3d of block l0 (-1: all): u, v are (ld, 7); w: 20 ld scratch;
+// impli2_eqt_3d of block l0 (-1: all): u, v are (ld, 7); w: 17 ld scratch;
 // rcp = 1: one reciprocal per line step instead of three divisions (the
 // reduced-precision forms; not bit-exact)
 // wall_ni: the first cells of the wall-law walls (nwall of them), whose

@@ -276,29 +276,29 @@ __global__ void __launch_bounds__(kTile) k_i2_coefs(const Blk* __restrict__ blks
 
 // one alternating-line sweep of direction dir (impli2_eqt_3d.f90:172-291),
 // in two kernels.  k_i2_rhs (a thread per real cell, fully parallel): the
-// tridiagonal coefficients ai, bi, cci of the cell and the right-hand sides
-// di6, di7, whose neighbours in the two other directions come from the
-// previous iterate.  k_i2_line (a thread per line): the backward recurrence
-// into al/b6/b7 (written over ai/bi/cci) and the forward substitution into
-// the new iterate -- the only sequential part, reading five values per cell.
+// right-hand sides di6, di7, whose neighbours in the two other directions come
+// from the previous iterate.  k_i2_line (a thread per line): the tridiagonal
+// coefficients ai, bi, cci, the backward recurrence into al/b6/b7 and the
+// forward substitution into the new iterate -- the only sequential part, reading
+// five values per cell: the coefficients take the face values u, e of the
+// direction (those of the upper face carried) and the diagonal, as many loads as
+// the coefficients themselves would, so k_i2_rhs (bound by DRAM) neither reads
+// nor writes anything for them (an iteration of the
+// 2.1M-cell plate 3.31 -> 3.23 ms).
 // The expressions and their order are the reference's, so the split is
 // bit-identical to evaluating everything inside the line loop.
 __global__ void __launch_bounds__(kTile) k_i2_rhs(
     const Blk* __restrict__ blks, Space sp, int dir, long long ld,
     const double* __restrict__ u, const double* __restrict__ uf,
-    const double* __restrict__ ce, const double* __restrict__ cd,
-    const double* __restrict__ o6, const double* __restrict__ o7, double* __restrict__ ta,
-    double* __restrict__ tb, double* __restrict__ tc, double* __restrict__ d6,
-    double* __restrict__ d7) {
+    const double* __restrict__ ce, const double* __restrict__ o6,
+    const double* __restrict__ o7, double* __restrict__ d6, double* __restrict__ d7) {
   int b, i, j, k;
   if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const int oa = dir == 0 ? 1 : 0, ob = dir == 2 ? 1 : 2;
-  const long long inc = ninc_of(B, dir), inca = ninc_of(B, oa), incb = ninc_of(B, ob);
-  const double *ua = uf + (long long)oa * ld, *ub = uf + (long long)ob * ld,
-               *ud = uf + (long long)dir * ld;
-  const double *ca = ce + (long long)oa * ld, *cb = ce + (long long)ob * ld,
-               *cdir = ce + (long long)dir * ld;
+  const long long inca = ninc_of(B, oa), incb = ninc_of(B, ob);
+  const double *ua = uf + (long long)oa * ld, *ub = uf + (long long)ob * ld;
+  const double *ca = ce + (long long)oa * ld, *cb = ce + (long long)ob * ld;
   const long long m = cell_index(B, i, j, k);
   const double td = -ua[m + inca] + ua[m] - ub[m + incb] + ub[m];
   const double tpa = ca[m + inca] - ua[m + inca], tma = ca[m] + ua[m];
@@ -307,9 +307,6 @@ __global__ void __launch_bounds__(kTile) k_i2_rhs(
           tmb * o6[m - incb] + tpb * o6[m + incb];
   d7[m] = -u[6 * ld + m] + td * o7[m] + tma * o7[m - inca] + tpa * o7[m + inca] +
           tmb * o7[m - incb] + tpb * o7[m + incb];
-  ta[m] = cdir[m] + ud[m];
-  tb[m] = cd[m] + ud[m + inc] - ud[m];
-  tc[m] = -cdir[m + inc] + ud[m + inc];
 }
 
 // The recurrence reads the coefficients from arrays it does not write, so
@@ -330,9 +327,9 @@ constexpr int kLineCta = 32;
 // chain per step shrinks from three divisions to one.
 template <bool RCP>
 __global__ void __launch_bounds__(kLineCta, 1) k_i2_line(const Blk* __restrict__ blks, Space sp,
-                                                      int dir, const double* __restrict__ ta,
-                                                      const double* __restrict__ tb,
-                                                      const double* __restrict__ tc,
+                                                      int dir, const double* __restrict__ uf,
+                                                      const double* __restrict__ ce,
+                                                      const double* __restrict__ cd,
                                                       const double* __restrict__ d6,
                                                       const double* __restrict__ d7,
                                                       double* __restrict__ al,
@@ -355,15 +352,16 @@ __global__ void __launch_bounds__(kLineCta, 1) k_i2_line(const Blk* __restrict__
   // p + 1 carried, zero past the end (the reference's never-written ghost
   // entries)
   double aln = 0., b6n = 0., b7n = 0.;
+  double un = uf[m1 + (long long)nc * inc], en = ce[m1 + (long long)nc * inc];
   double xa[U], xb[U], xc[U], x6[U], x7[U];
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     const int p = nc - u;
     if (p >= 1) {
       const long long m = m1 + (long long)(p - 1) * inc;
-      xa[u] = ta[m];
-      xb[u] = tb[m];
-      xc[u] = tc[m];
+      xa[u] = uf[m];
+      xb[u] = cd[m];
+      xc[u] = ce[m];
       x6[u] = d6[m];
       x7[u] = d7[m];
     }
@@ -383,9 +381,9 @@ __global__ void __launch_bounds__(kLineCta, 1) k_i2_line(const Blk* __restrict__
       const int p = nc - (q0 + U + u);
       if (p >= 1) {
         const long long m = m1 + (long long)(p - 1) * inc;
-        xa[u] = ta[m];
-        xb[u] = tb[m];
-        xc[u] = tc[m];
+        xa[u] = uf[m];
+        xb[u] = cd[m];
+        xc[u] = ce[m];
         x6[u] = d6[m];
         x7[u] = d7[m];
       }
@@ -395,16 +393,19 @@ __global__ void __launch_bounds__(kLineCta, 1) k_i2_line(const Blk* __restrict__
       const int p = nc - (q0 + u);
       if (p >= 1) {
         const long long m = m1 + (long long)(p - 1) * inc;
-        const double den = yb[u] + yc[u] * aln;
+        const double ai = yc[u] + ya[u], bi = yb[u] + un - ya[u], ci = -en + un;
+        un = ya[u];
+        en = yc[u];
+        const double den = bi + ci * aln;
         if (RCP) {
           const double r = 1. / den;
-          aln = ya[u] * r;
-          b6n = (y6[u] - yc[u] * b6n) * r;
-          b7n = (y7[u] - yc[u] * b7n) * r;
+          aln = ai * r;
+          b6n = (y6[u] - ci * b6n) * r;
+          b7n = (y7[u] - ci * b7n) * r;
         } else {
-          aln = ya[u] / den;
-          b6n = (y6[u] - yc[u] * b6n) / den;
-          b7n = (y7[u] - yc[u] * b7n) / den;
+          aln = ai / den;
+          b6n = (y6[u] - ci * b6n) / den;
+          b7n = (y7[u] - ci * b7n) / den;
         }
         al[m] = aln;
         b6[m] = b6n;
@@ -824,15 +825,13 @@ cudaError_t launch_impli2(const Blk* blks, const SpaceBuf* lines, Space cells, i
                           double* w, int rcp, const long long* wall_ni, long long nwall,
                           cudaStream_t st) {
   // scratch w, zeroed when allocated: rv, cd, uf[3], ce[3], al, b6, b7, two
-  // iterates x (6, 7), the tridiagonal coefficients ta, tb, tc and right-hand
-  // sides d6, d7 of a sweep = 20 ld.  The ghost entries of rv and of the
+  // iterates x (6, 7) and the right-hand sides d6, d7 of a sweep = 17 ld.  The ghost entries of rv and of the
   // iterates are never written (the reference's zeroed rv and never-written
   // neighbours); every other entry read is written first.
   double *rv = w, *cd = w + ld, *uf = w + 2 * ld, *ce = w + 5 * ld, *al = w + 8 * ld,
          *b6 = w + 9 * ld, *b7 = w + 10 * ld;
   double* it[2][2] = {{w + 11 * ld, w + 12 * ld}, {w + 13 * ld, w + 14 * ld}};
-  double *ta = w + 15 * ld, *tb = w + 16 * ld, *tc = w + 17 * ld, *d6 = w + 18 * ld,
-         *d7 = w + 19 * ld;
+  double *d6 = w + 15 * ld, *d7 = w + 16 * ld;
   if (cells.ntiles == 0) return cudaSuccess;
   pdl(k_i2_cell, grid_of(cells), kTile, 0, st)(blks, cells, v, mu, mut, dt, cfke, vol, cmt, rv,
                                                cd, it[0][0], it[0][1]);
@@ -841,18 +840,17 @@ cudaError_t launch_impli2(const Blk* blks, const SpaceBuf* lines, Space cells, i
   for (int dir = 0; dir < 3; ++dir) {
     const Space sp = lines[dir].view(l0);
     for (int sw = 0; sw < 2; ++sw) {
-      pdl(k_i2_rhs, grid_of(cells), kTile, 0, st)(blks, cells, dir, ld, u, uf, ce, cd,
-                                                 it[cur][0], it[cur][1], ta, tb, tc, d6, d7);
+      pdl(k_i2_rhs, grid_of(cells), kTile, 0, st)(blks, cells, dir, ld, u, uf, ce, it[cur][0],
+                                                  it[cur][1], d6, d7);
       // launched only when the chip is empty: placed while the kernel before
       // drains, the few one-warp CTAs crowd on the first free SMs (an iteration
       // of the 2.1M-cell plate 3.64 against 3.43 ms)
       const int lg = grid_of(sp) * (kTile / kLineCta);
-      if (sp.ntiles > 0 && rcp)
-        k_i2_line<true><<<lg, kLineCta, 0, st>>>(blks, sp, dir, ta, tb, tc, d6, d7, al, b6, b7,
-                                                 it[1 - cur][0], it[1 - cur][1]);
-      else if (sp.ntiles > 0)
-        k_i2_line<false><<<lg, kLineCta, 0, st>>>(blks, sp, dir, ta, tb, tc, d6, d7, al, b6,
-                                                  b7, it[1 - cur][0], it[1 - cur][1]);
+      auto line = [&](auto kernel) {
+        kernel<<<lg, kLineCta, 0, st>>>(blks, sp, dir, uf + dir * ld, ce + dir * ld, cd, d6, d7, al,
+                                        b6, b7, it[1 - cur][0], it[1 - cur][1]);
+      };
+      if (sp.ntiles > 0) rcp ? line(k_i2_line<true>) : line(k_i2_line<false>);
       cur = 1 - cur;
     }
   }
