@@ -712,6 +712,13 @@ __global__ void __launch_bounds__(kTile) k_impl_coefs(
   if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
   const Blk& B = blks[b];
   const long long n = cell_index(B, i, j, k);
+  double d[5];
+  if (ACC) {
+    if (V)
+      accumulate_cell<true>(B, i, j, k, n, G, V, ld, d);
+    else
+      accumulate_cell<false>(B, i, j, k, n, G, V, ld, d);
+  }
   double q0[6];
   radius_cell<EU>(v, prim, ld, vol, cson, rv, n, q0);
   const double vn = vol[n];
@@ -738,9 +745,7 @@ __global__ void __launch_bounds__(kTile) k_impl_coefs(
   }
   if (!EU && dtpas > 0.) c = c + 1.5 * vn / dtpas;
   coefdiag[n] = c;
-  double d[5];
   if (ACC) {
-    accumulate_cell(B, i, j, k, n, G, V, ld, d);
 #pragma unroll
     for (int a = 0; a < 5; ++a) u_out[a * ld + n] = d[a];
   }
