@@ -569,7 +569,7 @@ cudaError_t ensure_dis(cns_ctx* c) {
 
 bool jameson(const cns_ctx* c) { return c->sc.ischema <= 4; }
 
-// whether the FP64 iteration's coefficient kernel sums the face fluxes into
+// whether the FP64 or mixed iteration's coefficient kernel sums the face fluxes into
 // the residual: the families with a face buffer and nothing between the
 // residual and the implicit phase (dual time's term)
 bool sum_in_coefs(const cns_ctx* c) {
@@ -910,6 +910,7 @@ cudaError_t enqueue_step_mixed(cns_ctx* c, MixedMode mode, bool first, bool dt_o
   const long long ld = c->lay.ld;
   const Space all = c->cells.view(-1);
   const bool lim = c->sc.ns && c->sc.ilim == 1;
+  const bool sum = mode == kMixed && sum_in_coefs(c);
   // zpres (+ zvismo), and chronos when the time step is recomputed, in one pass
   cudaError_t e =
       dt_on ? launch_zpres_chronos(c->d_blks, all, c->ph, c->sc, s.v, ld, s.pression, s.ztemp,
@@ -988,7 +989,7 @@ cudaError_t enqueue_step_mixed(cns_ctx* c, MixedMode mode, bool first, bool dt_o
         if (e == cudaSuccess)
           e = launch_face_flux_fma(c->d_blks, c->faces, -1, c->ph, c->sc, s.v, w.prim, ld,
                                    s.pression, s.tau, s.sn, w.R, w.G, c->st, w.V);
-        if (e == cudaSuccess)
+        if (e == cudaSuccess && !sum)
           e = launch_accumulate_t<double>(c->d_blks, all, w.G, ld, nullptr, s.u, w.u32, c->st,
                                           w.V);
       }
@@ -1005,7 +1006,7 @@ cudaError_t enqueue_step_mixed(cns_ctx* c, MixedMode mode, bool first, bool dt_o
                               w.cv32, w.sn32, w.coefdiag32, w.snc32, w.u32,
                               c->sc.lmax >= 1 && !point ? w.d32pp[0] : nullptr,
                               point ? w.pt32[0] : nullptr, w.st32, c->ph,
-                              c->sc.ns ? 0 : c->sc.qfix_dfez, c->st);
+                              c->sc.ns ? 0 : c->sc.qfix_dfez, sum ? w.G : nullptr, w.V, s.u, c->st);
   int cur = 0;
   if (e == cudaSuccess && point)
     e = launch_point_sweeps32(c->d_blks, all, c->ph, c->sc, !c->sc.ns, c->sc.lmax, ld,

@@ -695,9 +695,9 @@ __device__ __forceinline__ void radius_cell(const double* __restrict__ v,
 // the face fluxes G, V (accumulate_cell) and stored, in place of a launch and a
 // re-read: an iteration of 16x12x8 Euler cells 77.1 -> 74.6 us, of 64x32x32
 // cells 121.0 -> 117.7 (Euler) and 159.1 -> 155.7 (limited Navier-Stokes), of
-// 1.07M cells 2025 -> 2023.  The FP32 coefficient kernel does not: the sums'
-// loads lengthen it by more than the launch costs (4.4M cells 3.41 -> 3.44 ms
-// an iteration).
+// 1.07M cells 2025 -> 2023.  With a
+// cell's loads issued together (accumulate_cell) the FP32 coefficient kernel
+// does the same.
 template <bool EU, bool ACC>
 __global__ void __launch_bounds__(kTile) k_impl_coefs(
     const Blk* __restrict__ blks, Space sp, double dtpas, const double* __restrict__ v,

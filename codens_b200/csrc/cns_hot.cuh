@@ -1010,8 +1010,8 @@ __device__ __forceinline__ void accumulate_cell(const Blk& B, int i, int j, int 
 }
 
 // the residual of each cell; with corr (defect correction, FP64) u = the sum +
-// corr; with u32 a single-precision copy of u is written too.  (The FP64
-// iteration's coefficient kernel sums the cell's faces itself.)
+// corr; with u32 a single-precision copy of u is written too.  (The FP64 and
+// mixed iterations' coefficient kernels sum the cell's faces themselves.)
 template <class T>
 __global__ void __launch_bounds__(kTile) k_accumulate(const Blk* __restrict__ blks,
                                                       Space sp, const T* __restrict__ G,

@@ -565,13 +565,15 @@ cudaError_t launch_defect(const Blk* blks, Space cells, long long ld, const doub
 // the FP32 implicit coefficients (snc32 per face, coefdiag32 per cell) of
 // the mixed sweeps in one pass over the real cells
 // (the per-cell inputs cq32, cv32 of PrimShadow); the first iterate in d1, or
-// with its increments in p1
+// with its increments in p1; with G the residual u, u32 is formed from the face
+// fluxes G, V first, else u32 is read
 cudaError_t launch_coefficients32(const Blk* blks, Space cells, int eu, long long ld,
                                   double dtpas, const double* dt, const double* vol,
                                   const float4* cq32, const float2* cv32, const float* sn32,
                                   float* coefdiag32, float4* snc32,
-                                  const float* u32, float* d1, float4* p1, const float* st32,
-                                  Phys ph, int qfix, cudaStream_t st);
+                                  float* u32, float* d1, float4* p1, const float* st32,
+                                  Phys ph, int qfix, const double* G, const double* V, double* u,
+                                  cudaStream_t st);
 // the face lanes of the FP32 sweep's pack: snc[dir * ld + n].xyz = S/2 of cell n's
 // lower face in dir (exact halves of sn32), .w = 0 until k_coef32 writes it
 cudaError_t launch_pack_faces32(const Blk* blks, int nblk, long long ncells, long long ld,
