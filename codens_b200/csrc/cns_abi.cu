@@ -690,14 +690,15 @@ cudaError_t enqueue_met_num_ke(cns_ctx* c) {
     long long b0, b1, n0, n1;
     block_range(c, b + 1, b0, b1);
     fludc_range(c, b + 1, n0, n1);
-    e = launch_teq_grads(c->d_blks, cb, 0, 3, s.v, nullptr, ld, s.sn, s.vol, c->sa_dv, c->sa_sc,
+    e = launch_teq_grads(c->d_blks, cb, 0, 3, s.v, nullptr, 0, ld, s.sn, s.vol, c->sa_dv, c->sa_sc,
                          b0, b1, c->st);
     if (e == cudaSuccess)
       e = launch_met_prod(c->d_blks, cb, ld, s.mut, s.v, c->sa_dv, c->ke_tprod, c->st);
-    for (int q = 0; q < 6 && e == cudaSuccess; ++q)
-      e = cudaMemsetAsync(fdw[q] + n0, 0, sizeof(double) * (size_t)(n1 - n0 + 1), c->st);
+    if (e == cudaSuccess)  // the six rows of fd in one node
+      e = cudaMemset2DAsync(fdw[0] + n0, sizeof(double) * ld, 0,
+                            sizeof(double) * (size_t)(n1 - n0 + 1), 6, c->st);
     if (e == cudaSuccess)
-      e = launch_teq_grads(c->d_blks, cb, 2, 2, s.v, nullptr, ld, s.sn, s.vol, fd, c->sa_sc, b0,
+      e = launch_teq_grads(c->d_blks, cb, 2, 2, s.v, nullptr, 0, ld, s.sn, s.vol, fd, c->sa_sc, b0,
                            b1, c->st);
     if (e == cudaSuccess) e = launch_exgr(c->lay.blks[b], ld, c->sa_dv, c->st);
     if (e == cudaSuccess)
@@ -711,16 +712,15 @@ cudaError_t enqueue_met_num_ke(cns_ctx* c) {
     e = launch_roe2o(c->d_blks, c->cells_ext.view(-1), sa_harten(c), c->epsroe, c->ph.gam,
                      c->ph.gam1, s.v, c->w.prim, ld, s.sn, s.d, c->st);
   if (e == cudaSuccess)
-    e = cudaMemsetAsync(s.u + 5 * ld, 0, sizeof(double) * c->lay.ncells, c->st);
-  if (e == cudaSuccess)
-    e = cudaMemsetAsync(s.u + 6 * ld, 0, sizeof(double) * c->lay.ncells, c->st);
+    e = cudaMemset2DAsync(s.u + 5 * ld, sizeof(double) * ld, 0, sizeof(double) * c->lay.ncells, 2,
+                          c->st);
   if (e == cudaSuccess)
     e = launch_sch_turb(c->d_blks, all, s.v, c->w.prim, ld, fdr, ts6, ts7, s.d, s.sn, s.vol, s.u,
                         c->st);
   if (e == cudaSuccess)
     e = launch_impli2(c->d_blks, c->lines, all, -1, ld, s.u, s.dt, s.v, c->w.prim, s.mu, s.mut,
                       c->sa_cfke, s.sn, s.vol, 1.0, c->sa_w, c->sc.precision != 0, nullptr, 0,
-                      c->st);
+                      nullptr, c->st);
   if (e == cudaSuccess) e = launch_cutke(c->d_blks, all, ld, s.v, c->ke_epsk, c->ke_epse, c->st);
   if (e == cudaSuccess) e = launch_kemut(c->d_blks, all, ld, s.v, s.mu, s.mut, c->st);
   return e;
@@ -742,7 +742,7 @@ cudaError_t enqueue_met_num(cns_ctx* c) {
     const Space cb = c->cells.view(b);
     long long b0, b1;
     block_range(c, b + 1, b0, b1);
-    e = launch_teq_grads(c->d_blks, cb, 0, 3, s.v, nullptr, ld, s.sn, s.vol, c->sa_dv, c->sa_sc,
+    e = launch_teq_grads(c->d_blks, cb, 0, 3, s.v, nullptr, 0, ld, s.sn, s.vol, c->sa_dv, c->sa_sc,
                          b0, b1, c->st);
     // met_num.f90:193-279: the wall law of the block's 'lp2' walls after
     // teq_gradv and met_prod, before met_gradtr reads rho nu~
@@ -752,17 +752,15 @@ cudaError_t enqueue_met_num(cns_ctx* c) {
     // reads there through its block-local index)
     long long n0, n1;
     fludc_range(c, b + 1, n0, n1);
-    for (int q = 0; q < 6 && e == cudaSuccess; ++q)
-      e = cudaMemsetAsync(fdw[q] + n0, 0, sizeof(double) * (size_t)(n1 - n0 + 1), c->st);
+    if (e == cudaSuccess)  // the six rows of fd in one node
+      e = cudaMemset2DAsync(fdw[0] + n0, sizeof(double) * ld, 0,
+                            sizeof(double) * (size_t)(n1 - n0 + 1), 6, c->st);
     if (e == cudaSuccess)
-      e = launch_teq_grads(c->d_blks, cb, 2, 2, s.v, nullptr, ld, s.sn, s.vol, fd, c->sa_sc, b0,
+      e = launch_teq_grads(c->d_blks, cb, 2, 2, s.v, nullptr, 0, ld, s.sn, s.vol, fd, c->sa_sc, b0,
                            b1, c->st);
-    if (e == cudaSuccess)
-      e = launch_teq_grads(c->d_blks, cb, 1, 1, s.v, s.v + 5 * ld, ld, s.sn, s.vol, c->sa_gr,
-                           nullptr, 0, 0, c->st);
-    if (e == cudaSuccess)
-      e = launch_teq_grads(c->d_blks, cb, 1, 1, s.v, s.v, ld, s.sn, s.vol, c->sa_gr + 3 * ld,
-                           nullptr, 0, 0, c->st);
+    if (e == cudaSuccess)  // of rho nu~, then of rho
+      e = launch_teq_grads(c->d_blks, cb, 1, 2, s.v, s.v + 5 * ld, -5 * ld, ld, s.sn, s.vol,
+                           c->sa_gr, nullptr, 0, 0, c->st);
     if (e == cudaSuccess)
       e = launch_smsa(c->d_blks, cb, ld, s.v, s.mu, c->sa_dist, c->sa_dv, c->sa_gr,
                       c->sa_gr + 3 * ld, fdr, ts6, ts7, c->sa_cfke, c->sa_fix, c->st);
@@ -775,18 +773,16 @@ cudaError_t enqueue_met_num(cns_ctx* c) {
                      c->ph.gam1, s.v, c->w.prim, ld, s.sn, s.d, c->st);
   // sch_turb.f90:59-66 zeroes u(:,6:7) over every block
   if (e == cudaSuccess)
-    e = cudaMemsetAsync(s.u + 5 * ld, 0, sizeof(double) * c->lay.ncells, c->st);
-  if (e == cudaSuccess)
-    e = cudaMemsetAsync(s.u + 6 * ld, 0, sizeof(double) * c->lay.ncells, c->st);
+    e = cudaMemset2DAsync(s.u + 5 * ld, sizeof(double) * ld, 0, sizeof(double) * c->lay.ncells, 2,
+                          c->st);
   if (e == cudaSuccess)
     e = launch_sch_turb(c->d_blks, all, s.v, c->w.prim, ld, fdr, ts6, ts7, s.d, s.sn, s.vol, s.u,
                         c->st);
+  const SaFinish fin{c->sa_epsk, s.mut};
   if (e == cudaSuccess)
     e = launch_impli2(c->d_blks, c->lines, all, -1, ld, s.u, s.dt, s.v, c->w.prim, s.mu, s.mut,
                       c->sa_cfke, s.sn, s.vol, 1.0, c->sa_w, c->sc.precision != 0,
-                      c->d_lp2_ni, c->n_lp2_ni, c->st);
-  if (e == cudaSuccess) e = launch_cutsa(c->d_blks, all, s.v, ld, c->sa_epsk, c->st);
-  if (e == cudaSuccess) e = launch_samut(c->d_blks, all, s.v + 5 * ld, s.mu, s.mut, c->st);
+                      c->d_lp2_ni, c->n_lp2_ni, &fin, c->st);
   return e;
 }
 
@@ -2007,7 +2003,7 @@ int cns_teq_gradv(cns_ctx* c, int l, const double* v, const double* sn, const do
   CK(ensure_sa(c));
   long long n0, n1;
   block_range(c, l, n0, n1);
-  CK(launch_teq_grads(c->d_blks, c->cells.view(l - 1), 0, 3, v, nullptr, c->lay.ld, sn, vol,
+  CK(launch_teq_grads(c->d_blks, c->cells.view(l - 1), 0, 3, v, nullptr, 0, c->lay.ld, sn, vol,
                       dv, c->sa_sc, n0, n1, c->st));
   return CNS_OK;
 }
@@ -2023,10 +2019,8 @@ int cns_met_smsa(cns_ctx* c, int l, const double* v, const double* mu, const dou
   const long long ld = c->lay.ld;
   const Space cells = c->cells.view(l - 1);
   // met_difsa: grad(rho nu~); met_smsa: grad(rho)
-  CK(launch_teq_grads(c->d_blks, cells, 1, 1, v, v + 5 * ld, ld, sn, vol, c->sa_gr, nullptr, 0,
-                      0, c->st));
-  CK(launch_teq_grads(c->d_blks, cells, 1, 1, v, v, ld, sn, vol, c->sa_gr + 3 * ld, nullptr, 0,
-                      0, c->st));
+  CK(launch_teq_grads(c->d_blks, cells, 1, 2, v, v + 5 * ld, -5 * ld, ld, sn, vol, c->sa_gr,
+                      nullptr, 0, 0, c->st));
   const double* fd5[3] = {fd5x, fd5y, fd5z};
   CK(launch_smsa(c->d_blks, cells, ld, v, mu, dist, dv, c->sa_gr, c->sa_gr + 3 * ld, fd5, ts6,
                  ts7, cfke, c->sa_fix, c->st));
@@ -2043,7 +2037,7 @@ int cns_impli2_eqt_3d(cns_ctx* c, int l, const double* u, const double* dt, doub
   CK(prim_of(c, l, v));
   CK(launch_impli2(c->d_blks, c->lines, c->cells.view(l - 1), l - 1, c->lay.ld, u, dt, v,
                    c->w.prim, mu, mut, cfke, sn, vol, cmt, c->sa_w, 0, c->d_lp2_ni, c->n_lp2_ni,
-                   c->st));
+                   nullptr, c->st));
   return CNS_OK;
 }
 
@@ -2096,7 +2090,7 @@ int cns_met_gradtr(cns_ctx* c, int l, const double* s, const double* sn, const d
       CK(cudaMemsetAsync(c->sa_fd + q * ld + n0, 0, sizeof(double) * cnt, c->st));
     long long b0, b1;
     block_range(c, b + 1, b0, b1);
-    CK(launch_teq_grads(c->d_blks, c->cells.view(b), 2, 2, s, nullptr, ld, sn, vol, c->sa_fd,
+    CK(launch_teq_grads(c->d_blks, c->cells.view(b), 2, 2, s, nullptr, 0, ld, sn, vol, c->sa_fd,
                         c->sa_sc, b0, b1, c->st));
     for (int q = 0; q < 6; ++q)
       CK(cudaMemcpyAsync(out[q] + n0, c->sa_fd + q * ld + n0, sizeof(double) * cnt,
@@ -2242,7 +2236,7 @@ int cns_met_ini(cns_ctx* c, int l, double* v, const double* mut, const double* m
   long long n0, n1;
   block_range(c, l, n0, n1);
   const Space cb = c->cells.view(l - 1);
-  CK(launch_teq_grads(c->d_blks, cb, 0, 3, v, nullptr, c->lay.ld, sn, vol, dv, c->sa_sc, n0, n1,
+  CK(launch_teq_grads(c->d_blks, cb, 0, 3, v, nullptr, 0, c->lay.ld, sn, vol, dv, c->sa_sc, n0, n1,
                       c->st));
   CK(launch_turb_init(c->d_blks, cb, 2, c->lay.ld, v, const_cast<double*>(mut), nullptr, dv,
                       c->st));

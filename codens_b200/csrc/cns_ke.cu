@@ -253,11 +253,11 @@ cudaError_t launch_smke(const Blk* blks, Space cells, long long ld, const double
   // w: gt [3][ld], g [9][ld], bare [ld], scalars [1][ld]
   double *gt = w, *g = w + 3 * ld, *bare = w + 12 * ld, *sc = w + 13 * ld;
   // met_bark: the gradient of sqrt(s6 / s1) over the block's cells
-  cudaError_t e = launch_teq_grads(blks, cells, 3, 1, s, nullptr, ld, sn, vol, gt, sc, n0, n1,
+  cudaError_t e = launch_teq_grads(blks, cells, 3, 1, s, nullptr, 0, ld, sn, vol, gt, sc, n0, n1,
                                    st);
   // met_bare: the gradients of the nine velocity gradients, three at a time
   for (int q = 0; q < 3 && e == cudaSuccess; ++q) {
-    e = launch_teq_grads(blks, cells, 1, 3, s, dv + 3 * q * ld, ld, sn, vol, g, nullptr, 0, 0,
+    e = launch_teq_grads(blks, cells, 1, 3, s, dv + 3 * q * ld, ld, ld, sn, vol, g, nullptr, 0, 0,
                          st);
     if (e == cudaSuccess)
       k_bare_acc<<<grid_of(cells), kTile, 0, st>>>(blks, cells, ld, g, bare, q == 0);

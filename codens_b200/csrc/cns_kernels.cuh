@@ -381,31 +381,37 @@ cudaError_t launch_sch_turb(const Blk* blks, Space cells, const double* v, const
                             const double* vol, double* u, cudaStream_t st);
 
 // teq_grads over the cells of the space into out[3 nsc][ld]: mode 0 = the
-// velocity (nsc 3), mode 1 = the fields f[q][ld], mode 2 = the transport
+// velocity (nsc 3), mode 1 = the fields f + q fs, mode 2 = the transport
 // variables per unit mass s6/s1, s7/s1 (nsc 2, met_gradtr), mode 3 =
 // sqrt(s6/s1) (nsc 1, met_bark); modes 0, 2 and 3
 // evaluate their scalars once into sc[nsc][ld] over the flat range [n0, n1)
 // covering the cells of the space and their ghosts.  met_smsa with its
 // gradients of rho nu~ (grt) and rho (grr)
 cudaError_t launch_teq_grads(const Blk* blks, Space cells, int mode, int nsc,
-                             const double* v, const double* f, long long ld, const double* sn,
-                             const double* vol, double* out, double* sc, long long n0,
-                             long long n1, cudaStream_t st);
+                             const double* v, const double* f, long long fs, long long ld,
+                             const double* sn, const double* vol, double* out, double* sc,
+                             long long n0, long long n1, cudaStream_t st);
 cudaError_t launch_smsa(const Blk* blks, Space cells, long long ld, const double* v,
                         const double* mu, const double* dist, const double* dv,
                         const double* grt, const double* grr, const double* const fd5[3],
                         double* ts6, double* ts7, double* cfke, int fix, cudaStream_t st);
+// the end of the Spalart-Allmaras step: met_cutsa's floor and met_samut's output
+struct SaFinish {
+  double epsk;
+  double* mut;
+};
 // impli2_eqt_3d of block l0 (-1: all): u, v are (ld, 7); w: 17 ld scratch;
 // rcp = 1: one reciprocal per line step instead of three divisions (the
 // reduced-precision forms; not bit-exact)
 // wall_ni: the first cells of the wall-law walls (nwall of them), whose
-// increments are zeroed before the update (impli2_eqt_3d.f90:384-405)
+// increments are zeroed before the update (impli2_eqt_3d.f90:384-405); fin: the
+// update followed by met_cutsa and met_samut
 cudaError_t launch_impli2(const Blk* blks, const SpaceBuf* lines, Space cells, int l0,
                           long long ld, const double* u, const double* dt, double* v,
                           const double* prim, const double* mu, const double* mut,
                           const double* cfke, const double* sn, const double* vol, double cmt,
                           double* w, int rcp, const long long* wall_ni, long long nwall,
-                          cudaStream_t st);
+                          const SaFinish* fin, cudaStream_t st);
 
 // wall laws of the adiabatic wall-law walls 'lp2' (rbord.f90:377-379: vkar,
 // cllog, yp0; the SA cv1 and the nu~ floor epsk) on the cnt list entries

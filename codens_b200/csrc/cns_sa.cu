@@ -65,13 +65,15 @@ __global__ void __launch_bounds__(256) k_teq_scalars(int mode, const double* __r
 // times 0.5 / vol.  A face value is S (s_upper + s_lower) inside the block
 // and (S * 2) s_ghost on a boundary face; every cell evaluates its six face
 // values itself (the face's two cells compute the same operands in the same
-// order, so the value is the one a stored face buffer would hold).  Without
+// order, so the value is the one a stored face buffer would hold).  Field q is
+// at f + q fs.  Without
 // branches, so that the seven cells' loads are issued together: 69 ->
 // 55 us for one scalar, 108 -> 74 for two, 121 -> 91 for three on a 2.1M-cell
 // plate (cold).
 template <int NSC>
 __global__ void __launch_bounds__(kTile) k_teq_cell(const Blk* __restrict__ blks, Space sp,
-                                                    const double* __restrict__ f, long long ld,
+                                                    const double* __restrict__ f, long long fs,
+                                                    long long ld,
                                                     const double* __restrict__ sn,
                                                     const double* __restrict__ vol,
                                                     double* __restrict__ out) {
@@ -81,14 +83,14 @@ __global__ void __launch_bounds__(kTile) k_teq_cell(const Blk* __restrict__ blks
   const long long n = cell_index(B, i, j, k);
   double s0[NSC], sl[3][NSC], su[3][NSC], Sl[3][3], Su[3][3];
 #pragma unroll
-  for (int q = 0; q < NSC; ++q) s0[q] = f[q * ld + n];
+  for (int q = 0; q < NSC; ++q) s0[q] = f[q * fs + n];
 #pragma unroll
   for (int dir = 0; dir < 3; ++dir) {
     const long long inc = ninc_of(B, dir);
 #pragma unroll
     for (int q = 0; q < NSC; ++q) {
-      sl[dir][q] = f[q * ld + n - inc];
-      su[dir][q] = f[q * ld + n + inc];
+      sl[dir][q] = f[q * fs + n - inc];
+      su[dir][q] = f[q * fs + n + inc];
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -145,6 +147,12 @@ __global__ void __launch_bounds__(kTile) k_smsa(
   const double cw1 = kCb1 / (kKappa * kKappa) + (1 + kCb2) / kSigma;
   const double kappa2 = kKappa * kKappa, uns6 = 1. / 6., cv13 = kCv1 * kCv1 * kCv1;
   const double cw36 = pow6(kCw3), cv133 = 3. * cv13, ct42 = 2. * kCt4, cb2sig = kCb2 / kSigma;
+  // the inputs of the last terms, loaded before the first division: its slow
+  // path is a branch that later loads would wait behind (128 -> 119 us on 2.1M
+  // cells, cold)
+  const double gr0 = grr[n], gr1 = grr[ld + n], gr2 = grr[2 * ld + n];
+  const double f0 = fd5x[m], f1 = fd5y[m], f2 = fd5z[m];
+  const double mun = mu[n], dn = dist[n];
   // met_difsa.f90:96-101
   double sdif = grt[n] * fd5x[n] + grt[ld + n] * fd5y[n] + grt[2 * ld + n] * fd5z[n];
   sdif = sdif * kCb2 / kSigma;
@@ -153,10 +161,10 @@ __global__ void __launch_bounds__(kTile) k_smsa(
   const double a2 = dv[2 * ld + n] - dv[6 * ld + n];  // dvxz - dvzx
   const double a3 = dv[3 * ld + n] - dv[ld + n];      // dvyx - dvxy
   const double vort = sqrt(a1 * a1 + a2 * a2 + a3 * a3);
-  const double xkhi = v6 / mu[n];
+  const double xkhi = v6 / mun;
   const double xkhi2 = xkhi * xkhi;
   const double xkhi3 = xkhi2 * xkhi;
-  const double dist2 = dist[n] * dist[n];
+  const double dist2 = dn * dn;
   const double nutilde = v6 / v1;
   const double kapd2 = kappa2 * dist2;
   const double fv1 = xkhi3 / (xkhi3 + cv13);
@@ -185,9 +193,9 @@ __global__ void __launch_bounds__(kTile) k_smsa(
   ts7[n] = 0.;
   const double xkhi4 = xkhi3 * xkhi;
   const double dfv1 =
-      (fix && !(xkhi4 > 0.)) ? 0. : cv133 * (fv1 * fv1) / (mu[n] * xkhi4);
+      (fix && !(xkhi4 > 0.)) ? 0. : cv133 * (fv1 * fv1) / (mun * xkhi4);
   const double t1 = 1. + xkhi * fv1;
-  const double dfv2 = (xkhi2 * dfv1 - 1. / mu[n]) / (t1 * t1);
+  const double dfv2 = (xkhi2 * dfv1 - 1. / mun) / (t1 * t1);
   const double dst = (fv2 / v1 + nutilde * dfv2) / kapd2;
   double dpr, dxg, dfw;
   if (!fix) {
@@ -207,7 +215,7 @@ __global__ void __launch_bounds__(kTile) k_smsa(
   const double dsm1 = kCb1 * ((1. - ft2) * (stilde + dst * v6) - stilde * v6 * dft2);
   const double dsm2 = 2. * sm2 / v6 - (cw1 * dfw - kCb1 * dft2 / kappa2) * nutilde * v6 / dist2;
   const double dsdif =
-      -cb2sig * (fd5x[m] * grr[n] + fd5y[m] * grr[ld + n] + fd5z[m] * grr[2 * ld + n]) /
+      -cb2sig * (f0 * gr0 + f1 * gr1 + f2 * gr2) /
       (v1 * v1);
   cfke[n] = fabs(dsm1 + dsm2 + dsdif);
 }
@@ -477,6 +485,28 @@ __global__ void __launch_bounds__(kTile) k_i2_update(const Blk* __restrict__ blk
   const long long n = cell_index(blks[b], i, j, k);
   v[5 * ld + n] = v[5 * ld + n] + w6[n];
   v[6 * ld + n] = v[6 * ld + n] + w7[n];
+}
+
+// the same, then met_cutsa.f90 (k_cutsa) and met_samut.f90 (k_samut) of the
+// cell, for the Spalart-Allmaras step: one pass in place of three
+// (21 + 20 + 20 -> 20 us on 2.1M cells, cold; DRAM)
+__global__ void __launch_bounds__(kTile) k_sa_finish(const Blk* __restrict__ blks, Space sp,
+                                                     long long ld,
+                                                     const double* __restrict__ w6,
+                                                     double* __restrict__ v, double epsk,
+                                                     const double* __restrict__ mu,
+                                                     double* __restrict__ mut, double cv13) {
+  int b, i, j, k;
+  if (!space_elem_sync(sp, threadIdx.x, b, i, j, k)) return;
+  const long long n = cell_index(blks[b], i, j, k);
+  double v6 = v[5 * ld + n] + w6[n];
+  if (v6 < 0.) v6 = epsk;
+  v[5 * ld + n] = v6;
+  v[6 * ld + n] = 0.;
+  const double xkhi = v6 / mu[n];
+  const double xkhi3 = xkhi * xkhi * xkhi;
+  const double fv1 = xkhi3 / (xkhi3 + cv13);
+  mut[n] = v6 * fv1;
 }
 
 // ---------------------------------------------------------------------------
@@ -798,9 +828,9 @@ cudaError_t launch_cutsa(const Blk* blks, Space cells, double* v, long long ld, 
 }
 
 cudaError_t launch_teq_grads(const Blk* blks, Space cells, int mode, int nsc,
-                             const double* v, const double* f, long long ld, const double* sn,
-                             const double* vol, double* out, double* sc, long long n0,
-                             long long n1, cudaStream_t st) {
+                             const double* v, const double* f, long long fs, long long ld,
+                             const double* sn, const double* vol, double* out, double* sc,
+                             long long n0, long long n1, cudaStream_t st) {
   if (cells.ntiles == 0) return cudaSuccess;
   if (mode != 1) {
     const int g = (int)((n1 - n0 + 255) / 256);
@@ -811,14 +841,15 @@ cudaError_t launch_teq_grads(const Blk* blks, Space cells, int mode, int nsc,
     else
       pdl(k_teq_scalars<1>, g, 256, 0, st)(mode, v, ld, n0, n1, sc);
     f = sc;
+    fs = ld;
   }
   {
     if (nsc == 3)
-      pdl(k_teq_cell<3>, grid_of(cells), kTile, 0, st)(blks, cells, f, ld, sn, vol, out);
+      pdl(k_teq_cell<3>, grid_of(cells), kTile, 0, st)(blks, cells, f, fs, ld, sn, vol, out);
     else if (nsc == 2)
-      pdl(k_teq_cell<2>, grid_of(cells), kTile, 0, st)(blks, cells, f, ld, sn, vol, out);
+      pdl(k_teq_cell<2>, grid_of(cells), kTile, 0, st)(blks, cells, f, fs, ld, sn, vol, out);
     else
-      pdl(k_teq_cell<1>, grid_of(cells), kTile, 0, st)(blks, cells, f, ld, sn, vol, out);
+      pdl(k_teq_cell<1>, grid_of(cells), kTile, 0, st)(blks, cells, f, fs, ld, sn, vol, out);
   }
   return cudaGetLastError();
 }
@@ -828,7 +859,7 @@ cudaError_t launch_impli2(const Blk* blks, const SpaceBuf* lines, Space cells, i
                           const double* prim, const double* mu, const double* mut,
                           const double* cfke, const double* sn, const double* vol, double cmt,
                           double* w, int rcp, const long long* wall_ni, long long nwall,
-                          cudaStream_t st) {
+                          const SaFinish* fin, cudaStream_t st) {
   // scratch w, zeroed when allocated: rv, cd, uf[3], ce[3], al, b6, b7, two
   // iterates x (6, 7) and the right-hand sides d6, d7 of a sweep = 17 ld.  The ghost entries of rv and of the
   // iterates are never written (the reference's zeroed rv and never-written
@@ -862,7 +893,11 @@ cudaError_t launch_impli2(const Blk* blks, const SpaceBuf* lines, Space cells, i
   if (nwall > 0)
     pdl(k_i2_wall_freeze, (unsigned)((nwall + 255) / 256), 256, 0, st)(wall_ni, nwall,
                                                                      it[cur][0], it[cur][1]);
-  pdl(k_i2_update, grid_of(cells), kTile, 0, st)(blks, cells, ld, it[cur][0], it[cur][1], v);
+  if (fin)
+    pdl(k_sa_finish, grid_of(cells), kTile, 0, st)(blks, cells, ld, it[cur][0], v, fin->epsk, mu,
+                                                   fin->mut, kCv1 * kCv1 * kCv1);
+  else
+    pdl(k_i2_update, grid_of(cells), kTile, 0, st)(blks, cells, ld, it[cur][0], it[cur][1], v);
   return cudaGetLastError();
 }
 
