@@ -895,9 +895,10 @@ cudaError_t refresh_sn32(cns_ctx* c, const double* sn) {
 }
 
 // one reduced-precision iteration on the bound state.  kMixed: FP64 residual
-// (face fluxes with FMA contraction), FP32 sweeps (precision 1).  kDefectRefresh / kDefectRegular (precision 2):
-// FP32 face fluxes; the refresh iteration also evaluates the FP64 residual,
-// advances with it and stores corr = R64 - R32 for the regular iterations.
+// (face fluxes with FMA contraction), FP32 sweeps (precision 1).
+// kDefectRefresh / kDefectRegular (precision 2): FP32 face fluxes; the refresh
+// iteration also evaluates the FP64 residual, advances with it and stores
+// corr = R64 - R32 for the regular iterations.
 enum MixedMode { kMixed, kDefectRefresh, kDefectRegular };
 
 cudaError_t enqueue_step_mixed(cns_ctx* c, MixedMode mode, bool first, bool dt_on) {
@@ -1323,7 +1324,8 @@ int cns_create(const cns_layout_t* layout, const cns_phys_t* phys,
   if (e == cudaSuccess)
     e = build_space(c, c->cells_ext, [](const Blk& B, int x[3]) {
       x[0] = B.ni + 1; x[1] = B.nj + 1; x[2] = B.nk + 1; });
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, c->device);
+  if (e == cudaSuccess)
+    e = cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, c->device);
   if (e == cudaSuccess) e = init_jacobi_25d();
   // until tuned or set: three FP64 CTAs of 16x8 per SM (one of 32x8), two
   // FP32 ones of 32x8

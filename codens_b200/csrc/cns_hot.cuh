@@ -930,8 +930,8 @@ cudaError_t residual_fused_dispatch(const Blk* blks, Tiles tl, Phys ph, Scheme s
 
 // the FP64 face kernels of one residual by flux family (atsch_num.f90:628-983):
 // ischema 14 HLLC (sch_hllc / sch_hllc_euler), 9 Rusanov (sch_rusanov, the
-// stresses always), 5 AUSM+ (sch_ausmp, Navier-Stokes), else Roe; each translation unit instantiates it with its
-// own contraction flags
+// stresses always), 5 AUSM+ (sch_ausmp, Navier-Stokes), else Roe; each
+// translation unit instantiates it with its own contraction flags
 static inline cudaError_t face_flux_dispatch(const Blk* blks, const SpaceBuf* faces, int l0,
                                              Phys ph, Scheme sc, const double* v,
                                              const double* prim, long long ld,
@@ -941,22 +941,17 @@ static inline cudaError_t face_flux_dispatch(const Blk* blks, const SpaceBuf* fa
   const Space3 sp{{faces[0].view(l0), faces[1].view(l0), faces[2].view(l0)}};
   const int g = sp.grid();
   if (g == 0) return cudaSuccess;
-  if (sc.ischema == 14 && sc.ns)
-    pdl(k_face_flux<double, true, kFluxHllc>, g, kTile, 0, st)(blks, sp, ph, sc, v, prim, ld, ps,
-                                                             tau, sn, R, G, V);
-  else if (sc.ischema == 14)
-    pdl(k_face_flux<double, false, kFluxHllc>, g, kTile, 0, st)(blks, sp, ph, sc, v, prim, ld, ps,
-                                                              tau, sn, R, G, V);
+  auto run = [&](auto kernel) {
+    pdl(kernel, g, kTile, 0, st)(blks, sp, ph, sc, v, prim, ld, ps, tau, sn, R, G, V);
+  };
+  if (sc.ischema == 14)
+    sc.ns ? run(k_face_flux<double, true, kFluxHllc>) : run(k_face_flux<double, false, kFluxHllc>);
   else if (sc.ischema == 9)
-    pdl(k_face_flux<double, true, kFluxRusanov>, g, kTile, 0, st)(blks, sp, ph, sc, v, prim, ld,
-                                                                ps, tau, sn, R, G, V);
+    run(k_face_flux<double, true, kFluxRusanov>);
   else if (sc.ischema == 5)
-    pdl(k_face_flux<double, true, kFluxAusm>, g, kTile, 0, st)(blks, sp, ph, sc, v, prim, ld, ps,
-                                                             tau, sn, R, G, V);
-  else if (sc.ns)
-    pdl(k_face_flux<double, true>, g, kTile, 0, st)(blks, sp, ph, sc, v, prim, ld, ps, tau, sn, R, G, V);
+    run(k_face_flux<double, true, kFluxAusm>);
   else
-    pdl(k_face_flux<double, false>, g, kTile, 0, st)(blks, sp, ph, sc, v, prim, ld, ps, tau, sn, R, G, V);
+    sc.ns ? run(k_face_flux<double, true>) : run(k_face_flux<double, false>);
   return cudaGetLastError();
 }
 
@@ -1565,12 +1560,14 @@ cudaError_t jacobi_25d_shape(const Blk* blks, Tiles tl, Phys ph, int qfix, int e
                              long long ld, const T* u, const T* v, const T* prim, const T* ps,
                              const T* sn, const T* coefe, const T* coefdiag, const T* d_in,
                              T* d_out, cudaStream_t st) {
+  auto run = [&](auto kernel, size_t smem) {
+    pdl(kernel, tl.ntiles, TI * TJ, smem, st)(blks, tl, ph, qfix, ld, u, v, prim, ps, sn, coefe,
+                                              coefdiag, d_in, d_out);
+  };
   if (eu)
-    pdl(k_jacobi_25d<T, true, FORM, TI, TJ>, tl.ntiles, TI * TJ, jacobi_25d_smem<TI, TJ, T, FORM, true>(), st)(
-            blks, tl, ph, qfix, ld, u, v, prim, ps, sn, coefe, coefdiag, d_in, d_out);
+    run(k_jacobi_25d<T, true, FORM, TI, TJ>, jacobi_25d_smem<TI, TJ, T, FORM, true>());
   else
-    pdl(k_jacobi_25d<T, false, FORM, TI, TJ>, tl.ntiles, TI * TJ, jacobi_25d_smem<TI, TJ, T, FORM, false>(), st)(
-            blks, tl, ph, qfix, ld, u, v, prim, ps, sn, coefe, coefdiag, d_in, d_out);
+    run(k_jacobi_25d<T, false, FORM, TI, TJ>, jacobi_25d_smem<TI, TJ, T, FORM, false>());
   return cudaGetLastError();
 }
 

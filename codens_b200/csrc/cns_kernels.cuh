@@ -231,7 +231,8 @@ template <class T>
 cudaError_t launch_accumulate_t(const Blk* blks, Space sp, const T* G, long long ld,
                                 const double* corr, double* u, float* u32,
                                 cudaStream_t st, const T* V);
-// lmx Jacobi sweeps over the real cells; the final iterate is in dpp[*cur_out]
+// the tiled Jacobi sweeps 2..lmx over the real cells (the first iterate is in
+// dpp[0]); the final iterate is in dpp[*cur_out]
 template <class T>
 cudaError_t launch_sweeps_t(const Blk* blks, Tiles tl, Phys ph, Scheme sc, int eu,
                             int lmx, long long ld, const T* u, const T* v, const T* prim,

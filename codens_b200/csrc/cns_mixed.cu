@@ -101,8 +101,8 @@ __device__ __forceinline__ float face_coef(const float4 qh, const float4 ql, flo
 // the implicit coefficients of the FP32 sweeps in one pass (the FP32 form of
 // implimf_3d.f90:111-203 / implimf_eu.f90:124-170): each real cell evaluates
 // the spectral radii of its six faces, stores the lower faces (and the upper
-// one at the end of each line) in the sweep's face pack and sums the diagonal in the reference order.
-// Every interior face is evaluated by both its cells (cheaper than a second
+// one at the end of each line) in the sweep's face pack and sums the diagonal
+// in the reference order.  Every interior face is evaluated by both its cells (cheaper than a second
 // pass over memory); a neighbour's inputs are two vector loads of the packed
 // cq32 = (u, v, w, c) and cv32 = (vol, rv) the primitive kernel writes.
 // With d1 given, the cell's first Jacobi iterate too: with a zero previous
@@ -220,15 +220,17 @@ __global__ void __launch_bounds__(256) k_pack_faces32(const Blk* __restrict__ bl
   if (q >= B.npc + B.nnn) return;
 #pragma unroll
   for (int dir = 0; dir < 3; ++dir)
-    snc[(long long)dir * ld + q] = make_float4(0.5f * sn_ptr(sn, B, dir, 0)[q], 0.5f * sn_ptr(sn, B, dir, 1)[q],
-                                   0.5f * sn_ptr(sn, B, dir, 2)[q], 0.f);
+    snc[(long long)dir * ld + q] =
+        make_float4(0.5f * sn_ptr(sn, B, dir, 0)[q], 0.5f * sn_ptr(sn, B, dir, 1)[q],
+                    0.5f * sn_ptr(sn, B, dir, 2)[q], 0.f);
 }
 }  // namespace
 
 cudaError_t launch_pack_faces32(const Blk* blks, int nblk, long long ncells, long long ld,
                                 const float* sn32, float4* snc32, cudaStream_t st) {
   if (ncells > 0)
-    pdl(k_pack_faces32, (int)((ncells + 255) / 256), 256, 0, st)(blks, nblk, ncells, ld, sn32, snc32);
+    pdl(k_pack_faces32, (int)((ncells + 255) / 256), 256, 0, st)(blks, nblk, ncells, ld, sn32,
+                                                                snc32);
   return cudaGetLastError();
 }
 

@@ -861,9 +861,10 @@ cudaError_t launch_impli2(const Blk* blks, const SpaceBuf* lines, Space cells, i
                           double* w, int rcp, const long long* wall_ni, long long nwall,
                           const SaFinish* fin, cudaStream_t st) {
   // scratch w, zeroed when allocated: rv, cd, uf[3], ce[3], al, b6, b7, two
-  // iterates x (6, 7) and the right-hand sides d6, d7 of a sweep = 17 ld.  The ghost entries of rv and of the
-  // iterates are never written (the reference's zeroed rv and never-written
-  // neighbours); every other entry read is written first.
+  // iterates x (6, 7) and the right-hand sides d6, d7 of a sweep = 17 ld.  The
+  // ghost entries of rv and of the iterates are never written (the reference's
+  // zeroed rv and never-written neighbours); every other entry read is written
+  // first.
   double *rv = w, *cd = w + ld, *uf = w + 2 * ld, *ce = w + 5 * ld, *al = w + 8 * ld,
          *b6 = w + 9 * ld, *b7 = w + 10 * ld;
   double* it[2][2] = {{w + 11 * ld, w + 12 * ld}, {w + 13 * ld, w + 14 * ld}};
