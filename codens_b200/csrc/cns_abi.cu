@@ -1007,7 +1007,7 @@ cudaError_t enqueue_step_mixed(cns_ctx* c, MixedMode mode, bool first, bool dt_o
   int cur = 0;
   if (e == cudaSuccess && point)
     e = launch_point_sweeps32(c->d_blks, all, c->ph, c->sc, !c->sc.ns, c->sc.lmax, ld,
-                              sweep32_args(c), w.snc32, w.pt32, w.d32pp[0], c->st);
+                              sweep32_args(c), w.snc32, w.pt32, w.d32pp[0], c->nsm, c->st);
   else if (e == cudaSuccess)
     e = launch_sweeps32(c->tiles32.view(-1), c->d_blks, c->ph, c->sc, !c->sc.ns, c->sc.lmax,
                         ld, c->lay.ldp, sweep32_args(c), w.d32pp, &cur, c->st);

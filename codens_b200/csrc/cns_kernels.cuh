@@ -287,7 +287,7 @@ struct Sweep32 {
 // increments in pt[0], the final iterate in d_out
 cudaError_t launch_point_sweeps32(const Blk* blks, Space cells, Phys ph, Scheme sc, int eu,
                                   int lmx, long long ld, const Sweep32& a, const float4* faces,
-                                  float4* const pt[2], float* d_out, cudaStream_t st);
+                                  float4* const pt[2], float* d_out, int nsm, cudaStream_t st);
 // sweeps 2..lmx, 2.5D over tl, after launch_coefficients32 has written the
 // first iterate into dpp[0] (lmx = 0: dpp[0] is zeroed); the final iterate
 // in dpp[*cur_out]; ldp: the padded arrays' component stride

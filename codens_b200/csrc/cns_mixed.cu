@@ -344,9 +344,13 @@ __device__ __forceinline__ void phi_acc(const Inc& x, float w0, float w1, float 
 // sums of the 2.5D sweep below in its order: the same bits): one thread per
 // cell, (d, f) of the cell and its six neighbours as four quads each from the
 // packed iterate, the new iterate and its increment written for the next
-// sweep, or (LAST) the plain iterate for the update.
-template <bool EU, bool LAST>
-__global__ void __launch_bounds__(kTile) k_sweep_point32(
+// sweep, or (LAST) the plain iterate for the update.  Latency of a cell's 40
+// loads bounds it while the grid is one wave of CTAs: MINB = 4 (128 registers)
+// issues them together, 64x32x32 cells 74 -> 67 us an iteration (Euler), 88 ->
+// 80 (Navier-Stokes).  Larger grids leave the registers to the compiler (MINB =
+// 0: 80, 6 CTAs a SM): 110592 cells 93 against 101 us.
+template <bool EU, bool LAST, int MINB>
+__global__ void __launch_bounds__(kTile, MINB) k_sweep_point32(
     const Blk* __restrict__ blks, Space sp, float gam1, float pinfl, int qfix, long long ld,
     Sweep32 a, const float4* __restrict__ faces, const float4* __restrict__ p_in,
     float4* __restrict__ p_out, float* __restrict__ d_out) {
@@ -936,7 +940,8 @@ cudaError_t launch_sweeps32(Tiles tl, const Blk* blks, Phys ph, Scheme sc, int e
 
 cudaError_t launch_point_sweeps32(const Blk* blks, Space cells, Phys ph, Scheme sc, int eu,
                                   int lmx, long long ld, const Sweep32& a, const float4* faces,
-                                  float4* const pt[2], float* d_out, cudaStream_t st) {
+                                  float4* const pt[2], float* d_out, int nsm,
+                                  cudaStream_t st) {
   if (cells.ntiles == 0) return cudaSuccess;
   const int g = grid_of(cells), q = eu ? sc.qfix_dfez : 0;
   const float g1 = (float)ph.gam1, pi = (float)ph.pinfl;
@@ -946,12 +951,15 @@ cudaError_t launch_point_sweeps32(const Blk* blks, Space cells, Phys ph, Scheme 
   for (int ls = 2; ls <= lmx; ++ls) {
     const float4* in = pt[ls & 1];
     float4* out = pt[(ls & 1) ^ 1];
-    if (eu)
-      ls < lmx ? run(k_sweep_point32<true, false>, in, out)
-               : run(k_sweep_point32<true, true>, in, out);
+    if (ls == lmx)
+      eu ? run(k_sweep_point32<true, true, 4>, in, out)
+         : run(k_sweep_point32<false, true, 4>, in, out);
+    else if (g <= 4 * nsm)
+      eu ? run(k_sweep_point32<true, false, 4>, in, out)
+         : run(k_sweep_point32<false, false, 4>, in, out);
     else
-      ls < lmx ? run(k_sweep_point32<false, false>, in, out)
-               : run(k_sweep_point32<false, true>, in, out);
+      eu ? run(k_sweep_point32<true, false, 0>, in, out)
+         : run(k_sweep_point32<false, false, 0>, in, out);
   }
   return cudaGetLastError();
 }

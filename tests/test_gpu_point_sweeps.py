@@ -74,3 +74,26 @@ def test_few_sweeps(cuda, lmax):
     v = _run(case, 2, 0)
     assert_equal_bits(v[:, rc], np.asarray(st.v).reshape(-1, case.layout.ld)[:5, rc], "state")
     assert np.isfinite(_run(case, 2, 1)[:, rc]).all()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("ns", [0, 1])
+def test_one_wave_and_more(cuda, precision, ns):
+    """FP32 point sweeps take another kernel once the cells are more than one
+    wave (four CTAs of 128 cells an SM): each of two boxes just inside one wave
+    ends in their common layout of two waves as it does alone"""
+    import torch
+    wave = 4 * 128 * torch.cuda.get_device_properties(0).multi_processor_count
+    n = int(wave ** (1. / 3.))  # 42 on 148 SMs
+
+    def batch():
+        bt = cases.batch_case(ncase=2, side=(n, n), seed=9, qfix_dfez=1 - ns, mach_range=(0.4, 0.5))
+        bt.scheme.ns = ns
+        bt.phys.reynz = 1.0e4
+        return bt
+    bt = batch()
+    v = _run(batch(), 2, precision)
+    for ib in range(2):
+        m = cases.batch_member(bt, ib)
+        want = _run(m, 2, precision)[:, m.layout.blocks[0].real_cells()]
+        assert_equal_bits(v[:, bt.layout.blocks[ib].real_cells()], want, f"box {ib}")
