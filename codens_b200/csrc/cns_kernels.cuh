@@ -123,12 +123,12 @@ struct TileBuf {
 // the sweeps touch stays in the 126 MB L2; the Navier-Stokes increments cost
 // the tiles six divisions a cell and ring cell, so their line lies higher, and
 // FP32 has half the bytes.  Whole iterations of ten sweeps, tiles against
-// points, Euler and Navier-Stokes: 64x32x32 cells 161 -> 113 us, 197 -> 135;
-// 131k 241 -> 189, 313 -> 226; 196k 289 and 305, 355 and 350; 262k 397 and
-// 419, 514 -> 479; 393k 553 and 610, 674 and 685.  FP32: 65k 131 -> 89, 145 ->
-// 105; 196k 235 -> 171, 266 -> 201; 262k 261 -> 222, 296 -> 261; 393k 348 ->
-// 338, 400 -> 397; 524k 428 and 449, 496 and 526.
-constexpr long long kPointEuler64 = 180000, kPointNs64 = 300000, kPoint32 = 400000;
+// points, Euler and Navier-Stokes: 131k cells 209 -> 178 us, 269 -> 209; 196k
+// 289 and 292, 350 -> 333; 262k 387 and 412, 467 -> 457; 295k 393 and 443, 474
+// and 491.  FP32: 131k 129 -> 116, 154 -> 141; 196k 203 -> 154, 231 -> 181;
+// 295k 271 -> 220, 310 -> 260; 393k 300 and 307, 353 and 366; 524k 369 and 416,
+// 436 and 492.
+constexpr long long kPointEuler64 = 180000, kPointNs64 = 270000, kPoint32 = 370000;
 
 // per-step scratch (device)
 struct Work {

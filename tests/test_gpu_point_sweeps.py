@@ -13,7 +13,7 @@ from ._helpers import assert_equal_bits, oracle_prepared, real
 pytestmark = pytest.mark.gpu
 
 # the largest layouts of point sweeps: FP64 Euler, FP64 Navier-Stokes, FP32
-POINT_EULER64, POINT_NS64, POINT_32 = 180000, 300000, 400000
+POINT_EULER64, POINT_NS64, POINT_32 = 180000, 270000, 370000
 
 
 def _run(case, nsteps, precision, tiles=None):
@@ -51,7 +51,7 @@ def test_point_equals_tiled(cuda, precision, ns):
 
 # the last point-sweep size and the first tiled one; odd sides, one-cell directions
 @pytest.mark.parametrize("ns,cells", [
-    (0, (60, 50, 60)), (0, (61, 59, 51)), (1, (100, 60, 50)), (1, (67, 67, 67)),
+    (0, (60, 50, 60)), (0, (61, 59, 51)), (1, (100, 60, 45)), (1, (65, 65, 64)),
     (0, (129, 2, 3)), (1, (129, 2, 3)), (0, (1, 33, 5)), (1, (1, 33, 5))])
 def test_fused_step_bits_at_the_line(cuda, ns, cells):
     case = cases.box_case(cells, seed=7, ns=bool(ns), skew=0.01, reynz=1.0e4,
