@@ -694,9 +694,8 @@ cudaError_t enqueue_met_num_ke(cns_ctx* c) {
                          b0, b1, c->st);
     if (e == cudaSuccess)
       e = launch_met_prod(c->d_blks, cb, ld, s.mut, s.v, c->sa_dv, c->ke_tprod, c->st);
-    if (e == cudaSuccess)  // the six rows of fd in one node
-      e = cudaMemset2DAsync(fdw[0] + n0, sizeof(double) * ld, 0,
-                            sizeof(double) * (size_t)(n1 - n0 + 1), 6, c->st);
+    for (int q = 0; q < 6 && e == cudaSuccess; ++q)
+      e = cudaMemsetAsync(fdw[q] + n0, 0, sizeof(double) * (size_t)(n1 - n0 + 1), c->st);
     if (e == cudaSuccess)
       e = launch_teq_grads(c->d_blks, cb, 2, 2, s.v, nullptr, 0, ld, s.sn, s.vol, fd, c->sa_sc, b0,
                            b1, c->st);
@@ -712,8 +711,9 @@ cudaError_t enqueue_met_num_ke(cns_ctx* c) {
     e = launch_roe2o(c->d_blks, c->cells_ext.view(-1), sa_harten(c), c->epsroe, c->ph.gam,
                      c->ph.gam1, s.v, c->w.prim, ld, s.sn, s.d, c->st);
   if (e == cudaSuccess)
-    e = cudaMemset2DAsync(s.u + 5 * ld, sizeof(double) * ld, 0, sizeof(double) * c->lay.ncells, 2,
-                          c->st);
+    e = cudaMemsetAsync(s.u + 5 * ld, 0, sizeof(double) * c->lay.ncells, c->st);
+  if (e == cudaSuccess)
+    e = cudaMemsetAsync(s.u + 6 * ld, 0, sizeof(double) * c->lay.ncells, c->st);
   if (e == cudaSuccess)
     e = launch_sch_turb(c->d_blks, all, s.v, c->w.prim, ld, fdr, ts6, ts7, s.d, s.sn, s.vol, s.u,
                         c->st);
@@ -752,9 +752,8 @@ cudaError_t enqueue_met_num(cns_ctx* c) {
     // reads there through its block-local index)
     long long n0, n1;
     fludc_range(c, b + 1, n0, n1);
-    if (e == cudaSuccess)  // the six rows of fd in one node
-      e = cudaMemset2DAsync(fdw[0] + n0, sizeof(double) * ld, 0,
-                            sizeof(double) * (size_t)(n1 - n0 + 1), 6, c->st);
+    for (int q = 0; q < 6 && e == cudaSuccess; ++q)
+      e = cudaMemsetAsync(fdw[q] + n0, 0, sizeof(double) * (size_t)(n1 - n0 + 1), c->st);
     if (e == cudaSuccess)
       e = launch_teq_grads(c->d_blks, cb, 2, 2, s.v, nullptr, 0, ld, s.sn, s.vol, fd, c->sa_sc, b0,
                            b1, c->st);
@@ -773,8 +772,9 @@ cudaError_t enqueue_met_num(cns_ctx* c) {
                      c->ph.gam1, s.v, c->w.prim, ld, s.sn, s.d, c->st);
   // sch_turb.f90:59-66 zeroes u(:,6:7) over every block
   if (e == cudaSuccess)
-    e = cudaMemset2DAsync(s.u + 5 * ld, sizeof(double) * ld, 0, sizeof(double) * c->lay.ncells, 2,
-                          c->st);
+    e = cudaMemsetAsync(s.u + 5 * ld, 0, sizeof(double) * c->lay.ncells, c->st);
+  if (e == cudaSuccess)
+    e = cudaMemsetAsync(s.u + 6 * ld, 0, sizeof(double) * c->lay.ncells, c->st);
   if (e == cudaSuccess)
     e = launch_sch_turb(c->d_blks, all, s.v, c->w.prim, ld, fdr, ts6, ts7, s.d, s.sn, s.vol, s.u,
                         c->st);
