@@ -364,6 +364,13 @@ cudaError_t prim_of(cns_ctx* c, int l, const double* v) {
   return launch_prim(n0, n1, v, c->lay.ld, c->w.prim, c->st);
 }
 
+// the viscous halves that accompany the face fluxes of the current scheme
+// (HLLC with the stresses), null for the other families: the buffer, allocated
+// when a scheme first needs it, then holds an earlier scheme's values
+double* viscous_halves(const cns_ctx* c) {
+  return c->sc.ischema == 14 && c->sc.ns ? c->w.V : nullptr;
+}
+
 // the residual of one block set: (optional) limiter ratios, face fluxes,
 // accumulation into u; the primitive velocities must be current
 cudaError_t residual(cns_ctx* c, int l0, double* u, const double* v,
@@ -382,9 +389,10 @@ cudaError_t residual(cns_ctx* c, int l0, double* u, const double* v,
                                  ld, ps, tau, sn, c->w.R, u, nullptr, c->st);
   if (e == cudaSuccess)
     e = launch_face_flux(c->d_blks, c->faces, l0, c->ph, c->sc, v, c->w.prim, ld, ps, tau,
-                         sn, c->w.R, c->w.G, c->st, c->w.V);
+                         sn, c->w.R, c->w.G, c->st, viscous_halves(c));
   if (e == cudaSuccess && !faces_only)
-    e = launch_accumulate(c->d_blks, c->cells.view(l0), c->w.G, ld, u, c->st, c->w.V);
+    e = launch_accumulate(c->d_blks, c->cells.view(l0), c->w.G, ld, u, c->st,
+                          viscous_halves(c));
   return e;
 }
 
@@ -825,8 +833,8 @@ cudaError_t enqueue_step(cns_ctx* c, bool first, bool dt_on) {
   if (e == cudaSuccess && c->sc.kfmg == 3) e = enqueue_dual(c, nullptr);
   if (e == cudaSuccess)
     e = launch_implicit(c->d_blks, all, c->tiles64.view(-1), c->ph, c->sc, !c->sc.ns,
-                        c->sc.lmax, s.u, sum, s.dt, s.v, nullptr, s.mu, s.mut, s.sn, s.vol,
-                        s.pression, s.cson, 1, c->w, 1, c->st);
+                        c->sc.lmax, s.u, sum, viscous_halves(c), s.dt, s.v, nullptr, s.mu, s.mut,
+                        s.sn, s.vol, s.pression, s.cson, 1, c->w, 1, c->st);
   if (e == cudaSuccess)
     e = finalize_norms(c);
   return e;
@@ -908,6 +916,7 @@ cudaError_t enqueue_step_mixed(cns_ctx* c, MixedMode mode, bool first, bool dt_o
   const Space all = c->cells.view(-1);
   const bool lim = c->sc.ns && c->sc.ilim == 1;
   const bool sum = mode == kMixed && sum_in_coefs(c);
+  double* const visc = viscous_halves(c);
   // zpres (+ zvismo), and chronos when the time step is recomputed, in one pass
   cudaError_t e =
       dt_on ? launch_zpres_chronos(c->d_blks, all, c->ph, c->sc, s.v, ld, s.pression, s.ztemp,
@@ -985,10 +994,10 @@ cudaError_t enqueue_step_mixed(cns_ctx* c, MixedMode mode, bool first, bool dt_o
       } else {
         if (e == cudaSuccess)
           e = launch_face_flux_fma(c->d_blks, c->faces, -1, c->ph, c->sc, s.v, w.prim, ld,
-                                   s.pression, s.tau, s.sn, w.R, w.G, c->st, w.V);
+                                   s.pression, s.tau, s.sn, w.R, w.G, c->st, visc);
         if (e == cudaSuccess && !sum)
           e = launch_accumulate_t<double>(c->d_blks, all, w.G, ld, nullptr, s.u, w.u32, c->st,
-                                          w.V);
+                                          visc);
       }
     }
     if (e == cudaSuccess && mode == kDefectRefresh)
@@ -1003,7 +1012,7 @@ cudaError_t enqueue_step_mixed(cns_ctx* c, MixedMode mode, bool first, bool dt_o
                               w.cv32, w.sn32, w.coefdiag32, w.snc32, w.u32,
                               c->sc.lmax >= 1 && !point ? w.d32pp[0] : nullptr,
                               point ? w.pt32[0] : nullptr, w.st32, c->ph,
-                              c->sc.ns ? 0 : c->sc.qfix_dfez, sum ? w.G : nullptr, w.V, s.u, c->st);
+                              c->sc.ns ? 0 : c->sc.qfix_dfez, sum ? w.G : nullptr, visc, s.u, c->st);
   int cur = 0;
   if (e == cudaSuccess && point)
     e = launch_point_sweeps32(c->d_blks, all, c->ph, c->sc, !c->sc.ns, c->sc.lmax, ld,
@@ -2280,8 +2289,8 @@ int cns_adjoint_prepare(cns_ctx* c) {
                   c->d_idd_ents, c->d_idd_work, c->st));
   CK(launch_prim(0, c->lay.ncells, s.v, ld, c->w.prim, c->st));
   CK(launch_implicit_coefficients(c->d_blks, all, c->ph, 1, 0., s.dt, s.v, c->w.prim, s.mu,
-                                  s.mut, s.sn, s.vol, s.cson, nullptr, 0, 0, nullptr, nullptr,
-                                  nullptr, 0, c->w, c->st));
+                                  s.mut, s.sn, s.vol, s.cson, nullptr, 0, nullptr, 0, nullptr,
+                                  nullptr, nullptr, 0, c->w, c->st));
   CK(launch_face_jac(c->d_blks, c->faces, c->ph, c->sc, s.v, s.pression, ld, s.sn, c->adj_J,
                      c->st));
   if (c->sc.precision != 0) {
@@ -2386,7 +2395,7 @@ static int implimf(cns_ctx* c, int l, int eu, const double* u, const double* dt,
   if (sc.kfmg == 3) sc.dt1min = dtpas;
   const Tiles tl = l == 0 ? c->tiles64.view() : c->tiles64_blk.view(l - 1);
   CK(launch_implicit(c->d_blks, c->cells.view(l - 1), tl, c->ph, sc, eu, lmx,
-                     const_cast<double*>(du), 0, ddt, dv, dd, dmu, dmut, sn_base(c, l, dsn), dvol,
+                     const_cast<double*>(du), 0, nullptr, ddt, dv, dd, dmu, dmut, sn_base(c, l, dsn), dvol,
                      dps, dcson, 0, c->w, 0, c->st));
   CK(sg.finish());
   return CNS_OK;

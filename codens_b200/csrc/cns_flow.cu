@@ -1205,15 +1205,15 @@ cudaError_t launch_implicit_coefficients(const Blk* blks, Space cells, Phys ph, 
                                          const double* prim, const double* mu,
                                          const double* mut, const double* sn,
                                          const double* vol, const double* cson, double* u,
-                                         int sum_faces, int rv_done, double* d1, double2* p1,
-                                         const double* ps, int qfix, Work& w,
-                                         cudaStream_t st) {
+                                         int sum_faces, const double* V, int rv_done,
+                                         double* d1, double2* p1, const double* ps, int qfix,
+                                         Work& w, cudaStream_t st) {
   if (cells.ntiles == 0) return cudaSuccess;
   const int g = grid_of(cells);
   if (!eu && !rv_done) pdl(k_impl_rv, g, kTile, 0, st)(blks, cells, ph, v, mu, mut, w.rv);
   auto run = [&](auto kernel) {
     pdl(kernel, g, kTile, 0, st)(blks, cells, dtpas, v, prim, w.ld, sn, vol, cson, w.rv, dt, u,
-                                 w.coefe, w.coefdiag, d1, p1, ps, ph, qfix, w.G, w.V, u);
+                                 w.coefe, w.coefdiag, d1, p1, ps, ph, qfix, w.G, V, u);
   };
   if (sum_faces)
     eu ? run(k_impl_coefs<true, true>) : run(k_impl_coefs<false, true>);
@@ -1246,8 +1246,8 @@ static cudaError_t point_sweeps64(const Blk* blks, Space cells, Phys ph, int qfi
 }
 
 cudaError_t launch_implicit(const Blk* blks, Space cells, Tiles tl, Phys ph, Scheme sc, int eu,
-                            int lmx, double* u, int sum_faces, const double* dt, double* v,
-                            double* d_out, const double* mu, const double* mut,
+                            int lmx, double* u, int sum_faces, const double* V, const double* dt,
+                            double* v, double* d_out, const double* mu, const double* mut,
                             const double* sn, const double* vol, const double* ps,
                             const double* cson, int rv_done, Work& w, int want_norms,
                             cudaStream_t st) {
@@ -1258,7 +1258,7 @@ cudaError_t launch_implicit(const Blk* blks, Space cells, Tiles tl, Phys ph, Sch
   // dtpas > 0: dual time stepping with physical step dtpas
   cudaError_t e = launch_implicit_coefficients(
       blks, cells, ph, eu, sc.kfmg == 3 ? sc.dt1min : 0., dt, v, w.prim, mu, mut, sn, vol, cson,
-      u, sum_faces, rv_done, lmx >= 1 && !point ? w.dpp[0] : nullptr,
+      u, sum_faces, V, rv_done, lmx >= 1 && !point ? w.dpp[0] : nullptr,
       point ? w.pt[0] : nullptr, ps, qfix, w, st);
   int cur = 0;
   if (e == cudaSuccess && point)

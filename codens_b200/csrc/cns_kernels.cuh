@@ -532,15 +532,16 @@ inline cudaError_t launch_accumulate(const Blk* blks, Space sp, const double* G,
 // dual time stepping) and, when d1 is given, the first Jacobi iterate -u / cd
 // (p1: that iterate with its flux increments, packed for the point sweeps);
 // rv_done: w.rv already holds the viscous factor (launch_grad wrote it);
-// sum_faces: u is formed from the face fluxes w.G, w.V first, else it is read
+// sum_faces: u is formed from the face fluxes w.G and, when given, the viscous
+// halves V first, else it is read
 cudaError_t launch_implicit_coefficients(const Blk* blks, Space cells, Phys ph, int eu,
                                          double dtpas, const double* dt, const double* v,
                                          const double* prim, const double* mu,
                                          const double* mut, const double* sn,
                                          const double* vol, const double* cson, double* u,
-                                         int sum_faces, int rv_done, double* d1, double2* p1,
-                                         const double* ps, int qfix, Work& w,
-                                         cudaStream_t st);
+                                         int sum_faces, const double* V, int rv_done,
+                                         double* d1, double2* p1, const double* ps, int qfix,
+                                         Work& w, cudaStream_t st);
 
 // The single-precision copies the primitive-velocity kernel writes for the
 // reduced-precision forms, each value rounded once from FP64:
@@ -596,11 +597,11 @@ cudaError_t launch_face_flux_fma(const Blk* blks, const SpaceBuf* faces, int l0,
 // the implicit phase of implimf_eu (eu = 1) or implimf_3d (eu = 0) on the
 // cells of the space: coefficients, lmx Jacobi sweeps, v += d; d_out
 // (optional) receives the final increment, want_norms stores per-tile
-// residual partials in w.normpart; sum_faces, rv_done as
+// residual partials in w.normpart; sum_faces, V, rv_done as
 // launch_implicit_coefficients
 cudaError_t launch_implicit(const Blk* blks, Space cells, Tiles tl, Phys ph, Scheme sc, int eu,
-                            int lmx, double* u, int sum_faces, const double* dt, double* v,
-                            double* d_out, const double* mu, const double* mut,
+                            int lmx, double* u, int sum_faces, const double* V, const double* dt,
+                            double* v, double* d_out, const double* mu, const double* mut,
                             const double* sn, const double* vol, const double* ps,
                             const double* cson, int rv_done, Work& w, int want_norms,
                             cudaStream_t st);
