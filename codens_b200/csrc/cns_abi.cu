@@ -1426,7 +1426,7 @@ int cns_create(const cns_layout_t* layout, const cns_phys_t* phys,
     if (e == cudaSuccess) e = upload(c, &c->d_wall_ents, wall_ents.data(), wall_ents.size());
     if (e == cudaSuccess) e = upload(c, &c->d_lp2_ni, lp2_ni.data(), lp2_ni.size());
     c->n_lp2_ni = (long long)lp2_ni.size();
-    if (e == cudaSuccess) e = dev_alloc(c, &c->d_idd_work, (size_t)(2 * nb + 1));
+    if (e == cudaSuccess) e = dev_alloc(c, &c->d_idd_work, (size_t)(3 * nb + 1));
     if (e == cudaSuccess) e = dev_alloc(c, &c->bd.nxn, (size_t)nl);
     if (e == cudaSuccess) e = dev_alloc(c, &c->bd.nyn, (size_t)nl);
     if (e == cudaSuccess) e = dev_alloc(c, &c->bd.nzn, (size_t)nl);

@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(256) k_rbord(Bnd bd, Phys ph, double* v,
   pdl_sync();
   // the injection boundaries' work starts at zero (k_clidd_count follows)
   if (blockIdx.x == 0)
-    for (int q = threadIdx.x; q < 2 * bd.nbnd + 1; q += blockDim.x) idd_work[q] = 0u;
+    for (int q = threadIdx.x; q < 3 * bd.nbnd + 1; q += blockDim.x) idd_work[q] = 0u;
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= bd.nlist) return;
   const int bb = bd.ent_bnd[e];
@@ -333,16 +333,21 @@ __global__ void __launch_bounds__(256) k_rbord(Bnd bd, Phys ph, double* v,
 // 1e-7 (at most 20 sweeps).  Each cell's iterate depends on that cell only;
 // only the number of sweeps is global.  So k_clidd_count takes every cell to
 // the first sweep t whose update is small and keeps the boundary's largest t
-// (every earlier sweep has that cell's large update); k_clidd_apply replays
-// that many sweeps and the one after, and looks at each cell's last update
-// again: a cell that was small earlier may be large there (a cell of reversed
-// flow counts as small, clidd.f90:113 divides by the signed velocity).  Then
-// its last CTA redoes the boundary from the record of all 20 sweeps.  The same
-// values as the sequential loop.  Latency of the dependent sweeps (a real
-// power each) bounds both: recording all 20 sweeps first took 28 us, the count
-// takes 12 us on a 5.5k-cell inlet.
-// work (unsigned): nbnd largest sweeps (then sweep masks of a redo), nbnd redo
-// flags, a counter of finished CTAs; k_rbord clears it.
+// (every earlier sweep has that cell's large update).  A cell of reversed flow
+// counts as small whatever its update (clidd.f90:113 divides by the signed
+// velocity) and may be large again once it turns, so such a cell records all
+// its sweeps: the boundary stops at the first sweep from t on that no reversed
+// cell holds open.  k_clidd_apply replays that many sweeps and looks at each
+// cell's last update again: should another cell be large there (rounding, at
+// velocities near 1e-9), its last CTA redoes the boundary from the record of all
+// 20 sweeps.  The same values as the sequential loop.  Latency of the dependent
+// sweeps (a real power each) bounds both: recording all 20 sweeps of every cell
+// takes 28 us on a 5.5k-cell inlet, the count 12 us.  With the redo for the
+// reversed cells too, ghosts with 5% of them took 8.2 ms on a 16k-cell inlet
+// (40 us without any), with their record 57 us.
+// work (unsigned): nbnd largest sweeps (then sweep masks of a redo), nbnd masks
+// of the reversed cells' large sweeps, nbnd redo flags, a counter of finished
+// CTAs; k_rbord clears it.
 struct IddCell {
   double usdn, usdn2, un, qn, roc0, am0, rpi, rti;
 };
@@ -395,9 +400,17 @@ __global__ void __launch_bounds__(64) k_clidd_count(Bnd bd, Phys ph, const long 
   const long long e = ents[q];
   IddCell c;
   idd_setup(bd, ph, v, ld, e, c);
+  const int b = bd.ent_bnd[e];
   unsigned t = 0;
-  while (t < 20 && idd_sweep(ph, c) > kIddTol) ++t;
-  atomicMax(&work[bd.ent_bnd[e]], t);
+  double resi = 0.;
+  while (t < 20 && (resi = idd_sweep(ph, c)) > kIddTol) ++t;
+  atomicMax(&work[b], t);
+  if (t < 20 && resi < 0.) {
+    unsigned late = 0u;
+    while (++t < 20)
+      if (idd_sweep(ph, c) > kIddTol) late |= 1u << t;
+    if (late) atomicOr(&work[bd.nbnd + b], late);
+  }
 }
 
 // nsweep sweeps of entry e, then its ghost state; returns the last update
@@ -441,13 +454,15 @@ __global__ void __launch_bounds__(64) k_clidd_apply(Bnd bd, Phys ph, const long 
                                                    double* ps, double* temp, double* cson,
                                                    unsigned* work) {
   pdl_sync();
-  unsigned *flag = work + bd.nbnd, *count = work + 2 * bd.nbnd;
+  const unsigned* late = work + bd.nbnd;
+  unsigned *flag = work + 2 * bd.nbnd, *count = work + 3 * bd.nbnd;
   const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (q < nent) {
     const long long e = ents[q];
     const int b = bd.ent_bnd[e];
-    const int m = (int)work[b], nsweep = m < 20 ? m + 1 : 20;
-    const double resi = idd_apply(bd, ph, e, nsweep, v, ld, ps, temp, cson);
+    // the first sweep from work[b] on that no reversed cell holds open (or 20)
+    const int m = __ffs((int)(~late[b] >> work[b])) - 1 + (int)work[b];
+    const double resi = idd_apply(bd, ph, e, m < 20 ? m + 1 : 20, v, ld, ps, temp, cson);
     if (m < 20 && resi > kIddTol) atomicOr(&flag[b], 1u);
   }
   __shared__ unsigned last;
