@@ -198,7 +198,11 @@ cudaError_t build_space(cns_ctx* c, SpaceBuf& s, F ext_of) {
 // iteration, a batch of 24 uneven boxes 1.56 -> 1.52 ms.
 constexpr double kTilePrologue = 2.5;
 
+// (kc past the deepest block is the tiling of whole columns; slots 0: no cut.)
 int sweep_depth(const Blk* b0, const Blk* b1, int ti, int tj, int kc, int slots) {
+  int planes = 1;
+  for (const Blk* p = b0; p < b1; ++p) planes = std::max(planes, p->nk - 1);
+  kc = std::min(kc, planes);
   int best = kc;
   double cost = 1e300;
   for (int d = kc; d >= 1 && slots > 0; --d) {

@@ -73,6 +73,29 @@ def test_rejects_unknown_shape(cuda):
     s.close()
 
 
+@pytest.mark.parametrize("kc", [10**9, 2**31 - 1])
+def test_any_plane_count_is_a_tiling(cuda, kc):
+    """a plane count past the deepest block means whole columns; setting it
+    takes no longer than any other (milliseconds; the bound allows a slow host)"""
+    import time
+
+    from codens_b200.solver import CodeNS
+    ref, _ = _run("channel", 0, (32, 8, 8))
+    case = SMALL["channel"]()
+    s = CodeNS(case)
+    s.metric()
+    t = time.perf_counter()
+    for precision in (0, 1):
+        s.set_sweep_tiles(precision, 16, 8, kc)
+        assert s.sweep_tiles(precision)[:3] == (16, 8, kc)
+    s.set_residual_tiles(16, 8, kc)
+    assert time.perf_counter() - t < 2.0
+    s.atsch_num(3)
+    v = s.v.cpu().numpy().reshape(5, case.layout.ld)[:, real(case)]
+    s.close()
+    assert_equal_bits(v, ref, "state")
+
+
 @pytest.mark.parametrize("name", ["box_ns", "channel", "box_eu_qfix", "box_pinfl"])
 def test_fused_residual_variant_gives_the_same_bits(cuda, name):
     """the fused residual kernel (three face directions and the accumulation
