@@ -338,9 +338,10 @@ __global__ void __launch_bounds__(256) k_rbord(Bnd bd, Phys ph, double* v,
 // velocity) and may be large again once it turns, so such a cell records all
 // its sweeps: the boundary stops at the first sweep from t on that no reversed
 // cell holds open.  k_clidd_apply replays that many sweeps and looks at each
-// cell's last update again: should another cell be large there (rounding, at
-// velocities near 1e-9), its last CTA redoes the boundary from the record of all
-// 20 sweeps.  The same values as the sequential loop.  Latency of the dependent
+// cell's last update again: should a forward cell be large there (in a rotating
+// frame the derivative may vanish beside its iterate), its last CTA redoes the
+// boundary from the record of all 20 sweeps.  The same values as the sequential
+// loop.  Latency of the dependent
 // sweeps (a real power each) bounds both: recording all 20 sweeps of every cell
 // takes 28 us on a 5.5k-cell inlet, the count 12 us.  With the redo for the
 // reversed cells too, ghosts with 5% of them took 8.2 ms on a 16k-cell inlet
