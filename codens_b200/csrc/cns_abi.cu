@@ -2288,6 +2288,7 @@ int cns_adjoint_prepare(cns_ctx* c) {
                   c->w.status, c->st));
   CK(launch_chronos(c->d_blks, all, c->ph, c->sc, s.mu, s.mut, s.v, ld, s.dt, s.sn, s.vol,
                     s.cson, c->st));
+  if (c->sc.kdtl == 0) CK(ensure_dtpart(c));
   CK(global_dt(c));
   CK(launch_rbord(c->bd, c->ph, s.v, ld, s.pression, s.ztemp, s.cson, c->n_idd_ent,
                   c->d_idd_ents, c->d_idd_work, c->st));

@@ -60,3 +60,34 @@ def test_global_dt_below_dt1min_is_an_error(cuda):
         s.atsch_num(1)
     assert ei.value.code == abi.CNS_EDT
     s.close()
+
+
+def test_adjoint_prepared_with_the_global_step(cuda):
+    """as the first call on a context (its step reduction has no scratch yet) and
+    after one that has made it: the same transposed implicit phase"""
+    from codens_b200.solver import CodeNS
+    torch = cuda
+    case = SMALL["box_eu_qfix"]()
+    case.scheme.kdtl = 0
+    case.scheme.dt1min = 1e-9
+    ld, rc = case.layout.ld, real(case)
+    y = torch.zeros(5, ld, dtype=torch.float64, device="cuda")
+    y[:, torch.as_tensor(rc, device="cuda")] = 1.0
+    y = y.reshape(-1)
+    outs = []
+    for warm in (False, True):
+        s = CodeNS(case)
+        s.metric()
+        if warm:
+            s.dt.fill_(1.0)
+            torch.cuda.synchronize()
+            s.chrono_global(s.dt)
+        s.adjoint_prepare()
+        out = torch.zeros(5 * ld, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        s.adjoint_lt(y, out)
+        s.sync()
+        outs.append(out.cpu().numpy().reshape(5, ld)[:, rc])
+        s.close()
+    assert np.isfinite(outs[0]).all() and (outs[0] != 0.0).any()
+    assert_equal_bits(outs[0], outs[1], "L^T y")
