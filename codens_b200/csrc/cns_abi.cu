@@ -870,7 +870,6 @@ cudaError_t ensure_mixed(cns_ctx* c) {
   if (e == cudaSuccess) e = dev_alloc(c, &w.G32, (size_t)(15 * ld));
   if (e == cudaSuccess) e = dev_alloc(c, &w.R32, (size_t)(15 * ld));
   if (e == cudaSuccess) e = dev_alloc(c, &w.u32, (size_t)(5 * ld));
-  if (e == cudaSuccess) e = dev_alloc(c, &w.coefe32, (size_t)(3 * ld));
   if (e == cudaSuccess) e = dev_alloc(c, &w.coefdiag32, (size_t)ld);
   // the sweep's padded arrays (zeroed: their padding and ghost cells are
   // never written, and the sweep masks them)
@@ -879,8 +878,7 @@ cudaError_t ensure_mixed(cns_ctx* c) {
   if (e == cudaSuccess) e = dev_alloc(c, &w.st32, (size_t)(6 * ldp));
   if (e == cudaSuccess) e = dev_alloc(c, &w.cq32, (size_t)ld);
   if (e == cudaSuccess) e = dev_alloc(c, &w.cv32, (size_t)ld);
-  for (int q = 0; q < 2 && e == cudaSuccess && c->lay.nreal <= kPoint32; ++q)
-    e = dev_alloc(c, &w.pt32[q], (size_t)(4 * ldp), false);
+  w.point32 = c->lay.nreal <= kPoint32;
   if (e == cudaSuccess) {
     std::vector<unsigned char> maps;
     e = encode_sweep32_maps(c->lay.blks, w.st32, w.d32pp, maps);
@@ -1009,18 +1007,18 @@ cudaError_t enqueue_step_mixed(cns_ctx* c, MixedMode mode, bool first, bool dt_o
   }
   if (e == cudaSuccess && c->sc.kfmg == 3) e = enqueue_dual(c, w.u32);
   // single-precision coefficients and implicit sweeps, FP64 update
-  const bool point = w.pt32[0] && c->sc.lmax >= 2;
+  const bool point = w.point32 && c->sc.lmax >= 2;
   if (e == cudaSuccess)
     e = launch_coefficients32(c->d_blks, all, !c->sc.ns, ld,
                               c->sc.kfmg == 3 ? c->sc.dt1min : 0., s.dt, s.vol, w.cq32,
                               w.cv32, w.sn32, w.coefdiag32, w.snc32, w.u32,
                               c->sc.lmax >= 1 && !point ? w.d32pp[0] : nullptr,
-                              point ? w.pt32[0] : nullptr, w.st32, c->ph,
+                              point ? w.point_iterate32(0) : nullptr, w.st32, c->ph,
                               c->sc.ns ? 0 : c->sc.qfix_dfez, sum ? w.G : nullptr, visc, s.u, c->st);
   int cur = 0;
   if (e == cudaSuccess && point)
     e = launch_point_sweeps32(c->d_blks, all, c->ph, c->sc, !c->sc.ns, c->sc.lmax, ld,
-                              sweep32_args(c), w.snc32, w.pt32, w.d32pp[0], c->nsm, c->st);
+                              sweep32_args(c), w.snc32, w, w.d32pp[0], c->nsm, c->st);
   else if (e == cudaSuccess)
     e = launch_sweeps32(c->tiles32.view(-1), c->d_blks, c->ph, c->sc, !c->sc.ns, c->sc.lmax,
                         ld, c->lay.ldp, sweep32_args(c), w.d32pp, &cur, c->st);
@@ -1461,11 +1459,7 @@ int cns_create(const cns_layout_t* layout, const cns_phys_t* phys,
   if (e == cudaSuccess) e = dev_alloc(c, &c->w.rv, (size_t)ld);
   c->w.point_eu = c->lay.nreal <= kPointEuler64;
   c->w.point_ns = c->lay.nreal <= kPointNs64;
-  for (int q = 0; q < 2 && e == cudaSuccess; ++q) {
-    e = dev_alloc(c, &c->w.dpp[q], (size_t)(5 * ld));
-    if (e == cudaSuccess && (c->w.point_eu || c->w.point_ns))
-      e = dev_alloc(c, &c->w.pt[q], (size_t)(7 * ld), false);
-  }
+  for (int q = 0; q < 2 && e == cudaSuccess; ++q) e = dev_alloc(c, &c->w.dpp[q], (size_t)(5 * ld));
   if (e == cudaSuccess) e = dev_alloc(c, &c->w.normpart, (size_t)(15 * c->cells.ntiles));
   if (e == cudaSuccess) e = dev_alloc(c, &c->w.norms, 16);
   for (size_t b = 0; b < c->lay.blks.size(); ++b) {
@@ -2303,6 +2297,7 @@ int cns_adjoint_prepare(cns_ctx* c) {
     // rounded once); A^T lambda stays FP64
     CK(ensure_mixed(c));
     CK(refresh_sn32(c, s.sn));
+    if (!c->w.coefe32) CK(dev_alloc(c, &c->w.coefe32, (size_t)(3 * ld)));
     CK(launch_to_float(c->w.coefe, c->w.coefe32, 3 * ld, c->st));
     CK(launch_to_float(c->w.coefdiag, c->w.coefdiag32, ld, c->st));
   }

@@ -1238,8 +1238,8 @@ cudaError_t launch_implicit_coefficients(const Blk* blks, Space cells, Phys ph, 
   return cudaGetLastError();
 }
 
-// sweeps 2..lmx of a small grid (the first iterate is in w.pt[0]); the final
-// iterate in w.dpp[0]
+// sweeps 2..lmx of a small grid (the first iterate is in w.point_iterate(0));
+// the final iterate in w.dpp[0]
 static cudaError_t point_sweeps64(const Blk* blks, Space cells, Phys ph, int qfix, int eu,
                                   int lmx, const double* u, const double* v, const double* ps,
                                   const double* sn, Work& w, cudaStream_t st) {
@@ -1249,8 +1249,8 @@ static cudaError_t point_sweeps64(const Blk* blks, Space cells, Phys ph, int qfi
                                 w.coefdiag, in, out, w.dpp[0]);
   };
   for (int ls = 2; ls <= lmx; ++ls) {
-    const double2* in = w.pt[ls & 1];
-    double2* out = w.pt[(ls & 1) ^ 1];
+    const double2* in = w.point_iterate(ls & 1);
+    double2* out = w.point_iterate((ls & 1) ^ 1);
     if (eu)
       ls < lmx ? run(k_jacobi_point<true, false>, in, out)
                : run(k_jacobi_point<true, true>, in, out);
@@ -1275,7 +1275,7 @@ cudaError_t launch_implicit(const Blk* blks, Space cells, Tiles tl, Phys ph, Sch
   cudaError_t e = launch_implicit_coefficients(
       blks, cells, ph, eu, sc.kfmg == 3 ? sc.dt1min : 0., dt, v, w.prim, mu, mut, sn, vol, cson,
       u, sum_faces, V, rv_done, lmx >= 1 && !point ? w.dpp[0] : nullptr,
-      point ? w.pt[0] : nullptr, ps, qfix, w, st);
+      point ? w.point_iterate(0) : nullptr, ps, qfix, w, st);
   int cur = 0;
   if (e == cudaSuccess && point)
     e = point_sweeps64(blks, cells, ph, qfix, eu, lmx, u, v, ps, sn, w, st);

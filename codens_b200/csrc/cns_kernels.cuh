@@ -144,9 +144,16 @@ struct Work {
   double* coefdiag = nullptr; // [ld]
   double* rv = nullptr;       // [ld]
   double* dpp[2] = {nullptr, nullptr};   // Jacobi iterates, [5][ld] each
-  double2* pt[2] = {nullptr, nullptr};   // point sweeps: (d, f) packed, [7][ld] each
   bool point_eu = false, point_ns = false;  // FP64 point sweeps by equations
-  float4* pt32[2] = {nullptr, nullptr};  // and in FP32, padded [4][ldp] each
+  bool point32 = false;                     // FP32 point sweeps
+  // The point sweeps' packed iterates (d, f): FP64 [7][ld] double2, FP32 padded
+  // [4][ldp] float4 (ldp <= 1.6 ld: rows of at least four cells rounded up to a
+  // multiple of four).  Iterate 0 lies in R, which the face fluxes have read
+  // when the coefficient kernel writes it, and iterate 1, first written by the
+  // second sweep, in G, which that kernel has summed: [15][ld] doubles each,
+  // written in full again before they are next read.
+  double2* point_iterate(int q) const { return reinterpret_cast<double2*>(q ? G : R); }
+  float4* point_iterate32(int q) const { return reinterpret_cast<float4*>(q ? G : R); }
   double* normpart = nullptr; // per tile partial norms [ntiles][15]
   double* norms = nullptr;    // [16]
   double* chunksum = nullptr; // norm sums [nblk * norm_chunks][15]
@@ -157,7 +164,7 @@ struct Work {
   bool mixed_ready = false;
   float *v32 = nullptr, *prim32 = nullptr, *ps32 = nullptr, *tau32 = nullptr;
   float *sn32 = nullptr, *G32 = nullptr, *R32 = nullptr, *u32 = nullptr;
-  float *coefe32 = nullptr, *coefdiag32 = nullptr;
+  float *coefe32 = nullptr, *coefdiag32 = nullptr;  // coefe32: the FP32 adjoint's
   float* d32pp[2] = {nullptr, nullptr};  // FP32 iterates, padded [5][ldp] each
   float* st32 = nullptr;      // the FP32 sweep's state, padded [6][ldp]
   float4* cq32 = nullptr;     // the FP32 coefficients' inputs (u, v, w, c) [ld]
@@ -284,10 +291,10 @@ struct Sweep32 {
   int* status;         // bit 4: a box wait gave up
 };
 // sweeps 2..lmx of a small grid (kPoint32): the first iterate with its
-// increments in pt[0], the final iterate in d_out
+// increments in w.point_iterate32(0), the final iterate in d_out
 cudaError_t launch_point_sweeps32(const Blk* blks, Space cells, Phys ph, Scheme sc, int eu,
                                   int lmx, long long ld, const Sweep32& a, const float4* faces,
-                                  float4* const pt[2], float* d_out, int nsm, cudaStream_t st);
+                                  const Work& w, float* d_out, int nsm, cudaStream_t st);
 // sweeps 2..lmx, 2.5D over tl, after launch_coefficients32 has written the
 // first iterate into dpp[0] (lmx = 0: dpp[0] is zeroed); the final iterate
 // in dpp[*cur_out]; ldp: the padded arrays' component stride

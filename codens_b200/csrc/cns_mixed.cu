@@ -940,8 +940,7 @@ cudaError_t launch_sweeps32(Tiles tl, const Blk* blks, Phys ph, Scheme sc, int e
 
 cudaError_t launch_point_sweeps32(const Blk* blks, Space cells, Phys ph, Scheme sc, int eu,
                                   int lmx, long long ld, const Sweep32& a, const float4* faces,
-                                  float4* const pt[2], float* d_out, int nsm,
-                                  cudaStream_t st) {
+                                  const Work& w, float* d_out, int nsm, cudaStream_t st) {
   if (cells.ntiles == 0) return cudaSuccess;
   const int g = grid_of(cells), q = eu ? sc.qfix_dfez : 0;
   const float g1 = (float)ph.gam1, pi = (float)ph.pinfl;
@@ -949,8 +948,8 @@ cudaError_t launch_point_sweeps32(const Blk* blks, Space cells, Phys ph, Scheme 
     pdl(kernel, g, kTile, 0, st)(blks, cells, g1, pi, q, ld, a, faces, in, out, d_out);
   };
   for (int ls = 2; ls <= lmx; ++ls) {
-    const float4* in = pt[ls & 1];
-    float4* out = pt[(ls & 1) ^ 1];
+    const float4* in = w.point_iterate32(ls & 1);
+    float4* out = w.point_iterate32((ls & 1) ^ 1);
     if (ls == lmx)
       eu ? run(k_sweep_point32<true, true, 4>, in, out)
          : run(k_sweep_point32<false, true, 4>, in, out);

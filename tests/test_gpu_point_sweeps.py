@@ -97,3 +97,21 @@ def test_one_wave_and_more(cuda, precision, ns):
         m = cases.batch_member(bt, ib)
         want = _run(m, 2, precision)[:, m.layout.blocks[0].real_cells()]
         assert_equal_bits(v[:, bt.layout.blocks[ib].real_cells()], want, f"box {ib}")
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_point_sweeps_take_no_scratch_of_their_own(cuda, precision):
+    """the packed iterates lie in buffers that are free during the sweeps: a
+    layout of point sweeps holds as much device scratch a cell as a tiled one (the
+    tile and boundary lists weigh a little more on the smaller)"""
+    from codens_b200.solver import CodeNS
+    per_cell = []
+    for cells in ((50, 50, 50), (80, 80, 80)):
+        case = cases.box_case(cells, seed=7, qfix_dfez=1)
+        case.scheme.precision = precision
+        s = CodeNS(case)
+        s.metric()
+        s.atsch_num(1)
+        per_cell.append(s.scratch_bytes / case.layout.ld)
+        s.close()
+    assert per_cell[0] < 1.1 * per_cell[1], per_cell
