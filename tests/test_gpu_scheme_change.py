@@ -72,3 +72,33 @@ def test_flux_routine_after_hllc(cuda):
         s.close()
     for q in range(3):
         assert_equal_bits(out[3 + q], out[q], "residual")
+
+
+def test_setting_a_scheme_waits_for_no_iteration(cuda):
+    """the block table follows the iterations in flight on the stream, so that the
+    call returns while they run, and those after it see the new values"""
+    import time
+
+    from codens_b200.solver import CodeNS
+    out = []
+    for wait in (True, False):
+        case = cases.box_case((96, 96, 96), seed=5, qfix_dfez=1, lmax=10)
+        s = CodeNS(case)
+        s.metric()
+        s.set_sweep_tiles(0, 16, 8, 16)
+        s.atsch_num(1)
+        t = time.perf_counter()
+        s.atsch_num_launch(200)
+        if wait:
+            s.sync()
+            march = time.perf_counter() - t
+        t = time.perf_counter()
+        case.scheme.eta = 2.0
+        s.set_scheme(case.scheme)
+        if not wait:
+            assert time.perf_counter() - t < 0.2 * march
+        s.atsch_num(2)
+        out.append(s.v.cpu().numpy().reshape(-1, case.layout.ld)[:, real(case)])
+        s.close()
+    assert np.isfinite(out[0]).all()
+    assert_equal_bits(out[1], out[0], "state")
