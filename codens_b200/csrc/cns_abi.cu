@@ -273,6 +273,14 @@ cudaError_t build_sweep_tiles(cns_ctx* c, bool fp32, TileBuf& t, int ti, int tj,
   return e;
 }
 
+// the same tilings cut again, after what the resident CTAs depend on has changed
+cudaError_t recut_sweep_tiles(cns_ctx* c, bool fp32) {
+  TileBuf& t = fp32 ? c->tiles32 : c->tiles64;
+  cudaError_t e = cudaStreamSynchronize(c->st);
+  if (e == cudaSuccess) e = build_sweep_tiles(c, fp32, t, t.ti, t.tj, t.kc);
+  return e;
+}
+
 // the FP32 sweep tiles run as a persistent launch: one CTA per resident slot
 // of the GPU (every SM times the kernel's CTAs per SM), taking tiles in turn
 void persistent_sweep32(cns_ctx* c) {
@@ -1521,6 +1529,7 @@ int cns_set_scheme(cns_ctx* c, const cns_scheme_t* s) {
                 "kdefect >= 1, ischema in {1,5,7,9,12,14} (5: ns only; defect correction: Roe "
                 "only), kfmg in "
                 "{0,3} (3: dt1min > 0, kdualns in {0,1,2})");
+  const bool other_sweeps = !c->sc.ns != !s->ns;  // Euler, Navier-Stokes kernels
   c->sc.ns = s->ns;
   c->sc.muscl = s->muscl;
   c->sc.xk = s->xk;
@@ -1550,7 +1559,11 @@ int cns_set_scheme(cns_ctx* c, const cns_scheme_t* s) {
   if (c->d_blks)
     CK(copy_in(c, c->d_blks, c->lay.blks.data(), sizeof(Blk) * c->lay.blks.size()));
   drop_graphs(c);
-  persistent_sweep32(c);  // the Euler and Navier-Stokes instantiations differ
+  if (c->d_blks && other_sweeps) {
+    CK(recut_sweep_tiles(c, false));
+    CK(recut_sweep_tiles(c, true));
+  }
+  persistent_sweep32(c);
   c->mixed_iter = 0;  // a new scheme restarts the defect refresh schedule
   if (c->w.ld > 0) CK(ensure_hllc_v(c));
   return CNS_OK;
@@ -2568,8 +2581,8 @@ int cns_set_sweep_tiles(cns_ctx* c, int precision, int ti, int tj, int kc) {
 
 int cns_set_sweep_staging(cns_ctx* c, int mode) {
   if (!c || mode < 0 || mode > 1) return CNS_EINVAL;
-  CK(cudaStreamSynchronize(c->st));
   c->staging32 = mode;
+  CK(recut_sweep_tiles(c, true));
   persistent_sweep32(c);
   drop_graphs(c);
   return CNS_OK;

@@ -105,3 +105,32 @@ def test_one_block_calls_equal_the_oracle(cuda, ns, tiles):
         assert np.isfinite(a).all()
         assert_equal_bits(t.cpu().numpy().reshape(5, ld)[:, rc], a, what)
     s.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_tiles_after_a_change_of_equations_and_staging(cuda, precision):
+    """the tile lists are cut for the equations and the staging: changed on one
+    context, the state of a fresh one"""
+    from codens_b200.solver import CodeNS
+    torch = cuda
+    want = _run("narrow", precision, (16, 8, 16), staging=1)
+    case = LARGE["narrow"]()
+    case.scheme.precision = precision
+    case.scheme.ns = 0
+    s = CodeNS(case)
+    s.metric()
+    s.set_sweep_tiles(precision, 16, 8, 16)
+    v0 = s.v.clone()
+    torch.cuda.synchronize()
+    s.atsch_num(1)
+    case.scheme.ns = 1
+    s.set_scheme(case.scheme)
+    s.set_sweep_staging(1)
+    assert s.sweep_tiles(precision)[:3] == (16, 8, 16)
+    with torch.cuda.stream(s.stream):
+        s.v.copy_(v0)
+    s.set_cycle(0, 0)
+    s.atsch_num(1 if precision == 0 else 2)
+    v = s.v.cpu().numpy().reshape(-1, case.layout.ld)[:5, real(case)]
+    s.close()
+    assert_equal_bits(v, want, "state")
