@@ -1150,15 +1150,15 @@ cudaError_t launch_jacobi_25d_t<double>(const Blk* blks, Tiles tl, Phys ph, int 
                                         const double* prim, const double* ps, const double* sn,
                                         const double* coefe, const double* coefdiag,
                                         const double* d_in, double* d_out, cudaStream_t st) {
-  return jacobi_25d_dispatch<double, 0>(blks, tl, ph, qfix, eu, ld, u, v, prim, ps, sn, coefe,
+  return jacobi_25d_dispatch<double>(blks, tl, ph, qfix, eu, ld, u, v, prim, ps, sn, coefe,
                                         coefdiag, d_in, d_out, st);
 }
 
 int jacobi_25d_blocks_per_sm(int ti, int tj, int eu) {
   int n = 0;
 #define CNS_OCC1(A, B, E)                                                                   \
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_jacobi_25d<double, E, 0, A, B>, A * B, \
-                                                jacobi_25d_smem<A, B, double, 0, E>())
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_jacobi_25d<double, E, A, B>, A * B, \
+                                                jacobi_25d_smem<A, B, double, E>())
 #define CNS_OCC(A, B)                                  \
   if (ti == A && tj == B) {                            \
     if (eu) CNS_OCC1(A, B, true);                      \
@@ -1175,7 +1175,7 @@ int jacobi_25d_blocks_per_sm(int ti, int tj, int eu) {
 }
 
 cudaError_t init_jacobi_25d() {
-  cudaError_t e = jacobi_25d_attr<double, 0>();
+  cudaError_t e = jacobi_25d_attr<double>();
   if (e == cudaSuccess) e = init_jacobi_25d_float();
   return e;
 }

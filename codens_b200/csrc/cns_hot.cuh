@@ -19,7 +19,6 @@
 // an anonymous namespace.
 #pragma once
 #include <cfloat>
-#include <type_traits>
 
 #include "cns_kernels.cuh"
 
@@ -1094,37 +1093,22 @@ __device__ __forceinline__ void jacobi_df(const T dn[5], T v1, T v2, T v3, T v4,
   }
 }
 
-// Reduced-precision sweep that stores no flux increments: each neighbour's
-// increment f(v+d) - f(v) is recomputed from its state and iterate (ghost
-// neighbours contribute zero, as their stored increments do in the reference
-// sweep).  A sweep then moves the iterate and the per-iteration constants
-// only.  Used by the mixed forms, where the sweeps only precondition the
-// pseudo-time step.
-//
-// The increment is evaluated in difference form: with q the velocity, rho'
-// = rho + d_rho, dq = (d_m - q d_rho) / rho' and dp = p' - p,
+// The increment f(v+d) - f(v) of the FP32 sweeps, in difference form: with q
+// the velocity, rho' = rho + d_rho, dq = (d_m - q d_rho) / rho' and dp = p' - p,
 //   rho' u'u' - rho u u = d_rho u u + rho' (2 u du + du du) (+ dp on the
 //   diagonal), u' (E' + p' - pinfl) - u (E + p - pinfl) = du H' + u (dE + dp),
 // the same quantities as implimf_3d.f90:430-463 / implimf_eu.f90:301-312 in
 // exact arithmetic, but exactly zero for d = 0.  The reference form cancels
 // O(1) fluxes, and in FP32 that leaves a rounding residue of ~1e-7 at d = 0
 // which would hold the iteration off the FP64 steady state.
-template <class T>
-__device__ __forceinline__ T rcpT(T a) {
-  return T(1.) / a;
-}
-template <>
-__device__ __forceinline__ float rcpT<float>(float a) {
-  return __fdividef(1.f, a);
-}
-
-// FP32 form of df_diff with every operation spelled out as a rounding
-// intrinsic (never contracted or reordered by the compiler).  A sweep
-// evaluates the same cell's increment at different places of the kernel --
-// a tile's first plane from global memory, a ring or patch cell staged in
-// shared memory -- and which place a cell takes depends on the tiling; with
-// explicit roundings every place gives the same bits, so the FP32 sweeps are
-// independent of the tiling the autotuner picks.
+//
+// Every operation is spelled out as a rounding intrinsic (never contracted or
+// reordered by the compiler).  A sweep evaluates the same cell's increment at
+// different places of the kernels -- a tile's first plane from global memory, a
+// ring or patch cell staged in shared memory, a point sweep's own cell -- and
+// which place a cell takes depends on the tiling; with explicit roundings every
+// place gives the same bits, so the FP32 sweeps are independent of the tiling
+// the autotuner picks.
 template <bool EU>
 __device__ __forceinline__ void df_diff_f32(const float dd[5], float rho, float E, float p,
                                             float qu, float qv, float qw, float gam1,
@@ -1159,48 +1143,6 @@ __device__ __forceinline__ void df_diff_f32(const float dd[5], float rho, float 
   // Euler form keeps it unless qfix (a flagged non-reference option) is set
   f[8] = (EU && !qfix) ? __fmaf_rn(h1, ir1, -__fmul_rn(h0, qw))
                        : __fmaf_rn(dw, h1, __fmul_rn(qw, de));
-}
-
-template <class T, bool EU>
-__device__ __forceinline__ void df_diff(const T dd[5], T rho, T E, T p, T qu, T qv, T qw,
-                                        T gam1, T pinfl, int qfix, T f[9]) {
-  if constexpr (std::is_same<T, float>::value) {
-    df_diff_f32<EU>(dd, rho, E, p, qu, qv, qw, gam1, pinfl, qfix, f);
-    return;
-  }
-  const T r1 = rho + dd[0];
-  const T ir1 = rcpT(r1);
-  const T du = (dd[1] - qu * dd[0]) * ir1;
-  const T dv = (dd[2] - qv * dd[0]) * ir1;
-  const T dw = (dd[3] - qw * dd[0]) * ir1;
-  const T dk = dd[0] * (qu * qu + qv * qv + qw * qw) +
-               r1 * (T(2.) * (qu * du + qv * dv + qw * dw) + du * du + dv * dv + dw * dw);
-  const T dp = gam1 * (dd[4] - T(0.5) * dk);
-  const T h0 = E + p - pinfl;
-  const T h1 = h0 + dd[4] + dp;
-  const T de = dd[4] + dp;
-  f[0] = dd[0] * qu * qu + r1 * (T(2.) * qu * du + du * du) + dp;
-  f[1] = dd[0] * qu * qv + r1 * (qu * dv + qv * du + du * dv);
-  f[2] = dd[0] * qu * qw + r1 * (qu * dw + qw * du + du * dw);
-  f[3] = du * h1 + qu * de;
-  f[4] = dd[0] * qv * qv + r1 * (T(2.) * qv * dv + dv * dv) + dp;
-  f[5] = dd[0] * qv * qw + r1 * (qv * dw + qw * dv + dv * dw);
-  f[6] = dv * h1 + qv * de;
-  f[7] = dd[0] * qw * qw + r1 * (T(2.) * qw * dw + dw * dw) + dp;
-  // implimf_eu.f90:312 lacks the *wi factor of the z energy increment; the
-  // Euler form keeps it unless qfix (a flagged non-reference option) is set
-  f[8] = (EU && !qfix) ? h1 * ir1 - h0 * qw : dw * h1 + qw * de;
-}
-
-template <class T, bool EU>
-__device__ __forceinline__ void df_of(const T* __restrict__ v, const T* __restrict__ prim,
-                                      const T* __restrict__ ps, const T* __restrict__ d,
-                                      long long ld, long long n, T gam1, T pinfl, int qfix,
-                                      T dd[5], T f[9]) {
-#pragma unroll
-  for (int a = 0; a < 5; ++a) dd[a] = d[a * ld + n];
-  df_diff<T, EU>(dd, v[n], v[4 * ld + n], ps[n], prim[n], prim[ld + n], prim[2 * ld + n], gam1,
-                 pinfl, qfix, f);
 }
 
 template <class T, bool EU>
@@ -1243,12 +1185,11 @@ __device__ __forceinline__ void face_tn(const T du[5], const T dl[5], const T fu
 // are loaded before the barrier that precedes its evaluation, so neither
 // waits on HBM latency in the critical path.
 //
-// FORM 0 evaluates the increment with the reference expressions
-// (jacobi_df: implimf_3d.f90:430-463, implimf_eu.f90:301-312), so the FP64
-// instantiation reproduces the stored-increment sweep bit for bit (the same
-// inputs through the same operations); FORM 1 uses the difference form of
-// df_diff (reduced precision).  Neighbours outside the block's real cells
-// contribute zero, as the reference's never-written ghost increments do.
+// The increment is evaluated with the reference expressions (jacobi_df:
+// implimf_3d.f90:430-463, implimf_eu.f90:301-312), so the kernel reproduces the
+// stored-increment sweep bit for bit (the same inputs through the same
+// operations).  Neighbours outside the block's real cells contribute zero, as
+// the reference's never-written ghost increments do.
 // ---------------------------------------------------------------------------
 template <class T>
 __device__ __forceinline__ void cp_async_elem(T* smem, const T* gmem, bool valid) {
@@ -1271,33 +1212,25 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 
 // the increment of one cell read straight from global memory
-template <class T, bool EU, int FORM>
+template <class T, bool EU>
 __device__ __forceinline__ void cell_df(const T* __restrict__ v, const T* __restrict__ prim,
                                         const T* __restrict__ ps, const T* __restrict__ d,
                                         long long ld, long long m, T gam1, T pinfl, int qfix,
                                         T dd[5], T f[9]) {
-  if (FORM == 1) {
-    df_of<T, EU>(v, prim, ps, d, ld, m, gam1, pinfl, qfix, dd, f);
-  } else {
 #pragma unroll
-    for (int a = 0; a < 5; ++a) dd[a] = d[a * ld + m];
-    jacobi_df<T, EU>(dd, v[m], v[ld + m], v[2 * ld + m], v[3 * ld + m], v[4 * ld + m], ps[m],
-                     EU ? T(0.) : prim[m], EU ? T(0.) : prim[ld + m],
-                     EU ? T(0.) : prim[2 * ld + m], gam1, pinfl, qfix, f);
-  }
+  for (int a = 0; a < 5; ++a) dd[a] = d[a * ld + m];
+  jacobi_df<T, EU>(dd, v[m], v[ld + m], v[2 * ld + m], v[3 * ld + m], v[4 * ld + m], ps[m],
+                   EU ? T(0.) : prim[m], EU ? T(0.) : prim[ld + m],
+                   EU ? T(0.) : prim[2 * ld + m], gam1, pinfl, qfix, f);
 }
 
-// staged inputs of one increment: 0-4 d, then rho, rho E, p and the
-// velocity (FORM 1), or v(1..5), p and the velocity (FORM 0, the reference
-// expressions; the Euler form reads no velocity)
-template <int FORM>
-__host__ __device__ constexpr int raw_count(bool eu) {
-  return FORM == 1 ? 11 : (eu ? 11 : 14);
-}
+// staged inputs of one increment: d, v(1..5), p and the velocity (which the
+// Euler form does not read)
+__host__ __device__ constexpr int raw_count(bool eu) { return eu ? 11 : 14; }
 
 // 128-thread patches fit three CTAs per SM (shared memory ~60-67 KB each):
 // registers capped to match
-template <class T, bool EU, int FORM, int TI, int TJ>
+template <class T, bool EU, int TI, int TJ>
 __global__ void __launch_bounds__(TI * TJ, TI * TJ <= 128 ? 3 : 1) k_jacobi_25d(
     const Blk* __restrict__ blks, Tiles tl, Phys ph64, int qfix, long long ld,
     const T* __restrict__ u, const T* __restrict__ v, const T* __restrict__ prim,
@@ -1305,10 +1238,9 @@ __global__ void __launch_bounds__(TI * TJ, TI * TJ <= 128 ? 3 : 1) k_jacobi_25d(
     const T* __restrict__ coefdiag, const T* __restrict__ d_in, T* __restrict__ d_out) {
   pdl_sync();
   constexpr int NX = TI + 2, NY = TJ + 2, NP = NX * NY, NT = TI * TJ;
-  constexpr int NR = raw_count<FORM>(EU);
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
   T* sdf = reinterpret_cast<T*>(smem_raw);  // [2 planes][14 values][NP]: d, f
-  T* sraw = sdf + 2 * 14 * NP;              // [NR inputs][NP]: one staged plane
+  T* sraw = sdf + 2 * 14 * NP;              // [raw_count inputs][NP]: one staged plane
   const int4 t = tl.tile[tl.tile0 + blockIdx.x];
   const Blk B = blks[t.x];
   const int tx = threadIdx.x % TI, ty = threadIdx.x / TI;
@@ -1348,21 +1280,12 @@ __global__ void __launch_bounds__(TI * TJ, TI * TJ <= 128 ? 3 : 1) k_jacobi_25d(
       const long long m = in ? col0[rr] + (long long)kk * B.nijd : 0;
 #pragma unroll
       for (int a = 0; a < 5; ++a) cp_async_elem(r + a * NP + q, d_in + a * ld + m, in);
-      if (FORM == 1) {
-        cp_async_elem(r + 5 * NP + q, v + m, in);
-        cp_async_elem(r + 6 * NP + q, v + 4 * ld + m, in);
-        cp_async_elem(r + 7 * NP + q, ps + m, in);
 #pragma unroll
-        for (int a = 0; a < 3; ++a) cp_async_elem(r + (8 + a) * NP + q, prim + a * ld + m, in);
-      } else {
+      for (int a = 0; a < 5; ++a) cp_async_elem(r + (5 + a) * NP + q, v + a * ld + m, in);
+      cp_async_elem(r + 10 * NP + q, ps + m, in);
+      if (!EU) {
 #pragma unroll
-        for (int a = 0; a < 5; ++a) cp_async_elem(r + (5 + a) * NP + q, v + a * ld + m, in);
-        cp_async_elem(r + 10 * NP + q, ps + m, in);
-        if (!EU) {
-#pragma unroll
-          for (int a = 0; a < 3; ++a)
-            cp_async_elem(r + (11 + a) * NP + q, prim + a * ld + m, in);
-        }
+        for (int a = 0; a < 3; ++a) cp_async_elem(r + (11 + a) * NP + q, prim + a * ld + m, in);
       }
     }
   };
@@ -1381,14 +1304,10 @@ __global__ void __launch_bounds__(TI * TJ, TI * TJ <= 128 ? 3 : 1) k_jacobi_25d(
 #pragma unroll
       for (int a = 0; a < 5; ++a) dd[a] = r[a * NP + q];
       if (in) {
-        if (FORM == 1)
-          df_diff<T, EU>(dd, r[5 * NP + q], r[6 * NP + q], r[7 * NP + q], r[8 * NP + q],
-                         r[9 * NP + q], r[10 * NP + q], gam1, pinfl, qfix, f);
-        else
-          jacobi_df<T, EU>(dd, r[5 * NP + q], r[6 * NP + q], r[7 * NP + q], r[8 * NP + q],
-                           r[9 * NP + q], r[10 * NP + q], EU ? T(0.) : r[11 * NP + q],
-                           EU ? T(0.) : r[12 * NP + q], EU ? T(0.) : r[13 * NP + q], gam1,
-                           pinfl, qfix, f);
+        jacobi_df<T, EU>(dd, r[5 * NP + q], r[6 * NP + q], r[7 * NP + q], r[8 * NP + q],
+                         r[9 * NP + q], r[10 * NP + q], EU ? T(0.) : r[11 * NP + q],
+                         EU ? T(0.) : r[12 * NP + q], EU ? T(0.) : r[13 * NP + q], gam1, pinfl,
+                         qfix, f);
       } else {
 #pragma unroll
         for (int a = 0; a < 9; ++a) f[a] = T(0.);
@@ -1403,8 +1322,8 @@ __global__ void __launch_bounds__(TI * TJ, TI * TJ <= 128 ? 3 : 1) k_jacobi_25d(
   // the own column's plane kbeg-1 (registers)
   T pd[5], pf[9];
   if (own && kbeg >= 2) {
-    cell_df<T, EU, FORM>(v, prim, ps, d_in, ld, cell_index(B, i, j, kbeg - 1), gam1, pinfl,
-                         qfix, pd, pf);
+    cell_df<T, EU>(v, prim, ps, d_in, ld, cell_index(B, i, j, kbeg - 1), gam1, pinfl, qfix, pd,
+                   pf);
   } else {
 #pragma unroll
     for (int a = 0; a < 5; ++a) pd[a] = T(0.);
@@ -1536,26 +1455,20 @@ __global__ void __launch_bounds__(TI * TJ, TI * TJ <= 128 ? 3 : 1) k_jacobi_25d(
       pd[a] = d0[a];
     }
     if (own) {
-      if (FORM == 1) {
-        const T rc = T(1.) / cd;
 #pragma unroll
-        for (int a = 0; a < 5; ++a) d_out[a * ld + n] = d2w[a] * rc;
-      } else {
-#pragma unroll
-        for (int a = 0; a < 5; ++a) d_out[a * ld + n] = d2w[a] / cd;
-      }
+      for (int a = 0; a < 5; ++a) d_out[a * ld + n] = d2w[a] / cd;
     }
   }
   cp_async_wait<0>();
 }
 
-template <int TI, int TJ, class T, int FORM, bool EU>
+template <int TI, int TJ, class T, bool EU>
 constexpr size_t jacobi_25d_smem() {
   // two planes of increments (d, f) and one staged plane of raw inputs
-  return sizeof(T) * (2 * 14 + raw_count<FORM>(EU)) * (TI + 2) * (TJ + 2);
+  return sizeof(T) * (2 * 14 + raw_count(EU)) * (TI + 2) * (TJ + 2);
 }
 
-template <class T, int FORM, int TI, int TJ>
+template <class T, int TI, int TJ>
 cudaError_t jacobi_25d_shape(const Blk* blks, Tiles tl, Phys ph, int qfix, int eu,
                              long long ld, const T* u, const T* v, const T* prim, const T* ps,
                              const T* sn, const T* coefe, const T* coefdiag, const T* d_in,
@@ -1565,13 +1478,13 @@ cudaError_t jacobi_25d_shape(const Blk* blks, Tiles tl, Phys ph, int qfix, int e
                                               coefdiag, d_in, d_out);
   };
   if (eu)
-    run(k_jacobi_25d<T, true, FORM, TI, TJ>, jacobi_25d_smem<TI, TJ, T, FORM, true>());
+    run(k_jacobi_25d<T, true, TI, TJ>, jacobi_25d_smem<TI, TJ, T, true>());
   else
-    run(k_jacobi_25d<T, false, FORM, TI, TJ>, jacobi_25d_smem<TI, TJ, T, FORM, false>());
+    run(k_jacobi_25d<T, false, TI, TJ>, jacobi_25d_smem<TI, TJ, T, false>());
   return cudaGetLastError();
 }
 
-template <class T, int FORM>
+template <class T>
 cudaError_t jacobi_25d_dispatch(const Blk* blks, Tiles tl, Phys ph, int qfix, int eu,
                                 long long ld, const T* u, const T* v, const T* prim,
                                 const T* ps, const T* sn, const T* coefe, const T* coefdiag,
@@ -1579,8 +1492,8 @@ cudaError_t jacobi_25d_dispatch(const Blk* blks, Tiles tl, Phys ph, int qfix, in
   if (tl.ntiles == 0) return cudaSuccess;
 #define CNS_SHAPE(A, B)                                                                   \
   if (tl.ti == A && tl.tj == B)                                                           \
-    return jacobi_25d_shape<T, FORM, A, B>(blks, tl, ph, qfix, eu, ld, u, v, prim, ps, sn, \
-                                           coefe, coefdiag, d_in, d_out, st);
+    return jacobi_25d_shape<T, A, B>(blks, tl, ph, qfix, eu, ld, u, v, prim, ps, sn, coefe, \
+                                     coefdiag, d_in, d_out, st);
   CNS_SHAPE(32, 4)
   CNS_SHAPE(32, 8)
   CNS_SHAPE(16, 8)
@@ -1589,24 +1502,24 @@ cudaError_t jacobi_25d_dispatch(const Blk* blks, Tiles tl, Phys ph, int qfix, in
   return cudaErrorInvalidValue;
 }
 
-template <class T, int FORM, int TI, int TJ>
+template <class T, int TI, int TJ>
 cudaError_t jacobi_25d_attr_shape() {
-  cudaError_t e = cudaFuncSetAttribute(k_jacobi_25d<T, true, FORM, TI, TJ>,
+  cudaError_t e = cudaFuncSetAttribute(k_jacobi_25d<T, true, TI, TJ>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)jacobi_25d_smem<TI, TJ, T, FORM, true>());
+                                       (int)jacobi_25d_smem<TI, TJ, T, true>());
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_jacobi_25d<T, false, FORM, TI, TJ>,
+    e = cudaFuncSetAttribute(k_jacobi_25d<T, false, TI, TJ>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)jacobi_25d_smem<TI, TJ, T, FORM, false>());
+                             (int)jacobi_25d_smem<TI, TJ, T, false>());
   return e;
 }
 
-template <class T, int FORM>
+template <class T>
 cudaError_t jacobi_25d_attr() {
-  cudaError_t e = jacobi_25d_attr_shape<T, FORM, 32, 4>();
-  if (e == cudaSuccess) e = jacobi_25d_attr_shape<T, FORM, 32, 8>();
-  if (e == cudaSuccess) e = jacobi_25d_attr_shape<T, FORM, 16, 8>();
-  if (e == cudaSuccess) e = jacobi_25d_attr_shape<T, FORM, 16, 16>();
+  cudaError_t e = jacobi_25d_attr_shape<T, 32, 4>();
+  if (e == cudaSuccess) e = jacobi_25d_attr_shape<T, 32, 8>();
+  if (e == cudaSuccess) e = jacobi_25d_attr_shape<T, 16, 8>();
+  if (e == cudaSuccess) e = jacobi_25d_attr_shape<T, 16, 16>();
   return e;
 }
 

@@ -77,7 +77,7 @@ template <bool EU>
 __device__ __forceinline__ void point_df32(const float* __restrict__ st, long long pld,
                                            long long pn, float gam1, float pinfl, int qfix,
                                            const float d[5], float f[9]) {
-  df_diff<float, EU>(d, st[pn], st[pld + pn], st[2 * pld + pn], st[3 * pld + pn],
+  df_diff_f32<EU>(d, st[pn], st[pld + pn], st[2 * pld + pn], st[3 * pld + pn],
                      st[4 * pld + pn], st[5 * pld + pn], gam1, pinfl, qfix, f);
 }
 
@@ -596,7 +596,7 @@ __device__ __forceinline__ bool sweep_f32_tile(const int4 t, const Blk* __restri
 #pragma unroll
       for (int c = 0; c < 5; ++c) x.d[c] = in ? rd[c * PL + o] : 0.f;
       if (in) {
-        df_diff<float, EU>(x.d, rs[o], rs[PL + o], rs[2 * PL + o], rs[3 * PL + o],
+        df_diff_f32<EU>(x.d, rs[o], rs[PL + o], rs[2 * PL + o], rs[3 * PL + o],
                            rs[4 * PL + o], rs[5 * PL + o], gam1, pinfl, qfix, x.f);
       } else {
 #pragma unroll
@@ -623,7 +623,7 @@ __device__ __forceinline__ bool sweep_f32_tile(const int4 t, const Blk* __restri
     const long long pm = pad_index(B, i, j, kbeg - 1);
 #pragma unroll
     for (int c = 0; c < 5; ++c) pk.d[c] = d_in[c * pld + pm];
-    df_diff<float, EU>(pk.d, st[pm], st[pld + pm], st[2 * pld + pm], st[3 * pld + pm],
+    df_diff_f32<EU>(pk.d, st[pm], st[pld + pm], st[2 * pld + pm], st[3 * pld + pm],
                        st[4 * pld + pm], st[5 * pld + pm], gam1, pinfl, qfix, pk.f);
   } else {
 #pragma unroll

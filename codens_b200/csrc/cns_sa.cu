@@ -33,19 +33,17 @@ __device__ __forceinline__ double pow6(double x) {  // gcc's x**6: x3 * x3
 }
 
 // scalar q of cell n: mode 0 = the velocity component q (teq_gradv.f90:
-// t(:,q+1) / max(t(:,1), 1e-20)), mode 1 = the field f, mode 2 = the
-// transport variable q per unit mass (met_gradtr.f90:78-84: s(:,6+q) / s(:,1)),
-// mode 3 = sqrt(s(:,6) / s(:,1)) (met_bark.f90:91-99)
+// t(:,q+1) / max(t(:,1), 1e-20)), mode 2 = the transport variable q per unit
+// mass (met_gradtr.f90:78-84: s(:,6+q) / s(:,1)), mode 3 = sqrt(s(:,6) / s(:,1))
+// (met_bark.f90:91-99)
 __device__ __forceinline__ double scalar_of(int mode, const double* __restrict__ v,
-                                            const double* __restrict__ f, long long ld,
-                                            long long n, int q) {
+                                            long long ld, long long n, int q) {
   if (mode == 0) return v[(q + 1) * ld + n] / fmax(v[n], 1.e-20);
   if (mode == 2) return v[(5 + q) * ld + n] / v[n];
-  if (mode == 3) return sqrt(v[5 * ld + n] / v[n]);
-  return f[q * ld + n];
+  return sqrt(v[5 * ld + n] / v[n]);
 }
 
-// the scalars of modes 0 and 2 over the flat cell range [n0, n1) into
+// the scalars of modes 0, 2 and 3 over the flat cell range [n0, n1) into
 // sc[q][ld], once per cell (the gradient kernel reads each six more times)
 template <int NSC>
 __global__ void __launch_bounds__(256) k_teq_scalars(int mode, const double* __restrict__ v,
@@ -55,7 +53,7 @@ __global__ void __launch_bounds__(256) k_teq_scalars(int mode, const double* __r
   const long long n = n0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= n1) return;
 #pragma unroll
-  for (int q = 0; q < NSC; ++q) sc[q * ld + n] = scalar_of(mode, v, nullptr, ld, n, q);
+  for (int q = 0; q < NSC; ++q) sc[q * ld + n] = scalar_of(mode, v, ld, n, q);
 }
 
 // teq_grads.f90:38-346 per real cell: the Green-Gauss sum over the six faces

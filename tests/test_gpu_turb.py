@@ -260,3 +260,34 @@ def test_impli2_eqt_3d_parity(cuda, name):
         s.sync()
         assert_equal_bits(tg.cpu().numpy().reshape(7, ld), to, f"v (l={l})")
     s.close()
+
+
+def test_impli2_after_a_call_on_a_broken_state(cuda):
+    """the step's scratch is not cleared between calls: every entry that a call
+    reads is one that it wrote, or a ghost entry that no call writes"""
+    torch = cuda
+    case = CASES["channel"]()
+    orc, st = oracle_prepared(case)
+    s = _gpu(case)
+    t = _transport_state(case, st)
+    ld = case.layout.ld
+    mu, mut, _ = _fields(case, 71)
+    r = cases.splitmix64_uniform(73, 4 * ld).reshape(4, ld)
+    dt, cfke = 0.01 + 0.01 * r[0], r[1]
+    u = np.zeros((7, ld))
+    u[5], u[6] = (r[2] - 0.5) * 1e-4, (r[3] - 0.5) * 1e-3
+
+    def step(l, u, t, mu):
+        tg = _t(torch, t.reshape(-1))
+        s.impli2_eqt_3d(l, _t(torch, u.reshape(-1)), _t(torch, dt), tg, _t(torch, mu),
+                        _t(torch, mut), _t(torch, cfke), s.sn, s.vol, 1.0)
+        s.sync()
+        return tg.cpu().numpy().reshape(7, ld)
+
+    for l in (2, 1, 3):
+        step(0, np.full_like(u, np.nan), np.full_like(t, np.nan), np.full_like(mu, np.inf))
+        to = t.copy()
+        orc_lib().orc_impli2_eqt_3d(l, u.reshape(-1), dt, to.reshape(-1), mu, mut, cfke, st.sn,
+                                    st.vol, 1.0)
+        assert_equal_bits(step(l, u, t, mu), to, f"v (l={l})")
+    s.close()
