@@ -157,7 +157,6 @@ __global__ void __launch_bounds__(256) k_prim(long long n0, long long n1,
   }
 }
 
-// chronos.f90:110-194 (kprec = 0)
 // the length of cell nc: volume by face area (chronos.f90:110-130)
 __device__ __forceinline__ double chronos_length(const Blk& B, long long nc,
                                                  const double* __restrict__ sn,
@@ -238,7 +237,8 @@ __global__ void __launch_bounds__(kTile) k_zpres_chronos(
 // ---------------------------------------------------------------------------
 
 // one list entry of a coincident, extrapolation, adiabatic-wall or
-// outlet-pressure boundary; injection boundaries are handled by k_clidd.
+// outlet-pressure boundary; injection boundaries are handled by
+// k_clidd_count and k_clidd_apply.
 // rbvc runs before and after the physical conditions in the reference; every
 // ghost cell depends on interior cells only, so one pass gives the same values.
 // An entry is a chain of latencies (the lists, then its cells): it loads all

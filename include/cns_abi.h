@@ -560,13 +560,14 @@ int cns_sch_dual(cns_ctx *ctx, int l, double *u, const double *v, int icycle,
  * the first runs 2.5D-blocked over patches of ti x tj cell columns, at most kc
  * planes deep (fewer where that fills the last wave of CTAs better); layouts
  * small enough for the L2 cache run one thread per cell instead and use no
- * tiles (the same bits).  The first fused iteration of each precision tunes the tiling
- * on its own data (no result depends on it: the FP32 sweeps round every
- * operation explicitly).  cns_sweep_tiles returns {ti, tj, kc, source} of
+ * tiles (the same bits); their tiling is tuned, cached and reported all the
+ * same.  The first fused iteration of each precision tunes the tiling on its own
+ * data (no result depends on it: the FP32 sweeps round every operation
+ * explicitly).  cns_sweep_tiles returns {ti, tj, kc, source} of
  * precision 0 (FP64) or 1/2 (FP32 sweeps), source 0 = the default or a tiling
  * set by cns_set_sweep_tiles, 1 = timed on the data, 2 = read from the tuning
  * cache; cns_set_sweep_tiles fixes a tiling (ti x tj one of 32x4, 32x8, 16x8,
- * 16x16; kc >= 1).  cns_set_tune_cache names a text file of tuned tilings,
+ * 16x16; kc >= 1, past the deepest block: whole columns).  cns_set_tune_cache names a text file of tuned tilings,
  * one line "key ti tj kc" per (GPU name, SM count, sweep precision,
  * equations, log2 real cells, log2 blocks, log2 cells of the smallest block):
  * a configuration found there is used without timing (the same tiling on
@@ -584,8 +585,8 @@ int cns_set_tune_cache(cns_ctx *ctx, const char *path);
 int cns_set_sweep_staging(cns_ctx *ctx, int mode);
 int cns_sweep_staging(cns_ctx *ctx, int32_t *mode);
 /* Residual kernel variant (no counterpart in the reference): ti = 0 selects
- * the face kernels (one launch per direction into a face buffer, then the
- * per-cell accumulation); ti x tj = 32 x 4 or 16 x 8 selects the fused kernel
+ * the face kernels (one launch for the three directions into a face buffer,
+ * then the per-cell accumulation); ti x tj = 32 x 4 or 16 x 8 selects the fused kernel
  * (all three directions and the accumulation in one launch over 2.5D tiles
  * of kc planes).  Both give the same bits in FP64.  cns_residual_tiles
  * returns {ti, tj, kc} (zeros for the face kernels). */

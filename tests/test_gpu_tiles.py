@@ -1,8 +1,9 @@
-"""The 2.5D Jacobi sweep tiling: every patch shape and plane count gives the
-same FP64 iteration bit for bit (each cell's arithmetic does not depend on
-the tiling), the autotuner runs on the first fused iteration, and the
-reduced-precision forms are tiling-independent bit for bit too, with the
-planes staged as tensor boxes (the default) or by cp.async element copies."""
+"""The 2.5D Jacobi sweep tiling as a setting: the autotuner runs on the first
+fused iteration, and on the small cases here, whose sweeps are point sweeps,
+no patch shape, plane count or staging changes the iteration.
+The tiled sweeps' own results are compared on layouts above the point sweeps'
+sizes (test_gpu_tiled_forms.py, test_gpu_point_sweeps.py).  The fused residual,
+which runs in tiles at every size, gives the face kernels' bits."""
 from __future__ import annotations
 
 import numpy as np
